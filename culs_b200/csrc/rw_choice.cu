@@ -2,21 +2,16 @@
 // loop of rw::CPUSolver::Rewrite (CULS src/algorithms/rewrite.cu:830-921,
 // rewrite.h:118-124,208-220) moved onto the GPU.
 //
-// Choice: one thread per graph walks that graph's candidates in id order and
-// replays FastDelete with an explicit stack that follows the reference's
-// recursion step by step (its order of reference-count updates matters when
-// a cone reaches a node along two paths: a node can be deleted twice) and
-// install with a worklist (its outcome does not depend on the order).  The walk is
-// a chain of dependent memory accesses, so it is written to shorten that
-// chain: each candidate's record (node, replacement, cut leaves) is gathered
-// beforehand in graph order and read one candidate ahead; the loads a
-// candidate needs before its first store are issued together; a traversal
-// frame carries its node's two fanins, the top frame lives in registers and
-// the next ones in shared memory; reference-count updates whose old value is
-// not needed are fire-and-forget atomics (a thread's own later loads of the
-// same word observe them).  A single graph of up to 65,536 objects runs on a
-// thread-block cluster instead, with its arrays in the blocks' distributed
-// shared memory (k_choice_cluster).
+// Choice: one block per graph works through that graph's candidates in id
+// order, a window of them at a time (k_choice).  Every thread of the window
+// replays one candidate -- install, FastDelete, commit or revert, step by
+// step as the reference's recursion does (its order of reference-count
+// updates matters when a cone reaches a node along two paths: a node can be
+// deleted twice) -- against the committed graph, with its own changes kept in
+// a small overlay.  A candidate whose overlay holds a node that an earlier
+// candidate of the window changes has seen a stale graph; everything before
+// the first such candidate is exactly what the sequential loop would have
+// done, is committed at once, and the next window starts there.
 //
 // Redundancy removal chases buffer chains.  The reference does it in one
 // sequential sweep in which a node's fanins, once rewritten, can make it
@@ -28,400 +23,473 @@
 #include <climits>
 #include <cstdlib>
 
-#include <cooperative_groups.h>
-
 #include "rw_work.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace culs {
 
 namespace {
 
-constexpr int kChoiceBlock = 32;   // graphs per block, one thread each
-constexpr int kChoiceFrames = 64;  // frames per graph held in shared memory
+// Nodes a candidate may touch in its overlay, and frames of its traversal
+// stack.  On the 1M-AND layered graph (rw -z) candidates touch 5 nodes above
+// the inputs on average and at most 53 reads of 24 traversed nodes; a
+// candidate that needs more is replayed alone on the committed graph.
+constexpr int kOverlay = 32;  // a multiple of 4
+constexpr int kSpecFrames = 16;
 
 struct ChoiceArgs {
     int64_t nL0;  // W positions [0, nL0) are constants and PIs
     const DevGraph *dg;
-    int *L0, *L1, *ref;
-    uint8_t *del;
+    int4 *rec;                // per node {L0, L1, ref, del}
+    int *mark;                // per node: lowest window place that changes it (INT_MAX: none)
     const int4 *recA, *recB;  // per candidate in graph order: {c, q, rep, -}, leaves
     const int *gStart, *gCount;
     int useZeros;
+    int serial;  // replay every candidate alone
     int4 *stack;
     int stackCap;
     int *choice;
-    unsigned long long *stats;  // replaced, pos, zero, reverted, compromised, newIdx, selfRef, expected
+    unsigned long long *stats;  // replaced, pos, zero, reverted, compromised, selfRef, expected
     int *status;
 };
 
-// The graph arrays the walk reads and writes.  GlobalMem: the arrays in HBM
-// (one thread per graph of a batch).  ClusterMem: for a single graph small
-// enough, the same arrays copied into the distributed shared memory of a
-// thread-block cluster, object x at offset x & mask of block x >> shift, so
-// that every access of the walk's dependent chain is a shared-memory access
-// of this SM or a neighbour instead of an L2 round trip.  Only one thread
-// walks, so the reference-count updates need no atomicity there; they stay
-// atomics because a fire-and-forget `red` does not stall the thread.
-struct GlobalMem {
-    int *L0, *L1, *ref;
-    uint8_t *del;
-    __device__ __forceinline__ int l0(int x) const { return L0[x]; }
-    __device__ __forceinline__ int l1(int x) const { return L1[x]; }
-    __device__ __forceinline__ int dl(int x) const { return del[x]; }
-    __device__ __forceinline__ int rf(int x) const { return ref[x]; }
-    __device__ __forceinline__ void set_del(int x, int v) const { del[x] = (uint8_t)v; }
-    __device__ __forceinline__ void set_fanins(int x, int a, int b) const {
-        L0[x] = a;
-        L1[x] = b;
-    }
-    __device__ __forceinline__ void rf_add(int x, int d) const { atomicAdd(ref + x, d); }
-    __device__ __forceinline__ int rf_add_old(int x, int d) const { return atomicAdd(ref + x, d); }
-    // del (or ref) and both fanins of x
-    __device__ __forceinline__ void dab(int x, int &d, int &a, int &b) const {
-        d = del[x];
-        a = L0[x];
-        b = L1[x];
-    }
-    __device__ __forceinline__ void rab(int x, int &r, int &a, int &b) const {
-        r = ref[x];
-        a = L0[x];
-        b = L1[x];
-    }
-    __device__ __forceinline__ void ab(int x, int &a, int &b) const {
-        a = L0[x];
-        b = L1[x];
-    }
-    static constexpr bool kPrefetch = true;
-};
+// Handles.  A node above the constant and the PIs is changed through its
+// handle; the constant and the PIs have none (-1): their counts
+// never decide anything (FastDelete does not enter them), they are never
+// deleted, and the choice's caller does not read them, so nothing is kept
+// for them.
 
-struct ClusterMem {
-    int4 *rec;  // this block's slice of {L0, L1, ref, del}; every block of the cluster has it at the same offset
-    int shift, mask;
-    __device__ __forceinline__ int4 *at(int x) const {
-        return cg::this_cluster().map_shared_rank(rec + (x & mask), (unsigned)(x >> shift));
-    }
-    __device__ __forceinline__ int l0(int x) const { return at(x)->x; }
-    __device__ __forceinline__ int l1(int x) const { return at(x)->y; }
-    __device__ __forceinline__ int dl(int x) const { return at(x)->w; }
-    __device__ __forceinline__ int rf(int x) const { return at(x)->z; }
-    __device__ __forceinline__ void set_del(int x, int v) const { at(x)->w = v; }
-    __device__ __forceinline__ void set_fanins(int x, int a, int b) const {
-        *reinterpret_cast<int2 *>(at(x)) = make_int2(a, b);
-    }
-    __device__ __forceinline__ void rf_add(int x, int d) const { atomicAdd(&at(x)->z, d); }
-    __device__ __forceinline__ int rf_add_old(int x, int d) const { return atomicAdd(&at(x)->z, d); }
-    __device__ __forceinline__ void dab(int x, int &d, int &a, int &b) const {
-        const int4 r = *at(x);
-        d = r.w;
-        a = r.x;
-        b = r.y;
-    }
-    __device__ __forceinline__ void rab(int x, int &f, int &a, int &b) const {
-        const int4 r = *at(x);
-        f = r.z;
-        a = r.x;
-        b = r.y;
-    }
-    __device__ __forceinline__ void ab(int x, int &a, int &b) const {
-        const int2 r = *reinterpret_cast<const int2 *>(at(x));
-        a = r.x;
-        b = r.y;
-    }
-    static constexpr bool kPrefetch = false;
-};
-
-// Stack frames: FastDelete's {node, step | count << 2, fanin0 literal,
-// fanin1 literal}, install's {node, fanin0 literal, fanin1 literal, 0};
-// frames below kChoiceFrames in shared memory (sh[sp * stride]), deeper ones
-// in the graph's global stack.  The scalars the walk reads at every node are copies held here: read
-// through the argument block, they would be reloaded after every store the
-// compiler cannot tell apart from it.
-template <class Mem>
-struct GraphCtx {
-    const ChoiceArgs *A;
-    Mem m;
-    int trueLit;
-    int4 *sh;
-    int stride;
-    int4 *stk;
+// The committed graph, changed in place; a node's handle is its position.
+struct GraphMem {
+    int4 *rec;
     int64_t nL0;
-    int stackCap;
-    int *status;
-    __device__ __forceinline__ void push(int sp, int4 f) const {
-        if (sp < kChoiceFrames)
-            sh[sp * stride] = f;
-        else
-            stk[sp] = f;
+    __device__ __forceinline__ int4 ld(int x) const { return rec[x]; }
+    __device__ __forceinline__ int append(int x, const int4 &) const { return x >= nL0 ? x : -1; }
+    __device__ __forceinline__ void slots(int x0, const int4 &, int x1, const int4 &, int &k0, int &k1) const {
+        k0 = x0 >= nL0 ? x0 : -1;
+        k1 = x1 >= nL0 ? x1 : -1;
     }
-    __device__ __forceinline__ int4 pop(int sp) const { return sp < kChoiceFrames ? sh[sp * stride] : stk[sp]; }
+    __device__ __forceinline__ int del(int k) const { return k >= 0 ? rec[k].w : 0; }
+    __device__ __forceinline__ int ref(int k, int base) const { return k >= 0 ? rec[k].z : base; }
+    __device__ __forceinline__ void add(int k, int d) {
+        if (k >= 0) rec[k].z += d;
+    }
+    __device__ __forceinline__ void set_del(int k, int v) { rec[k].w = v; }
+    __device__ __forceinline__ void set_fanins(int k, int a, int b) {
+        rec[k].x = a;
+        rec[k].y = b;
+    }
+    __device__ __forceinline__ bool failed() const { return false; }
 };
 
-template <class Mem>
-__device__ __forceinline__ int ch_red(const GraphCtx<Mem> &C, int x, int l0, int l1) {
-    return x >= C.nL0 && (l0 == l1 || l0 == C.trueLit);
-}
+// The committed graph under one candidate's changes; a node's handle is its
+// entry in the thread's overlay.  Entry k: node id and {deleted before: bit
+// 0, deleted now: bit 1, fanins rewritten: bit 2, change of ref: bits 16-31}.
+// The ids lie four to a 16-byte word, words and states thread-minor in shared
+// memory.
+struct OverlayMem {
+    const int4 *rec;
+    int64_t nL0;
+    int4 *ids;
+    int *sts;
+    int stride;
+    int n;
+    bool full;
+    __device__ __forceinline__ int4 ld(int x) const { return rec[x]; }
+    __device__ __forceinline__ int id(int k) const { return reinterpret_cast<const int *>(ids + (k >> 2) * stride)[k & 3]; }
+    // new entry of node x with record r; x has none
+    __device__ __forceinline__ int append(int x, const int4 &r) {
+        if (x < nL0) return -1;
+        if (n == kOverlay) {
+            full = true;
+            return 0;  // the candidate is abandoned, so any entry will do
+        }
+        reinterpret_cast<int *>(ids + (n >> 2) * stride)[n & 3] = x;
+        sts[n * stride] = r.w ? 3 : 0;
+        return n++;
+    }
+    // the entries of x0 and x1, made when absent (places beyond n hold
+    // leftovers, which are not entries)
+    __device__ __forceinline__ void slots(int x0, const int4 &r0, int x1, const int4 &r1, int &k0, int &k1) {
+        k0 = k1 = -1;
+        for (int k = 0; k < n; k += 4) {
+            const int4 v = ids[(k >> 2) * stride];
+            const int left = n - k;
+            if (v.x == x0) k0 = k;
+            if (v.x == x1) k1 = k;
+            if (v.y == x0 && left > 1) k0 = k + 1;
+            if (v.y == x1 && left > 1) k1 = k + 1;
+            if (v.z == x0 && left > 2) k0 = k + 2;
+            if (v.z == x1 && left > 2) k1 = k + 2;
+            if (v.w == x0 && left > 3) k0 = k + 3;
+            if (v.w == x1 && left > 3) k1 = k + 3;
+        }
+        if (k0 < 0) {
+            k0 = append(x0, r0);
+            if (x0 == x1) k1 = k0;
+        }
+        if (k1 < 0) k1 = append(x1, r1);
+    }
+    __device__ __forceinline__ int del(int k) const { return k >= 0 ? (sts[k * stride] >> 1) & 1 : 0; }
+    __device__ __forceinline__ int ref(int k, int base) const { return k >= 0 ? base + (sts[k * stride] >> 16) : base; }
+    __device__ __forceinline__ void add(int k, int d) {
+        if (k >= 0) sts[k * stride] += d * 65536;
+    }
+    __device__ __forceinline__ void set_del(int k, int v) { sts[k * stride] = (sts[k * stride] & ~2) | (v << 1); }
+    __device__ __forceinline__ void set_fanins(int k, int, int) { sts[k * stride] |= 4; }
+    __device__ __forceinline__ bool failed() const { return full; }
+    // whether the node of state st ends up changed
+    static __device__ __forceinline__ bool changed(int st) { return (st >> 16) != 0 || (st & 4) || ((st ^ (st >> 1)) & 1); }
+};
 
-// A pushed FastDelete frame's two fanins are read together: their (ref, L0,
-// L1).  L0 and L1 do not change during FastDelete, and the ref of the second
-// fanin changes only inside the first fanin's subtree, so the second fanin
-// is read again only when its frame resumes after that subtree.
+// Traversal stacks.  Frames: FastDelete's {handle, count << 2 | where to
+// resume (1: at fanin 1, 2: at the end), fanin0 literal, fanin1 literal},
+// install's {handle, 0, fanin0 literal, fanin1 literal}.
+struct GraphStack {
+    int4 *s;
+    int cap;
+    int *status;
+    bool full;
+    __device__ __forceinline__ void push(int &sp, int4 f) {
+        if (sp + 1 >= cap) {
+            set_status(status, kDevStackOverflow);
+            full = true;
+            return;
+        }
+        s[sp++] = f;
+    }
+    __device__ __forceinline__ int4 pop(int &sp) const { return s[--sp]; }
+};
 
-// install lambda, rewrite.cu:835-847; rootDel, r0, r1 = del, L0, L1 of root.
-// Whether a node is installed depends only on the deletion flags, which the
-// walk clears as it reaches nodes, and install reads no reference count, so
-// every visiting order installs the same nodes, makes the same increments
-// and returns the same count: a worklist (a node's deleted fanins are
-// cleared and queued when the node is taken) instead of the recursion.
-template <class Mem>
-__device__ int ch_install(const GraphCtx<Mem> &C, int root, int rootDel, int r0, int r1) {
-    const Mem &m = C.m;
-    if (!rootDel) return 0;
-    m.set_del(root, 0);
-    int cnt = 0, sp = 0;
-    int x = root, l0 = r0, l1 = r1;
-    while (true) {
-        cnt += 1 - ch_red(C, x, l0, l1);
+// (the frames are an array of their own, so that the walk's scalars beside
+// them stay in registers)
+struct SpecStack {
+    int4 *s;
+    bool full;
+    __device__ __forceinline__ void push(int &sp, int4 f) {
+        if (sp >= kSpecFrames) {
+            full = true;
+            return;
+        }
+        s[sp++] = f;
+    }
+    __device__ __forceinline__ int4 pop(int &sp) const { return s[--sp]; }
+};
+
+// One candidate of the choice loop (rewrite.cu:849-897), replayed one
+// traversed node per step, so that the lanes of a warp, each with a candidate
+// of its own, take every node's loads together (as nested loops the lanes
+// drifted apart and a window's replays ran one lane at a time: 80 us a round
+// instead of 9).
+//
+// install (rewrite.cu:835-847): whether a node is installed depends only on
+// the deletion flags, which the walk clears as it reaches nodes, and install
+// reads no reference count, so every visiting order installs the same nodes,
+// makes the same increments and returns the same count: a worklist (a node's
+// deleted fanins are cleared and queued when the node is taken) instead of
+// the recursion.
+//
+// FastDelete (rewrite.h:208-220): the recursion with an explicit stack.  A
+// node is opened (both fanins' decrements), then its fanin 0 entered if its
+// count fell to zero, then -- with fanin 1's count read again, since fanin
+// 0's subtree may have changed it -- its fanin 1, then it is marked deleted
+// and its count handed to its parent.
+template <class Mem, class Stack>
+struct Replay {
+    Mem m;
+    Stack st;
+    int trueLit;
+    int64_t nL0;
+    int useZeros;
+    // the candidate: its node and replacement, their handles and fanins
+    int rep, kq, q0, q1, kn, n0, n1, nRef;
+    // the walk
+    enum Mode { kInstall, kOpen, kRecheck };
+    int phase, mode, k, l0, l1, cnt, sp;
+    int added, gain, code;
+    bool busy;
+
+    __device__ __forceinline__ int red(int a, int b) const { return a == b || a == trueLit; }
+
+    __device__ __forceinline__ void begin_install(int h, int a, int b) {
+        m.set_del(h, 0);
+        mode = kInstall, k = h, l0 = a, l1 = b, cnt = 0, sp = 0;
+    }
+    __device__ __forceinline__ void begin_delete(int h, int a, int b) { mode = kOpen, k = h, l0 = a, l1 = b, sp = 0; }
+    __device__ __forceinline__ void done(int c) {
+        code = c;
+        busy = false;
+    }
+
+    // a = {c, q, rep, -}, lv the cut's leaves
+    __device__ __forceinline__ void start(int4 a, int4 lv) {
+        const int q = a.y;
+        rep = a.z;
+        const int x = rep >> 1;
+        const int4 rn = m.ld(x), rq = m.ld(q);
+        const int4 r0 = m.ld(lv.x), r1 = m.ld(lv.y), r2 = m.ld(lv.z), r3 = m.ld(lv.w);
+        busy = true;
+        gain = 0;
+        n0 = rn.x, n1 = rn.y, nRef = rn.z, q0 = rq.x, q1 = rq.y;
+        // the leaves are distinct nodes below q; the replacement may be one
+        m.append(lv.x, r0);
+        m.append(lv.y, r1);
+        m.append(lv.z, r2);
+        m.append(lv.w, r3);
+        m.slots(q, rq, x, rn, kq, kn);
+        if (x == q || (n1 >> 1) == q) return done(kChSelfRef);
+        if (r0.w | r1.w | r2.w | r3.w) return done(kChCompromised);
+        phase = 0;
+        if (m.del(kn))
+            begin_install(kn, n0, n1);
+        else
+            finish(0);
+    }
+
+    // the walk of the current phase ended with count c
+    __device__ __forceinline__ void finish(int c) {
+        if (phase == 0) {  // the replacement is installed: delete the node
+            added = c;
+            m.add(kn, 1);
+            phase = 1;
+            return begin_delete(kq, q0, q1);
+        }
+        if (phase == 1) {
+            m.add(kn, -1);
+            gain = c - added;
+            if (gain > 0 || (gain == 0 && useZeros)) {
+                m.set_del(kq, 0);
+                m.set_fanins(kq, trueLit, rep);
+                m.add(kn, 1);
+                return done(kChCommitted);
+            }
+            phase = 2;
+            if (m.del(kq)) return begin_install(kq, q0, q1);
+        }
+        if (phase == 2) {  // the node is back: drop the replacement
+            m.add(kq, 1);
+            phase = 3;
+            if (kn >= 0 && m.ref(kn, nRef) == 0) return begin_delete(kn, n0, n1);
+        }
+        m.add(kq, -1);
+        done(kChReverted);
+    }
+
+    // one node of the walk
+    __device__ __forceinline__ void step() {
         const int c0 = l0 >> 1, c1 = l1 >> 1;
-        int d0, a0, b0, d1, a1, b1;
-        m.dab(c0, d0, a0, b0);
-        m.dab(c1, d1, a1, b1);
-        m.rf_add(c0, 1);
-        m.rf_add(c1, 1);
-        if (d1 && c1 != c0) {
-            if (sp + 1 >= C.stackCap) {
-                set_status(C.status, kDevStackOverflow);
-                return 0;
+        const int4 r0 = m.ld(c0), r1 = m.ld(c1);
+        int k0, k1;
+        m.slots(c0, r0, c1, r1, k0, k1);
+        if (mode == kInstall) {
+            cnt += 1 - red(l0, l1);
+            const int d0 = m.del(k0), d1 = m.del(k1);
+            m.add(k0, 1);
+            m.add(k1, 1);
+            if (d1 && c1 != c0) {
+                m.set_del(k1, 0);
+                st.push(sp, make_int4(k1, 0, r1.x, r1.y));
             }
-            m.set_del(c1, 0);
-            C.push(sp++, make_int4(c1, a1, b1, 0));
-        }
-        if (d0) {
-            m.set_del(c0, 0);
-            x = c0, l0 = a0, l1 = b0;
-        } else if (sp > 0) {
-            const int4 f = C.pop(--sp);
-            x = f.x, l0 = f.y, l1 = f.z;
+            if (d0) {
+                m.set_del(k0, 0);
+                k = k0, l0 = r0.x, l1 = r0.y;
+            } else if (sp > 0) {
+                const int4 f = st.pop(sp);
+                k = f.x, l0 = f.z, l1 = f.w;
+            } else {
+                finish(cnt);
+            }
         } else {
-            return cnt;
-        }
-    }
-}
-
-// FastDelete's two reference-count decrements of a frame's fanins, whose
-// returned values give the fanins' counts; L0 / L1 of both fanins
-template <class Mem>
-__device__ __forceinline__ void fd_open(const Mem &m, int l0, int l1, int &v0, int &a0, int &b0, int &v1, int &a1,
-                                        int &b1) {
-    const int c0 = l0 >> 1, c1 = l1 >> 1;
-    const int o0 = m.rf_add_old(c0, -1);
-    const int o1 = m.rf_add_old(c1, -1);
-    m.ab(c0, a0, b0);
-    m.ab(c1, a1, b1);
-    v1 = o1 - 1;
-    v0 = c0 == c1 ? v1 : o0 - 1;  // one node twice: both decrements precede the first check
-}
-
-// FastDelete, rewrite.h:208-220; r0, r1 = L0, L1 of root.  The recursion
-// replayed with an explicit stack: a node is opened (both fanins'
-// decrements), then its fanin 0 entered if its count fell to zero, then --
-// with fanin 1's count read again, since fanin 0's subtree may have changed
-// it -- its fanin 1, then it is marked deleted and its count handed to its
-// parent.  A pushed frame is {node, count << 2 | where to resume (1: at
-// fanin 1, 2: at the end), fanin0 literal, fanin1 literal}.
-template <class Mem>
-__device__ int ch_fast_delete(const GraphCtx<Mem> &C, int root, int r0, int r1) {
-    const Mem &m = C.m;
-    if (root < C.nL0) return 0;
-    int v0, a0, b0, v1, a1, b1;
-    int x = root, l0 = r0, l1 = r1, sp = 0;
-    fd_open(m, l0, l1, v0, a0, b0, v1, a1, b1);
-    int cnt = 1 - ch_red(C, x, l0, l1);
-    while (true) {
-        // x is open: enter fanin 0 when its count fell to zero
-        if (v0 == 0 && (l0 >> 1) >= C.nL0) {
-            if (sp + 1 >= C.stackCap) {
-                set_status(C.status, kDevStackOverflow);
-                return 0;
+            int v0 = 1, v1;
+            if (mode == kOpen) {
+                cnt = 1 - red(l0, l1);
+                const int o0 = m.ref(k0, r0.z);
+                m.add(k0, -1);
+                v1 = m.ref(k1, r1.z) - 1;
+                m.add(k1, -1);
+                v0 = c0 == c1 ? v1 : o0 - 1;  // one node twice: both decrements precede the first check
+            } else {
+                v1 = m.ref(k1, r1.z);
             }
-            C.push(sp++, make_int4(x, (cnt << 2) | 1, l0, l1));
-            x = l0 >> 1, l0 = a0, l1 = b0;
-            fd_open(m, l0, l1, v0, a0, b0, v1, a1, b1);
-            cnt = 1 - ch_red(C, x, l0, l1);
-            continue;
-        }
-        int resume = 1;  // 1: at fanin 1 of x, 2: x is finished
-        while (true) {
-            if (resume == 1 && v1 == 0 && (l1 >> 1) >= C.nL0) {
-                if (sp + 1 >= C.stackCap) {
-                    set_status(C.status, kDevStackOverflow);
-                    return 0;
+            if (v0 == 0 && k0 >= 0) {
+                st.push(sp, make_int4(k, (cnt << 2) | 1, l0, l1));
+                mode = kOpen, k = k0, l0 = r0.x, l1 = r0.y;
+            } else if (v1 == 0 && k1 >= 0) {
+                st.push(sp, make_int4(k, (cnt << 2) | 2, l0, l1));
+                mode = kOpen, k = k1, l0 = r1.x, l1 = r1.y;
+            } else {
+                while (true) {
+                    m.set_del(k, 1);
+                    if (sp == 0) {
+                        finish(cnt);
+                        break;
+                    }
+                    const int4 f = st.pop(sp);
+                    k = f.x, l0 = f.z, l1 = f.w;
+                    cnt += f.y >> 2;
+                    if ((f.y & 3) == 1) {
+                        mode = kRecheck;
+                        break;
+                    }
                 }
-                C.push(sp++, make_int4(x, (cnt << 2) | 2, l0, l1));
-                x = l1 >> 1, l0 = a1, l1 = b1;
-                fd_open(m, l0, l1, v0, a0, b0, v1, a1, b1);
-                cnt = 1 - ch_red(C, x, l0, l1);
-                break;  // the new node is open
             }
-            m.set_del(x, 1);
-            if (sp == 0) return cnt;
-            const int4 f = C.pop(--sp);
-            x = f.x, l0 = f.z, l1 = f.w;
-            cnt += f.y >> 2;
-            resume = f.y & 3;
-            if (resume == 1) m.rab(l1 >> 1, v1, a1, b1);
         }
+        if (m.failed() || st.full) busy = false;
+    }
+};
+
+// Rounds of a window of candidates, one per thread (see the top of the
+// file); T threads, the window's places dealt to the warps in turn.  A round
+// is three block barriers: every thread replays its candidate and lowers the
+// mark of each node it changes to its place in the window (one red per node);
+// a thread whose overlay holds a node marked by a lower place must wait, and
+// the lowest such place ends the part that is committed; committing adds the
+// overlay's changes to the records, which no other committed candidate has
+// read.  A candidate that outgrows its overlay ends the window and, at its
+// start, is replayed by thread 0 on the committed graph.  The next window is
+// up to four times the part committed, at least two places a warp.
+//
+// Bound: the latency of a replay's dependent record loads (about ten), 9 us a
+// round.  One thread walking the candidates took 2.3-2.5 us for each.  64x64
+// multiplier (4,157 candidates, 25 committed at a time): 9.6 -> 1.5 ms;
+// 1M-AND layered graph with rw -z (80,251 tried, 295 at a time): 202 -> 4.5
+// ms; 256 graphs of up to 200k ANDs: 15.1 -> 2.6 ms.
+template <int T>
+__global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
+    extern __shared__ int4 s_overlay[];
+    __shared__ int s_stop[2];
+    constexpr int kWarps = T / 32;
+    const int tid = threadIdx.x, g = blockIdx.x;
+    const int t = (tid & 31) * kWarps + (tid >> 5);  // place in the window
+    const int64_t nL0 = A.nL0;
+    const int trueLit = 2 * A.dg[g].cpos + 1;
+    int base = A.gStart[g];
+    const int end = base + A.gCount[g];
+    if (tid < 2) s_stop[tid] = INT_MAX;
+    __syncthreads();
+    int nDone[kChReverted + 1] = {}, nPos = 0, expected = 0;
+    int window = A.serial ? 1 : T;
+    for (int round = 0; base < end; round++) {
+        const int nAct = min(window, end - base);
+        const bool act = t < nAct;
+        int *stop = &s_stop[round & 1];
+        Replay<OverlayMem, SpecStack> R;
+        int4 frames[kSpecFrames];
+        R.m = OverlayMem{A.rec, nL0, s_overlay + tid, reinterpret_cast<int *>(s_overlay + kOverlay / 4 * T) + tid, T, 0, false};
+        R.st = SpecStack{frames, false};
+        R.trueLit = trueLit;
+        R.nL0 = nL0;
+        R.useZeros = A.useZeros;
+        R.busy = false;
+        int4 a = make_int4(-1, -1, -1, -1);
+        if (act) {
+            a = A.recA[base + t];
+            R.start(a, A.recB[base + t]);
+        }
+        while (__any_sync(0xffffffffu, R.busy)) {
+            if (R.busy) R.step();
+            __syncwarp();
+        }
+        const bool alone = R.m.full || R.st.full || A.serial;
+        if (act && !alone)
+            for (int k = 0; k < R.m.n; k++)
+                if (OverlayMem::changed(R.m.sts[k * T])) atomicMin(&A.mark[R.m.id(k)], t);
+        if (tid == 0) s_stop[(round + 1) & 1] = INT_MAX;
+        __syncthreads();
+        if (act) {
+            bool wait = alone;
+            if (!wait) {
+                int low = INT_MAX;  // four marks in flight at a time
+                for (int k = 0; k < R.m.n; k += 4) {
+                    const int4 x = R.m.ids[(k >> 2) * T];
+                    const int left = R.m.n - k;
+                    const int m0 = __ldcg(&A.mark[x.x]), m1 = left > 1 ? __ldcg(&A.mark[x.y]) : INT_MAX,
+                              m2 = left > 2 ? __ldcg(&A.mark[x.z]) : INT_MAX,
+                              m3 = left > 3 ? __ldcg(&A.mark[x.w]) : INT_MAX;
+                    low = min(min(low, min(m0, m1)), min(m2, m3));
+                }
+                wait = low < t;
+            }
+            if (wait) atomicMin(stop, t);
+        }
+        __syncthreads();
+        int done = min(*stop, nAct);
+        if (act && !alone) {
+            for (int k = 0; k < R.m.n; k++) {
+                const int st = R.m.sts[k * T], x = R.m.id(k);
+                if (!OverlayMem::changed(st)) continue;
+                A.mark[x] = INT_MAX;
+                if (t >= done) continue;
+                if (st >> 16) atomicAdd(&A.rec[x].z, st >> 16);
+                if ((st ^ (st >> 1)) & 1) A.rec[x].w = (st >> 1) & 1;
+                if (st & 4) {
+                    A.rec[x].x = trueLit;
+                    A.rec[x].y = a.z;
+                }
+            }
+        }
+        int code = R.code, gain = R.gain;
+        if (done == 0) {  // the first candidate alone
+            __syncthreads();
+            if (t == 0) {
+                Replay<GraphMem, GraphStack> S;
+                S.m = GraphMem{A.rec, nL0};
+                S.st = GraphStack{A.stack + (int64_t)g * A.stackCap, A.stackCap, A.status, false};
+                S.trueLit = trueLit;
+                S.nL0 = nL0;
+                S.useZeros = A.useZeros;
+                S.code = kChNotVisited;
+                S.start(a, A.recB[base]);
+                while (S.busy) S.step();
+                code = S.code, gain = S.gain;
+            }
+            done = 1;
+        }
+        if (t < done) {
+            A.choice[a.x] = code;
+#pragma unroll
+            for (int k = 0; k <= kChReverted; k++) nDone[k] += code == k;
+            if (code == kChCommitted) {
+                nPos += gain > 0;
+                expected += gain;
+            }
+        }
+        base += done;
+        window = A.serial ? 1 : min(T, max(2 * kWarps, 4 * done));
+        __syncthreads();
+    }
+    const int tot[7] = {nDone[kChCommitted],   nPos,     nDone[kChCommitted] - nPos, nDone[kChReverted],
+                        nDone[kChCompromised], nDone[kChSelfRef], expected};
+#pragma unroll
+    for (int k = 0; k < 7; k++) {
+        const int v = __reduce_add_sync(0xffffffffu, tot[k]);
+        if ((tid & 31) == 0 && v) atomicAdd(&A.stats[k], (unsigned long long)(long long)v);
     }
 }
 
-// The choice loop over graph g's candidates in id order (rewrite.cu:849-897).
-template <class Mem>
-__device__ void choice_graph(const GraphCtx<Mem> &C, int g) {
-    const ChoiceArgs &A = *C.A;
-    const Mem &m = C.m;
-    const int4 *recA = A.recA, *recB = A.recB;
-    int *choice = A.choice;
-    const bool useZeros = A.useZeros != 0;
-    const int cpos = A.dg[g].cpos;
-    unsigned long long replaced = 0, pos = 0, zero = 0, reverted = 0, comp = 0, noRep = 0, selfRef = 0;
-    long long expected = 0;
-    int i = A.gStart[g];
-    const int e = i + A.gCount[g];
-    int4 na = make_int4(-1, -1, -1, -1), nb = na;
-    if (i < e) {
-        na = recA[i];
-        nb = recB[i];
+// Gathers the nodes' records and clears their marks.
+__global__ void k_choice_pack(int64_t M, const int *L0, const int *L1, const int *ref, const uint8_t *del, int4 *rec,
+                              int *mark) {
+    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < M; x += stride) {
+        rec[x] = make_int4(L0[x], L1[x], ref[x], del[x]);
+        mark[x] = INT_MAX;
     }
-    for (; i < e; i++) {
-        const int4 a = na, lv = nb;
-        if (i + 1 < e) {
-            na = recA[i + 1];
-            nb = recB[i + 1];
-        }
-        if (Mem::kPrefetch && i + 1 < e && (na.z >> 1) >= 0) {
-            // the next candidate's first loads, into L1 while this one runs
-            // (a prefetch carries no value, so later stores cannot make it stale)
-            const int nn = na.z >> 1, nq = na.y;
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.L0 + nn));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.L1 + nn));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.del + nn));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.L0 + nq));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.L1 + nq));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.del + nb.x));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.del + nb.y));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.del + nb.z));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(A.del + nb.w));
-        }
-        const int c = a.x, q = a.y, rep = a.z;
-        const int newIdx = rep >> 1;
-        if (newIdx < 0) {
-            noRep++;
-            choice[c] = kChNoReplace;
-            continue;
-        }
-        // everything read before this candidate's first store
-        int n0, n1, dn, q0, q1;
-        m.dab(newIdx, dn, n0, n1);
-        const int dl = m.dl(lv.x) | m.dl(lv.y) | m.dl(lv.z) | m.dl(lv.w);
-        m.ab(q, q0, q1);
-        if (newIdx == q || (n1 >> 1) == q) {
-            selfRef++;
-            choice[c] = kChSelfRef;
-            continue;
-        }
-        if (dl) {
-            comp++;
-            choice[c] = kChCompromised;
-            continue;
-        }
-        int added = ch_install(C, newIdx, dn, n0, n1);
-        m.rf_add(newIdx, 1);
-        int saved = ch_fast_delete(C, q, q0, q1);
-        m.rf_add(newIdx, -1);
-        if (saved - added > 0 || (saved == added && useZeros)) {
-            replaced++;
-            if (saved - added > 0)
-                pos++;
-            else
-                zero++;
-            expected += saved - added;
-            m.set_del(q, 0);
-            m.set_fanins(q, C.trueLit, rep);
-            m.rf_add(cpos, 1);
-            m.rf_add(newIdx, 1);
-            choice[c] = kChCommitted;
-        } else {
-            reverted++;
-            ch_install(C, q, m.dl(q), q0, q1);
-            m.rf_add(q, 1);
-            if (m.rf(newIdx) == 0) ch_fast_delete(C, newIdx, n0, n1);
-            m.rf_add(q, -1);
-            choice[c] = kChReverted;
-        }
-    }
-    atomicAdd(&A.stats[0], replaced);
-    atomicAdd(&A.stats[1], pos);
-    atomicAdd(&A.stats[2], zero);
-    atomicAdd(&A.stats[3], reverted);
-    atomicAdd(&A.stats[4], comp);
-    atomicAdd(&A.stats[5], noRep);
-    atomicAdd(&A.stats[6], selfRef);
-    atomicAdd(&A.stats[7], (unsigned long long)expected);
 }
 
-__global__ void __launch_bounds__(kChoiceBlock) k_choice(ChoiceArgs A, int G) {
-    __shared__ int4 sh[kChoiceFrames * kChoiceBlock];
-    int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= G) return;
-    GraphCtx<GlobalMem> C{&A,           GlobalMem{A.L0, A.L1, A.ref, A.del}, 2 * A.dg[g].cpos + 1,
-                          sh + threadIdx.x, kChoiceBlock, A.stack + (int64_t)g * A.stackCap,
-                          A.nL0,        A.stackCap,   A.status};
-    choice_graph(C, g);
-}
-
-constexpr int kClusterBlock = 256;
-constexpr int kClusterMaxBlocks = 8;  // the portable cluster size
-constexpr int kClusterMaxShift = 13;  // objects per block: 8192 16-byte records, 128 KB of shared memory
-
-// One graph (G = 1) on a cluster: its M objects' {L0, L1, ref, del} records
-// are copied into the blocks' shared memory, thread 0 of block 0 walks the
-// candidates on them (one 16-byte load gives a node's flag or count and
-// both fanins), and every block writes its slice back.  The blocks that do
-// not walk wait at the cluster barrier.
-__global__ void __launch_bounds__(kClusterBlock) k_choice_cluster(ChoiceArgs A, int64_t M, int shift) {
-    extern __shared__ __align__(16) unsigned char dyn[];
-    __shared__ int4 sh[kChoiceFrames];
-    const int per = 1 << shift;
-    int4 *rec = reinterpret_cast<int4 *>(dyn);
-    cg::cluster_group cl = cg::this_cluster();
-    const int64_t base = (int64_t)cl.block_rank() << shift;
-    for (int k = threadIdx.x; k < per; k += blockDim.x) {
-        const int64_t x = base + k;
-        if (x < M) rec[k] = make_int4(A.L0[x], A.L1[x], A.ref[x], A.del[x]);
-    }
-    cl.sync();
-    if (cl.block_rank() == 0 && threadIdx.x == 0) {
-        GraphCtx<ClusterMem> C{&A,    ClusterMem{rec, shift, per - 1}, 2 * A.dg[0].cpos + 1, sh, 1, A.stack,
-                               A.nL0, A.stackCap,                      A.status};
-        choice_graph(C, 0);
-    }
-    cl.sync();
-    for (int k = threadIdx.x; k < per; k += blockDim.x) {
-        const int64_t x = base + k;
-        if (x < M) {
-            const int4 r = rec[k];
-            A.L0[x] = r.x;
-            A.L1[x] = r.y;
-            A.ref[x] = r.z;
-            A.del[x] = (uint8_t)r.w;
-        }
+// The walk's result (the reference counts are not needed any more).
+__global__ void k_choice_unpack(int64_t M, const int4 *rec, int *L0, int *L1, uint8_t *del) {
+    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < M; x += stride) {
+        const int4 r = rec[x];
+        L0[x] = r.x;
+        L1[x] = r.y;
+        del[x] = (uint8_t)r.w;
     }
 }
 
 // the choice's record of the i-th candidate in graph order: {c, q, rep, -}
 // and the chosen cut's four leaves (the constant in the fourth place of a
-// three-leaf cut); leaves are read only for candidates with a replacement
+// three-leaf cut)
 __global__ void k_cand_records(int64_t n, const int *candByG, const int *cand, const int *repW, const int8_t *bestCut,
                                const int4 *cutL, const int2 *cutM, const int *wg, const DevGraph *dg, int4 *recA,
                                int4 *recB) {
@@ -429,105 +497,106 @@ __global__ void k_cand_records(int64_t n, const int *candByG, const int *cand, c
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         const int c = candByG[i];
         const int q = cand[c];
-        const int rep = repW[c];
-        int4 l = make_int4(0, 0, 0, 0);
-        if ((rep >> 1) >= 0) {
-            const int slot = bestCut[q];
-            l = cutL[(int64_t)q * 8 + slot];
-            if (packed_nleaves((uint32_t)cutM[(int64_t)q * 8 + slot].y) == 3) l.w = dg[wg[q]].cpos;
-        }
-        recA[i] = make_int4(c, q, rep, 0);
+        const int slot = bestCut[q];
+        int4 l = cutL[(int64_t)q * 8 + slot];
+        if (packed_nleaves((uint32_t)cutM[(int64_t)q * 8 + slot].y) == 3) l.w = dg[wg[q]].cpos;
+        recA[i] = make_int4(c, q, repW[c], 0);
         recB[i] = l;
     }
 }
 
-__global__ void k_cand_gid(int64_t n, const int *cand, const int *wg, uint32_t *keys, int *vals, int *gCount) {
+// graph of the i-th candidate that has a replacement
+__global__ void k_cand_gid(int64_t n, const int *withRep, const int *cand, const int *wg, uint32_t *keys, int *vals,
+                           int *gCount) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += stride) {
-        int g = wg[cand[c]];
-        keys[c] = (uint32_t)g;
-        vals[c] = (int)c;
-        atomicAdd(&gCount[g], 1);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const int c = withRep[i];
+        const int g = wg[cand[c]];
+        keys[i] = (uint32_t)g;
+        vals[i] = c;
+        agg_add(gCount, g, 1);
     }
+}
+
+template <int T>
+cudaError_t launch_choice(const ChoiceArgs &A, int G, cudaStream_t s) {
+    const int smem = 2 * kOverlay * T * (int)sizeof(int);  // ids and states
+    cudaError_t e = cudaFuncSetAttribute(k_choice<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_choice<T><<<G, T, smem, s>>>(A);
+    return cudaGetLastError();
 }
 
 }  // namespace
 
 int rw_choice(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats) {
     const int G = w.G;
-    const int64_t nCand = w.nCand;
+    const int64_t nCand = w.nCand, nRep = w.nRep;
+    const int64_t M = w.N + w.nNew;  // extent of L0, L1, ref, del
     cudaStream_t s = X.s;
     Arena &ar = *X.ar;
     int rc;
-    int *gCount = ar.get<int>(G + 1), *gStart = ar.get<int>(G + 1), *candByG = ar.get<int>(nCand + 1);
-    uint32_t *keys = ar.get<uint32_t>(nCand + 1), *keys2 = ar.get<uint32_t>(nCand + 1);
-    int *vals = ar.get<int>(nCand + 1);
-    int4 *recA = ar.get<int4>(nCand + 1), *recB = ar.get<int4>(nCand + 1);
+    int *gCount = ar.get<int>(G + 1), *gStart = ar.get<int>(G + 1), *candByG = ar.get<int>(nRep + 1);
+    uint32_t *keys = ar.get<uint32_t>(nRep + 1), *keys2 = ar.get<uint32_t>(nRep + 1);
+    int *vals = ar.get<int>(nRep + 1);
+    int4 *recA = ar.get<int4>(nRep + 1), *recB = ar.get<int4>(nRep + 1);
     w.choice = ar.get<int>(nCand + 1);
     unsigned long long *dstats = ar.get<unsigned long long>(8);
     // explicit recursion stacks: deep enough for any chain through the
     // levels plus the new nodes
     int64_t stackCap = (int64_t)w.maxLevel + 64;
-    for (int g = 0; g < G; g++) stackCap = std::max<int64_t>(stackCap, 64);
     stackCap = std::min<int64_t>(2 * stackCap + w.nNew / std::max(G, 1) + 64, 1 << 20);
     int4 *stack = ar.get<int4>((size_t)stackCap * G);
-    if (!gCount || !gStart || !candByG || !keys || !keys2 || !vals || !recA || !recB || !w.choice || !dstats || !stack)
+    // the records and marks take the place of the enumeration's cut
+    // attributes (64 bytes per original node), which nothing reads any more
+    int4 *rec;
+    int *mark;
+    if (20 * M <= 64 * w.N) {
+        rec = reinterpret_cast<int4 *>(w.cutA);
+        mark = reinterpret_cast<int *>(rec + M);
+    } else {
+        rec = ar.get<int4>(M);
+        mark = ar.get<int>(M);
+    }
+    if (!gCount || !gStart || !candByG || !keys || !keys2 || !vals || !recA || !recB || !w.choice || !dstats || !stack ||
+        !rec || !mark)
         return X.fail(CULS_E_OOM, "rw: arena exhausted (choice)");
     if ((rc = X.check(cudaMemsetAsync(gCount, 0, sizeof(int) * (G + 1), s), "memset"))) return rc;
     if ((rc = X.check(cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * 8, s), "memset"))) return rc;
-    if (nCand > 0) {
-        k_cand_gid<<<X.grid(nCand), kBlock, 0, s>>>(nCand, w.cand, w.wg, keys, vals, gCount);
+    if ((rc = X.check(fill_i32(w.choice, kChNoReplace, nCand, s), "fill"))) return rc;
+    if (nRep > 0) {
+        k_cand_gid<<<X.grid(nRep), kBlock, 0, s>>>(nRep, w.withRep, w.cand, w.wg, keys, vals, gCount);
         X.launched(1);
         if (G > 1) {
             int bits = 1;
             while ((1ll << bits) < G) bits++;
-            if ((rc = X.check(radix_sort_pairs(keys, vals, keys2, candByG, nCand, bits, ar, s), "sort"))) return rc;
+            if ((rc = X.check(radix_sort_pairs(keys, vals, keys2, candByG, nRep, bits, ar, s), "sort"))) return rc;
         } else {
-            if ((rc = X.check(iota_i32(candByG, 0, nCand, s), "iota"))) return rc;
+            candByG = w.withRep;
         }
-        k_cand_records<<<X.grid(nCand), kBlock, 0, s>>>(nCand, candByG, w.cand, w.repW, w.bestCut, w.cutL, w.cutM, w.wg,
-                                                        w.dg, recA, recB);
-        X.launched(1);
+        k_cand_records<<<X.grid(nRep), kBlock, 0, s>>>(nRep, candByG, w.cand, w.repW, w.bestCut, w.cutL, w.cutM, w.wg,
+                                                       w.dg, recA, recB);
+        if ((rc = X.check(scan_exclusive(gCount, gStart, G, nullptr, ar, s), "scan"))) return rc;
+        k_choice_pack<<<X.grid(M), kBlock, 0, s>>>(M, w.L0, w.L1, w.ref, w.del, rec, mark);
+        // CULS_CHOICE_GLOBAL replays every candidate alone (the tests compare
+        // the two)
+        ChoiceArgs A{w.nL0,  w.dg,  rec,           mark,     recA,   recB,    gStart, gCount, w.useZeros ? 1 : 0,
+                     getenv("CULS_CHOICE_GLOBAL") ? 1 : 0, stack, (int)stackCap, w.choice, dstats, X.status};
+        // Threads per graph: a window as wide as an SM's shared memory allows
+        // while there is an SM for every graph, narrower ones so that more
+        // graphs are resident when there are more (a batch's graphs have
+        // short windows: 7 candidates are committed at a time on the c4
+        // family's, 340 on the 1M-AND graph).
+        if (G <= X.sms)
+            rc = X.check(launch_choice<512>(A, G, s), "choice launch");
+        else if (G <= 3 * X.sms)
+            rc = X.check(launch_choice<256>(A, G, s), "choice launch");
+        else
+            rc = X.check(launch_choice<64>(A, G, s), "choice launch");
+        if (rc) return rc;
+        k_choice_unpack<<<X.grid(M), kBlock, 0, s>>>(M, rec, w.L0, w.L1, w.del);
+        X.launched(4);
     }
-    if ((rc = X.check(scan_exclusive(gCount, gStart, G, nullptr, ar, s), "scan"))) return rc;
-    ChoiceArgs A{w.nL0, w.dg,   w.L0,   w.L1,     w.ref,    w.del,       recA,   recB,  gStart,
-                 gCount, w.useZeros ? 1 : 0,    stack,  (int)stackCap,       w.choice, dstats, X.status};
-    // a single graph that fits: the cluster walk (not on an SM partition,
-    // whose SMs need not hold a whole cluster)
-    const int64_t M = w.N + w.nNew;  // extent of L0, L1, ref, del
-    bool onCluster = false;
-    if (G == 1 && X.clusters && M <= ((int64_t)kClusterMaxBlocks << kClusterMaxShift) && !getenv("CULS_CHOICE_GLOBAL")) {
-        int shift = 8;
-        while (((int64_t)kClusterMaxBlocks << shift) < M) shift++;
-        const int blocks = (int)((M + (1 << shift) - 1) >> shift);
-        const size_t smem = sizeof(int4) << shift;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)blocks);
-        cfg.blockDim = dim3(kClusterBlock);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = (unsigned)blocks;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        int fits = 0;
-        if (cudaFuncSetAttribute(k_choice_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) ==
-                cudaSuccess &&
-            cudaOccupancyMaxActiveClusters(&fits, k_choice_cluster, &cfg) == cudaSuccess && fits > 0) {
-            onCluster = cudaLaunchKernelEx(&cfg, k_choice_cluster, A, M, shift) == cudaSuccess;
-        }
-        (void)cudaGetLastError();  // a configuration the device refuses leaves no error behind
-    }
-    if (!onCluster) {
-        // the walk's working set is the graph's fanins, flags and counts: the
-        // smallest shared-memory carveout leaves the most L1 for it
-        cudaFuncSetAttribute(k_choice, cudaFuncAttributePreferredSharedMemoryCarveout, 0);
-        k_choice<<<(G + kChoiceBlock - 1) / kChoiceBlock, kChoiceBlock, 0, s>>>(A, G);
-    }
-    X.launched(1);
     unsigned long long hs[8], warpPairs = 0;
     if ((rc = X.check(cudaMemcpyAsync(hs, dstats, sizeof hs, cudaMemcpyDeviceToHost, s), "d2h"))) return rc;
     if (w.warpPairs &&
@@ -542,8 +611,8 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats) {
         stats->replacedZero = (long long)hs[2];
         stats->reverted = (long long)hs[3];
         stats->compromised = (long long)hs[4];
-        stats->newIdx = (long long)hs[5];
-        stats->expected = (long long)hs[7];
+        stats->newIdx = nCand - nRep;
+        stats->expected = (long long)hs[6];
         stats->preEval = nAnd - nCand;
         stats->smallCut = 0;
         stats->newNodes = w.nNew;

@@ -549,10 +549,10 @@ int rw_enumerate(ExecCtx &X, RwWork &w) {
     cudaStream_t s = X.s;
     w.cutL = X.ar->get<int4>(N * 8);
     w.cutM = X.ar->get<int2>(N * 8);
-    int2 *cutA = X.ar->get<int2>(N * 8);
+    w.cutA = X.ar->get<int2>(N * 8);
     int *done = X.ar->get<int>(N);
     w.warpPairs = X.ar->get<unsigned long long>(1);
-    if (!w.cutL || !w.cutM || !cutA || !done || !w.warpPairs)
+    if (!w.cutL || !w.cutM || !w.cutA || !done || !w.warpPairs)
         return X.fail(CULS_E_OOM, "rw: scratch arena exhausted (cuts)");
     int rc;
     if ((rc = X.check(cudaMemsetAsync(w.cutM, 0, sizeof(int2) * N * 8, s), "memset"))) return rc;
@@ -568,10 +568,10 @@ int rw_enumerate(ExecCtx &X, RwWork &w) {
     k_level_chunks<<<grid_1d(L, kBlock, X.sms * 16), kBlock, 0, s>>>(L - 1, lvlCnt, X.tune->enumWideMin, cc);
     if ((rc = X.check(scan_exclusive(lvlCnt, lvlStart, L - 1, nullptr, *X.ar, s), "scan"))) return rc;
     if ((rc = X.check(scan_exclusive(cc, chunkStart, L - 1, chunkStart + L - 1, *X.ar, s), "scan"))) return rc;
-    k_enum_init<<<X.grid(N), kBlock, 0, s>>>(N, w.wlev, w.wl, w.lidLow, w.ref, w.cutL, w.cutM, cutA, done);
+    k_enum_init<<<X.grid(N), kBlock, 0, s>>>(N, w.wlev, w.wl, w.lidLow, w.ref, w.cutL, w.cutM, w.cutA, done);
     // lvlStart counts AND nodes only: the AND positions of W start at nL0
     EnumArgs A{w.nL0, N,       lvlCnt, lvlStart, chunkStart, w.maxLevel, X.tune->enumWideMin, w.w0, w.w1,
-               w.ref, w.lidLow, w.cutL, w.cutM, cutA,       done,       X.counters, w.warpPairs, X.status};
+               w.ref, w.lidLow, w.cutL, w.cutM, w.cutA,     done,       X.counters, w.warpPairs, X.status};
     X.mark(kMkEnumK0);
     // a wide batch fills the GPU; a narrow one runs about sixteen levels'
     // worth of chunks at a time (32 nodes a warp on wide levels, 1 on narrow)

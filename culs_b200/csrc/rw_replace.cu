@@ -312,11 +312,13 @@ __global__ void k_rep_newnodes(int64_t K, int64_t N, const int *canon, const int
     }
 }
 
-__global__ void k_rep_final(int64_t nCand, int64_t N, const int *repT, const int *newPos, int *repW) {
+__global__ void k_rep_final(int64_t nCand, int64_t N, const int *repT, const int *newPos, int *repW, uint8_t *hasRep) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nCand; c += stride) {
         int r = repT[c];
-        repW[c] = (r >= 2 * N) ? 2 * newPos[(r >> 1) - N] + (r & 1) : r;
+        r = (r >= 2 * N) ? 2 * newPos[(r >> 1) - N] + (r & 1) : r;
+        repW[c] = r;
+        hasRep[c] = r >= 0;
     }
 }
 
@@ -361,7 +363,9 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
     Arena &ar = *X.ar;
     int rc;
     w.repW = ar.get<int>(nCand + 1);
-    if (!w.repW) return X.fail(CULS_E_OOM, "rw: arena exhausted (replace)");
+    w.withRep = ar.get<int>(nCand + 1);
+    uint8_t *hasRep = ar.get<uint8_t>(nCand + 1);
+    if (!w.repW || !w.withRep || !hasRep) return X.fail(CULS_E_OOM, "rw: arena exhausted (replace)");
     if (nCand == 0) return rep_extend_only(X, w, 0);
     int *kcnt = ar.get<int>(nCand + 1), *koff = ar.get<int>(nCand + 1), *rootRef = ar.get<int>(nCand + 1);
     int *repT = ar.get<int>(nCand + 1);
@@ -432,9 +436,13 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
     if (K > 0)
         k_rep_newnodes<<<X.grid(K), kBlock, 0, s>>>(K, N, canon, f0, f1, c0, c1, newPos, owner, w.cand, w.wg, w.wlev,
                                                     w.L0, w.L1, w.gidAll, w.newOwnLev);
-    k_rep_final<<<X.grid(nCand), kBlock, 0, s>>>(nCand, N, repT, newPos, w.repW);
+    k_rep_final<<<X.grid(nCand), kBlock, 0, s>>>(nCand, N, repT, newPos, w.repW, hasRep);
     X.launched(2);
+    if ((rc = X.check(compact_flags(hasRep, nCand, w.withRep, cnt + 3, ar, s), "compact"))) return rc;
+    if ((rc = X.check(cudaMemcpyAsync(X.hostSmall + 16, cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h")))
+        return rc;
     if ((rc = X.sync())) return rc;
+    w.nRep = X.hostSmall[19];
     return X.status_check("rw replace");
 }
 

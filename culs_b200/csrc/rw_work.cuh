@@ -20,7 +20,6 @@ struct ExecCtx {
     int *hostSmall = nullptr; // 64 pinned host ints
     const RwLib *lib = nullptr;
     int sms = 148;
-    bool clusters = true;  // thread-block clusters may be launched on s (not on an SM-partition stream)
     int *launches = nullptr;
     std::string *err = nullptr;
     const Tune *tune = nullptr;  // launch and schedule parameters
@@ -75,6 +74,7 @@ struct RwWork {
     int *wpo = nullptr;                // PO literals
     int4 *cutL = nullptr;              // 8 cut slots per object: leaves
     int2 *cutM = nullptr;              //   {sign, packed}
+    int2 *cutA = nullptr;              //   leaf attributes, read by the enumeration only
     int *byGraph = nullptr;            // W positions grouped by graph (W order inside a graph)
     RegionTable tab{};                 // existence table, one region per graph
     int8_t *bestCut = nullptr;  // chosen slot or -1
@@ -83,6 +83,8 @@ struct RwWork {
     int64_t nCand = 0;
     int *cand = nullptr;  // W positions of nodes with a chosen cut, W order
     int *repW = nullptr;  // per candidate: replacement literal (rebuilt ids) or -1
+    int64_t nRep = 0;
+    int *withRep = nullptr;  // the candidates that have a replacement, W order
 
     // after the replacement stage: W positions [N, N + nNew) hold new nodes
     int64_t nNew = 0;
