@@ -63,12 +63,13 @@ CULS_DEV int ld_relaxed(const int *p) {
     return v;
 }
 CULS_DEV void st_relaxed(int *p, int v) { asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
+CULS_DEV void acquire_fence() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 CULS_DEV int ld_cg(const int *p) { return __ldcg(p); }
 CULS_DEV int4 ld_cg(const int4 *p) { return __ldcg(p); }
 CULS_DEV int2 ld_cg(const int2 *p) { return __ldcg(p); }
 CULS_DEV void set_status(int *status, int code) { atomicCAS(status, 0, code); }
 CULS_DEV void backoff(int64_t it) {
-    if (it > 64) __nanosleep(it > 4096 ? 256 : 64);
+    if (it > 64) __nanosleep(it > 4096 ? 256 : 32);
 }
 #else
 inline int at_add(int *p, int v) {
@@ -105,6 +106,7 @@ inline int ld_acquire(const int *p) { return *p; }
 inline void st_release(int *p, int v) { *p = v; }
 inline int ld_relaxed(const int *p) { return *p; }
 inline void st_relaxed(int *p, int v) { *p = v; }
+inline void acquire_fence() {}
 inline int ld_cg(const int *p) { return *p; }
 inline void set_status(int *status, int code) {
     if (*status == 0) *status = code;
@@ -128,7 +130,10 @@ CULS_HD int64_t spin_limit(const int *status) {
 // for may itself have been skipped, so one expired wait does not make every
 // dependent wait spin out its own bound.
 CULS_HD bool wait_ge(const int *flag, int target, int *status) {
-    if (ld_acquire(flag) >= target) return true;
+    if (ld_relaxed(flag) >= target) {
+        acquire_fence();
+        return true;
+    }
     const int64_t lim = spin_limit(status);
     for (int64_t it = 1;; ++it) {
         if ((it & 31) == 1 && ld_cg(status) != kDevOk) return false;
@@ -137,7 +142,10 @@ CULS_HD bool wait_ge(const int *flag, int target, int *status) {
             return false;
         }
         backoff(it);
-        if (ld_acquire(flag) >= target) return true;
+        if (ld_relaxed(flag) >= target) {
+            acquire_fence();
+            return true;
+        }
     }
 }
 

@@ -61,11 +61,13 @@ __device__ __forceinline__ T pick4(const T (&v)[4], int i) {
 // MergeCutOrdered / MergeCut with the leaf attributes carried along: four
 // merge steps, each taking the smaller head leaf (both when equal), without
 // branches -- the lanes of the warp-wide enumeration merge different cuts.
-__device__ __forceinline__ bool rc_merge(const RCut &a0, const RCut &b0, RCut &o) {
+// Bit s of pa0 (pb0) is set when a0 (b0) has the merged leaf s: CutTruthPhase
+// (rewrite.cu:195-201).
+__device__ __forceinline__ bool rc_merge(const RCut &a0, const RCut &b0, RCut &o, int &pa0, int &pb0) {
     const bool sw = a0.n < b0.n;
     const RCut &a = sw ? b0 : a0;
     const RCut &b = sw ? a0 : b0;
-    int i = 0, k = 0, c = 0;
+    int i = 0, k = 0, c = 0, pa = 0, pb = 0;
     const int na = (int)a.n, nb = (int)b.n;
 #pragma unroll
     for (int s = 0; s < 4; s++) {
@@ -77,35 +79,32 @@ __device__ __forceinline__ bool rc_merge(const RCut &a0, const RCut &b0, RCut &o
         o.l[s] = act ? (take == 1 ? bk : ai) : 0;
         o.ref[s] = act ? (take == 1 ? pick4(b.ref, k) : pick4(a.ref, i)) : 0u;
         o.lid[s] = act ? (take == 1 ? pick4(b.lid, k) : pick4(a.lid, i)) : 0u;
-        i += (act && take != 1) ? 1 : 0;
-        k += (act && take != 0) ? 1 : 0;
+        const int ta = (act && take != 1) ? 1 : 0, tb = (act && take != 0) ? 1 : 0;
+        i += ta;
+        k += tb;
+        pa |= ta << s;
+        pb |= tb << s;
         c = act ? s + 1 : c;
     }
     o.n = (uint32_t)c;
     o.sign = a0.sign | b0.sign;
     o.used = 1;
+    pa0 = sw ? pb : pa;
+    pb0 = sw ? pa : pb;
     return i >= na && k >= nb;
 }
 
-// CutTruthPhase over register leaves.
-__device__ __forceinline__ int rc_phase(const RCut &x, const RCut &cut) {
-    int ph = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        if ((uint32_t)i >= cut.n) continue;
-        bool in = false;
-#pragma unroll
-        for (int j = 0; j < 4; j++) in |= ((uint32_t)j < x.n) && x.l[j] == cut.l[i];
-        if (in) ph |= 1 << i;
-    }
-    return ph;
+__device__ __forceinline__ bool rc_merge(const RCut &a, const RCut &b, RCut &o) {
+    int pa, pb;
+    return rc_merge(a, b, o, pa, pb);
 }
 
-__device__ __forceinline__ uint32_t rc_truth(const RCut &cut, const RCut &a, const RCut &b, int ca, int cb) {
+// CutTruthtable (rewrite.cu:223-229); pa, pb as rc_merge gives them.
+__device__ __forceinline__ uint32_t rc_truth(const RCut &a, const RCut &b, int ca, int cb, int pa, int pb) {
     uint32_t t0 = ca ? (~a.tt & 0xFFFFu) : a.tt;
     uint32_t t1 = cb ? (~b.tt & 0xFFFFu) : b.tt;
-    t0 = tt_stretch_flat(t0, (int)a.n, rc_phase(a, cut));
-    t1 = tt_stretch_flat(t1, (int)b.n, rc_phase(b, cut));
+    t0 = tt_stretch_flat(t0, (int)a.n, pa);
+    t1 = tt_stretch_flat(t1, (int)b.n, pb);
     return (t0 & t1) & 0xFFFFu;
 }
 
@@ -148,20 +147,6 @@ __device__ __forceinline__ bool rc_minimize(RCut &c) {
     o.n = (uint32_t)nl;
     c = o;
     return true;
-}
-
-// leaves(a) subset of leaves(b)
-__device__ __forceinline__ bool rc_subset(const RCut &a, const RCut &b) {
-    bool all = true;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-        if ((uint32_t)i >= a.n) continue;
-        bool in = false;
-#pragma unroll
-        for (int j = 0; j < 4; j++) in |= ((uint32_t)j < b.n) && b.l[j] == a.l[i];
-        all &= in;
-    }
-    return all;
 }
 
 }  // namespace culs

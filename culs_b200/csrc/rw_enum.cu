@@ -119,84 +119,82 @@ __device__ __forceinline__ void load_rcut(const EnumArgs &A, int64_t idx, int2 m
 }
 
 // ------------------------------------------------- warp-per-node variant
-// One candidate of a node's enumeration: the pair's merged cut (the first
-// CutFilter sees it) and its final form after the truth table and
-// MinimizeCutSupport, with value and aux.
-struct Cand {
-    int x0, x1, x2, x3;  // merged leaves
-    uint32_t xs, xn;     // merged signature, leaf count
-    int y0, y1, y2, y3;  // final leaves
-    uint32_t ys, yn, ytt, yval, a0, a1;
-    uint32_t ok, mini;   // merge succeeded; minimisation removed leaves
+// A warp's scratch: its node's candidates, one per admissible pair.
+struct WarpCands {
+    int4 leaves[64];  // final leaves
+    int4 rec[64];     // final {sign, packed tt / value / nLeaves / used, cutA words}
+    uint4 rel[64];    // the merged cut against earlier candidates' final cuts
+    uint4 relMin[64]; // the same for the final cut, where minimisation removed leaves
+    uint8_t pair[64]; // the k-th admissible pair
 };
 
-__device__ __forceinline__ void make_cand(const RCut &a, const RCut &b, int c0, int c1, Cand &c) {
-    RCut m;
-    c.ok = rc_merge(a, b, m) ? 1u : 0u;
-    c.x0 = m.l[0];
-    c.x1 = m.l[1];
-    c.x2 = m.l[2];
-    c.x3 = m.l[3];
-    c.xs = m.sign;
-    c.xn = m.n;
-    m.tt = rc_truth(m, a, b, c0, c1);
-    c.mini = rc_minimize(m) ? 1u : 0u;
-    c.y0 = m.l[0];
-    c.y1 = m.l[1];
-    c.y2 = m.l[2];
-    c.y3 = m.l[3];
-    c.ys = m.sign;
-    c.yn = m.n;
-    c.ytt = m.tt;
-    c.yval = rc_value(m);
-    rc_pack_aux(m, c.a0, c.a1);
-}
-
-// A candidate in shared memory: four 16-byte words, written once by the lane
-// that built it and read by the whole warp (a broadcast) when its turn in
-// the slot policy comes.
-__device__ __forceinline__ void put_cand(int4 *d, const Cand &c) {
-    d[0] = make_int4(c.x0, c.x1, c.x2, c.x3);
-    d[1] = make_int4(c.y0, c.y1, c.y2, c.y3);
-    d[2] = make_int4((int)c.xs, (int)(c.xn | (c.ok << 8) | (c.mini << 9)), (int)c.ys, (int)c.yn);
-    d[3] = make_int4((int)c.ytt, (int)c.yval, (int)c.a0, (int)c.a1);
-}
-
-__device__ __forceinline__ void get_cand(const int4 *d, Cand &c) {
-    const int4 w0 = d[0], w1 = d[1], w2 = d[2], w3 = d[3];
-    c.x0 = w0.x, c.x1 = w0.y, c.x2 = w0.z, c.x3 = w0.w;
-    c.y0 = w1.x, c.y1 = w1.y, c.y2 = w1.z, c.y3 = w1.w;
-    c.xs = (uint32_t)w2.x;
-    c.xn = (uint32_t)w2.y & 0xFFu;
-    c.ok = ((uint32_t)w2.y >> 8) & 1u;
-    c.mini = ((uint32_t)w2.y >> 9) & 1u;
-    c.ys = (uint32_t)w2.z, c.yn = (uint32_t)w2.w;
-    c.ytt = (uint32_t)w3.x, c.yval = (uint32_t)w3.y, c.a0 = (uint32_t)w3.z, c.a1 = (uint32_t)w3.w;
-}
-
-// CutFilter (rewrite.cu:178-193) with slot k on lane k (k < 8): visiting the
-// slots in index order, a larger slot containing X is dropped and the first
-// slot contained in X drops X and ends the visit.  So every slot lane tests
-// its own slot, one ballot finds the first containing slot, and only the
-// supersets before it are dropped.  Returns true when X is dropped.
-__device__ __forceinline__ bool warp_filter(int lane, int id, const int (&sl)[4], uint32_t ssign, uint32_t &spk,
-                                            const int (&xl)[4], uint32_t xn, uint32_t xs) {
-    bool clr = false, inX = false;
-    if (lane < 8 && lane != id && packed_used(spk)) {
-        const uint32_t kn = packed_nleaves(spk);
-        if (kn > xn)
-            clr = (ssign & xs) == xs && leaves_subset(xl, xn, sl, kn);
+// How cut X stands to the final cuts of candidates 0 .. n - 1 (n <= 64), one
+// bit each: {contained in X: 0-31, larger than X and containing it: 0-31,
+// contained: 32-63, containing: 32-63}.  A cut's leaves are distinct, so the
+// number of equal pairs of leaves decides containment either way; unused
+// places are -1 in X and 0 in the candidates, which no leaf equals (position
+// 0 is a constant, which has no cuts).  CutFilter's signature tests
+// (rewrite.cu:178-193) follow from containment, as a cut's signature is the
+// union of its leaves' bits.
+// With at most 16 candidates, lane and lane + 16 hold the same X and take half
+// of them each.
+__device__ __forceinline__ uint4 relate(const WarpCands &W, int n, int lane, const int (&l)[4], uint32_t xn) {
+    uint4 r = make_uint4(0, 0, 0, 0);
+    const int x0 = xn > 0 ? l[0] : -1, x1 = xn > 1 ? l[1] : -1, x2 = xn > 2 ? l[2] : -1, x3 = xn > 3 ? l[3] : -1;
+    const bool split = n <= 16;
+    for (int h = 0; h < n; h += 32) {
+        uint32_t sub = 0, sup = 0;
+        const int e = n - h < 32 ? n - h : 32, half = (e + 1) >> 1;
+        const int mEnd = split && lane < 16 ? half : e;
+#pragma unroll 2
+        for (int m = split && lane >= 16 ? half : 0; m < mEnd; m++) {
+            const int4 y = W.leaves[h + m];
+            const uint32_t yn = packed_nleaves((uint32_t)W.rec[h + m].y);
+            uint32_t c = 0;
+            c += (y.x == x0) + (y.x == x1) + (y.x == x2) + (y.x == x3);
+            c += (y.y == x0) + (y.y == x1) + (y.y == x2) + (y.y == x3);
+            c += (y.z == x0) + (y.z == x1) + (y.z == x2) + (y.z == x3);
+            c += (y.w == x0) + (y.w == x1) + (y.w == x2) + (y.w == x3);
+            sub |= (c == yn ? 1u : 0u) << m;
+            sup |= (c == xn && yn > xn ? 1u : 0u) << m;
+        }
+        if (split) {
+            sub |= __shfl_xor_sync(0xffffffffu, sub, 16);
+            sup |= __shfl_xor_sync(0xffffffffu, sup, 16);
+        }
+        if (h == 0)
+            r.x = sub, r.y = sup;
         else
-            inX = (ssign & xs) == ssign && leaves_subset(sl, kn, xl, xn);
+            r.z = sub, r.w = sup;
     }
-    const unsigned C = __ballot_sync(0xffffffffu, clr), D = __ballot_sync(0xffffffffu, inX);
-    const unsigned drop = D ? (C & ((1u << (__ffs(D) - 1)) - 1u)) : C;
-    if ((drop >> lane) & 1u) spk &= ~(1u << 30);
+    // bit 63 stands for the node's trivial cut (candidate 63 has no successor
+    // to compare it with): only an empty cut is related to it
+    r.z &= 0x7FFFFFFFu;
+    r.w = (r.w & 0x7FFFFFFFu) | (xn == 0 ? 1u << 31 : 0u);
+    return r;
+}
+
+// CutFilter (rewrite.cu:178-193) over the slots in `used`, the cuts related
+// to X by r, slot `lane` holding candidate c: visiting the slots in index
+// order, a larger slot containing X is dropped and the first slot contained
+// in X drops X and ends the visit -- so only the supersets before it are
+// dropped.  Returns true when X is dropped.
+__device__ __forceinline__ bool filter_related(uint4 r, int c, uint32_t among, uint32_t &used) {
+    const uint32_t sub = (c & 32) ? r.z : r.x, sup = (c & 32) ? r.w : r.y;
+    const uint32_t D = __ballot_sync(0xffffffffu, (sub >> (c & 31)) & 1u) & among;
+    const uint32_t C = __ballot_sync(0xffffffffu, (sup >> (c & 31)) & 1u) & among;
+    used &= ~(D ? C & ((D & (0u - D)) - 1u) : C);
     return D != 0;
 }
 
-// Fanin slot `lane` of the warp's node, read from the lane holding it.
-__device__ __forceinline__ void fetch_slot(int src, int4 L, int2 M, int2 X, RCut &c, uint32_t &used) {
+// FindCut's order among full slots: class by leaves, then value.
+__device__ __forceinline__ uint32_t slot_key(uint32_t pk) {
+    const uint32_t n = packed_nleaves(pk);
+    return ((n > 2 ? 0u : (n == 2 ? 1u : 2u)) << 20) | (((pk >> 16) & 0x7FFu) << 3);
+}
+
+// Fanin cut record held by lane src.
+__device__ __forceinline__ void fetch_slot(int src, int4 L, int2 M, int2 X, RCut &c) {
     const unsigned F = 0xffffffffu;
     c.l[0] = __shfl_sync(F, L.x, src);
     c.l[1] = __shfl_sync(F, L.y, src);
@@ -208,66 +206,51 @@ __device__ __forceinline__ void fetch_slot(int src, int4 L, int2 M, int2 X, RCut
     c.tt = pk & 0xFFFFu;
     c.n = packed_nleaves(pk);
     c.used = 1;
-    used = packed_used(pk);
     rc_unpack_aux(x0, x1, c);
 }
 
-// Position of the k-th (from 0) set bit of m; m has more than k set bits.
-__device__ __forceinline__ int select_bit64(uint64_t m, int k) {
-    int p = 0;
-#pragma unroll
-    for (int w = 32; w >= 1; w >>= 1) {
-        const int c = __popcll(m & ((1ull << w) - 1ull));
-        const bool up = k >= c;
-        k -= up ? c : 0;
-        m = up ? m >> w : m;
-        p += up ? w : 0;
-    }
-    return p;
-}
-
 // A warp enumerates one node at a time: lanes 0-7 hold u0's cut slots and
-// lanes 8-15 u1's.  The admissible pairs (pair bit i * 8 + j, the
-// reference's i-major order; both slots used, at most four leaves by
-// signature) are found from the slots' signatures first and dealt out in
-// order, the k-th to lane k % 32, so a node with at most 32 of them -- most
-// nodes -- builds its candidates in one round; each lands in shared memory.
-// Then the warp replays
-// CutEnumerate's slot policy over them in order with the node's 8 slots on
-// lanes 0-7 -- FindCut is a min over those lanes, CutFilter two ballots --
-// and lanes 0-7 write the slots.  Same results as the per-thread replay,
-// with a node's latency cut to its sequential core.
-__device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int lane, int4 (*sc)[4]) {
+// lanes 8-15 u1's.  The admissible pairs (pair bit i * 8 + j, the reference's
+// i-major order; both slots used, at most four leaves by signature) are
+// listed in order and dealt out, the k-th to lane k % 32, so a node with at
+// most 32 of them -- most nodes -- builds its candidates in one round.  The
+// lanes then compare their candidates with all earlier ones, which turns
+// CutEnumerate's slot policy, the sequential part, into a few bit operations
+// a pair: slot s on lane s names the candidate it holds, the used slots are
+// a mask in every lane, FindCut is its first clear bit or a min over the
+// slots, CutFilter two ballots of precomputed bits.
+//
+// Bound: the node's latency on a narrow level.  Comparing the leaves inside
+// the policy loop took 0.38 us a pair and the 64x64 multiplier (15 pairs a
+// node, 501 levels) 15.9 us a level.
+__device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int lane, WarpCands &W) {
     const unsigned F = 0xffffffffu;
+    constexpr int kTrivial = 64 + 63;  // the trivial cut's index: bit 63 of the relations
     const int f0 = A.w0[q], f1 = A.w1[q];
     const int u0 = f0 >> 1, u1 = f1 >> 1, c0 = f0 & 1, c1 = f1 & 1;
-    int ok = 1;
-    if (lane == 0) ok = wait_ge(&A.done[u0], 1, A.status) && wait_ge(&A.done[u1], 1, A.status);
-    ok = __shfl_sync(F, ok, 0);
-    __syncwarp();
-    // the node's slots: slot 0 the trivial cut
-    int sl[4] = {0, 0, 0, 0};
-    uint32_t ssign = 0, spk = 0, sa0 = 0, sa1 = 0;
-    if (lane == 0) {
+    int4 sl = make_int4(0, 0, 0, 0), sr = make_int4(0, 0, 0, 0);
+    if (lane == 0) {  // slot 0: the trivial cut
         Cut c;
         c.sign = 1u << A.lidLow[q];
         c.tt = 0xAAAAu;
         c.nLeaves = 1;
         c.used = 1;
         c.value = 1001u;
-        sl[0] = (int)q;
-        ssign = c.sign;
-        spk = cut_pack(c);
-        sa0 = clamp_ref(A.ref[q]);
-        sa1 = (uint32_t)A.lidLow[q] << 12;
+        sl.x = (int)q;
+        sr = make_int4((int)c.sign, (int)cut_pack(c), (int)clamp_ref(A.ref[q]), (int)((uint32_t)A.lidLow[q] << 12));
     }
+    int ok = 1;
+    if (lane < 2) ok = wait_ge(&A.done[lane ? u1 : u0], 1, A.status);
+    ok = __all_sync(F, ok);
+    int held = lane == 0 ? kTrivial : -1;  // candidate in this lane's slot
+    uint32_t used = 1;
     if (ok) {
         int4 L = make_int4(0, 0, 0, 0);
         int2 M = make_int2(0, 0), X = make_int2(0, 0);
         if (lane < 16) {
             const int64_t idx = (int64_t)(lane < 8 ? u0 : u1) * 8 + (lane & 7);
-            L = __ldcg(&A.cutL[idx]);
             M = __ldcg(&A.cutM[idx]);
+            L = __ldcg(&A.cutL[idx]);
             X = __ldcg(&A.cutA[idx]);
         }
         // admissible pairs from the signatures: pair lane (i = lane / 8)
@@ -279,81 +262,102 @@ __device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int
                        pJ = (uint32_t)__shfl_sync(F, M.y, 8 + (lane & 7));
         const bool adm0 = packed_used(pA) && packed_used(pJ) && popc32(sA | sJ) <= 4;
         const bool adm1 = packed_used(pB) && packed_used(pJ) && popc32(sB | sJ) <= 4;
-        const uint64_t pairs = (uint64_t)__ballot_sync(F, adm0) | ((uint64_t)__ballot_sync(F, adm1) << 32);
-        const int nPairs = __popcll(pairs);
-        // candidate k built by lane k % 32, kept in sc[k]
+        const uint32_t b0 = __ballot_sync(F, adm0), b1 = __ballot_sync(F, adm1);
+        const uint32_t below = (1u << lane) - 1u;
+        const int n0 = __popc(b0), nPairs = n0 + __popc(b1);
+        if (adm0) W.pair[__popc(b0 & below)] = (uint8_t)lane;
+        if (adm1) W.pair[n0 + __popc(b1 & below)] = (uint8_t)(lane + 32);
+        __syncwarp();
+        // candidate k built by lane k % 32; merged cuts of both rounds kept
+        // until every final cut is in shared memory
+        int ml[2][4];
+        uint32_t mn[2] = {0, 0}, flags[2] = {0, 0};  // flags: 1 merged, 2 minimised, 4 fewer than two leaves
 #pragma unroll
         for (int r = 0; r < 2; r++) {
             if (r * 32 >= nPairs) break;
-            const int k = r * 32 + lane;
-            const int p = k < nPairs ? select_bit64(pairs, k) : 0;
-            RCut a, b;
-            uint32_t ua, ub;
-            fetch_slot(p >> 3, L, M, X, a, ua);
-            fetch_slot(8 + (p & 7), L, M, X, b, ub);
-            if (k < nPairs) {
-                Cand c;
-                make_cand(a, b, c0, c1, c);
-                put_cand(sc[k], c);
+            const int k = r * 32 + (nPairs <= 16 ? lane & 15 : lane);
+            const int p = W.pair[k < nPairs ? k : 0];
+            RCut a, b, m;
+            fetch_slot(p >> 3, L, M, X, a);
+            fetch_slot(8 + (p & 7), L, M, X, b);
+            int pa, pb;
+            const bool merged = rc_merge(a, b, m, pa, pb);
+#pragma unroll
+            for (int i = 0; i < 4; i++) ml[r][i] = m.l[i];
+            mn[r] = m.n;
+            m.tt = rc_truth(a, b, c0, c1, pa, pb);
+            const bool mini = rc_minimize(m);
+            if (k < nPairs && (nPairs > 16 || lane < 16)) {
+                flags[r] = (merged ? 1u : 0u) | (mini ? 2u : 0u) | (m.n < 2 ? 4u : 0u);
+                Cut pc;
+                pc.tt = m.tt;
+                pc.nLeaves = m.n;
+                pc.used = 1;
+                pc.value = rc_value(m);
+                uint32_t x0, x1;
+                rc_pack_aux(m, x0, x1);
+                W.leaves[k] = make_int4(m.n > 0 ? m.l[0] : 0, m.n > 1 ? m.l[1] : 0, m.n > 2 ? m.l[2] : 0,
+                                        m.n > 3 ? m.l[3] : 0);
+                W.rec[k] = make_int4((int)m.sign, (int)cut_pack(pc), (int)x0, (int)x1);
             }
         }
         __syncwarp();
+        uint64_t merged = 0, mini = 0, stop = 0;
+#pragma unroll
+        for (int r = 0; r < 2; r++) {
+            if (r * 32 >= nPairs) break;
+            const int k = r * 32 + (nPairs <= 16 ? lane & 15 : lane), n = r == 0 && nPairs > 32 ? 32 : nPairs;
+            const uint4 rel = relate(W, n, lane, ml[r], mn[r]);
+            if (k < nPairs) W.rel[k] = rel;
+            merged |= (uint64_t)__ballot_sync(F, flags[r] & 1u) << (r * 32);
+            const uint32_t mm = __ballot_sync(F, (flags[r] & 3u) == 3u);
+            stop |= (uint64_t)__ballot_sync(F, flags[r] & 4u) << (r * 32);
+            if (mm) {
+                const int4 y = W.leaves[k < nPairs ? k : 0];
+                const int yl[4] = {y.x, y.y, y.z, y.w};
+                const uint4 rm = relate(W, n, lane, yl, packed_nleaves((uint32_t)W.rec[k < nPairs ? k : 0].y));
+                if (k < nPairs) W.relMin[k] = rm;
+                mini |= (uint64_t)mm << (r * 32);
+            }
+        }
+        __syncwarp();
+        // the slot policy, pair by pair
+        uint32_t key = lane < 8 ? slot_key((uint32_t)sr.y) | (uint32_t)lane : 0xFFFFFFFFu;
         int k = 0;
         for (; k < nPairs; k++) {
-            Cand m;
-            get_cand(sc[k], m);
+            const uint4 rel = W.rel[k];
+            const uint32_t pk = (uint32_t)W.rec[k].y;
             // FindCut (rewrite.cu:84-109): the first free slot, else the
-            // lowest (class, value, index); both computed, one kept
-            const unsigned freeSlots = __ballot_sync(F, lane < 8 && !packed_used(spk)) & 0xFFu;
-            uint32_t key = 0xFFFFFFFFu;
-            if (lane < 8) {
-                const uint32_t n = packed_nleaves(spk);
-                const uint32_t cls = n > 2 ? 0u : (n == 2 ? 1u : 2u);
-                key = (cls << 20) | (((spk >> 16) & 0x7FFu) << 3) | (uint32_t)lane;
-            }
-            const uint32_t lowest = __reduce_min_sync(F, key);
-            const int id = freeSlots ? __ffs(freeSlots) - 1 : (int)(lowest & 7u);
-            if (lane == id) spk &= ~(1u << 30);
-            if (!m.ok) continue;
-            const int xl[4] = {m.x0, m.x1, m.x2, m.x3};
-            if (warp_filter(lane, id, sl, ssign, spk, xl, m.xn, m.xs)) continue;  // slot stays free
-            Cut pc;
-            pc.tt = m.ytt;
-            pc.nLeaves = m.yn;
-            pc.used = 1;
-            pc.value = 0;
+            // lowest (class, value, index)
+            const uint32_t freeSlots = ~used & 0xFFu;
+            const int id = freeSlots ? __ffs(freeSlots) - 1 : (int)(__reduce_min_sync(F, key) & 7u);
+            used &= ~(1u << id);
+            if (!((merged >> k) & 1u)) continue;
+            if (filter_related(rel, held, used, used)) continue;  // the slot stays free
             if (lane == id) {
-                sl[0] = m.y0;
-                sl[1] = m.y1;
-                sl[2] = m.y2;
-                sl[3] = m.y3;
-                ssign = m.ys;
-                spk = cut_pack(pc);
-                sa0 = m.a0;
-                sa1 = m.a1;
+                held = k;
+                key = slot_key(pk) | (uint32_t)lane;
             }
-            bool keep = true;
-            if (m.mini) {
-                const int yl[4] = {m.y0, m.y1, m.y2, m.y3};
-                keep = !warp_filter(lane, id, sl, ssign, spk, yl, m.yn, m.ys);
-            }
-            pc.value = m.yval;
-            pc.used = keep ? 1u : 0u;
-            if (lane == id) spk = cut_pack(pc);
-            if (m.yn < 2) {  // enumeration of this node stops (rewrite.cu:291)
+            bool drop = false;
+            if ((mini >> k) & 1u) drop = filter_related(W.relMin[k], held, used, used);
+            if (!drop) used |= 1u << id;
+            if ((stop >> k) & 1u) {  // enumeration of this node stops (rewrite.cu:291)
                 k++;
                 break;
             }
         }
         if (lane == 0 && k > 0) atomicAdd(A.warpPairs, (unsigned long long)k);  // pairs replayed
+        if (held >= 0 && held != kTrivial) sl = W.leaves[held], sr = W.rec[held];
     }
     if (lane < 8) {
-        A.cutL[q * 8 + lane] = make_int4(sl[0], sl[1], sl[2], sl[3]);
-        A.cutM[q * 8 + lane] = make_int2((int)ssign, (int)spk);
-        A.cutA[q * 8 + lane] = make_int2((int)sa0, (int)sa1);
-        __threadfence();
+        if (!((used >> lane) & 1u)) sr.y &= ~(1 << 30);
+        A.cutL[q * 8 + lane] = sl;
+        A.cutM[q * 8 + lane] = make_int2(sr.x, sr.y);
+        A.cutA[q * 8 + lane] = make_int2(sr.z, sr.w);
     }
-    __syncwarp();  // also: every lane is done reading sc before the next node overwrites it
+    // orders the lanes' stores before lane 0's release, which publishes them;
+    // also: every lane is done reading W before the next node overwrites it
+    __syncwarp();
     if (lane == 0) st_release(&A.done[q], 1);
 }
 
@@ -444,9 +448,10 @@ __device__ __forceinline__ void enum_node_thread(const EnumArgs &A, int64_t q, b
                 for (int k = 0; k < 8; k++)
                     if (k == id) sl_clear_used(S[k]);
                 RCut m;
-                if (!rc_merge(a, b, m)) continue;
+                int pa, pb;
+                if (!rc_merge(a, b, m, pa, pb)) continue;
                 if (filter_slots(S, id, m.l, m.n, m.sign)) continue;  // dropped: slot stays free
-                m.tt = rc_truth(m, a, b, c0, c1);
+                m.tt = rc_truth(a, b, c0, c1, pa, pb);
                 const bool mini = rc_minimize(m);
                 m.value = 0;
                 Cut pc;
@@ -485,7 +490,6 @@ __device__ __forceinline__ void enum_node_thread(const EnumArgs &A, int64_t q, b
         A.cutL[q * 8 + k] = make_int4(S[k].l[0], S[k].l[1], S[k].l[2], S[k].l[3]);
         A.cutM[q * 8 + k] = make_int2((int)S[k].sign, (int)S[k].pk);
     }
-    __threadfence();
     st_release(&A.done[q], 1);
 }
 
@@ -495,7 +499,7 @@ __device__ __forceinline__ void enum_node_thread(const EnumArgs &A, int64_t q, b
 // time is the time of its slowest node).  Warps claim chunks in level
 // order, so every fanin of a claimed node lies in an earlier, claimed chunk.
 __global__ void __launch_bounds__(kEnumBlock, 4) k_enumerate(EnumArgs A) {
-    __shared__ int4 s_cand[kEnumBlock / 32][64][4];
+    __shared__ WarpCands s_cand[kEnumBlock / 32];
     const unsigned F = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int total = A.chunkStart[A.maxLevel + 1];
