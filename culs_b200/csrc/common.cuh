@@ -174,6 +174,28 @@ CULS_HD bool wait_word(const int *w, int floor, int *status, int *val) {
     }
 }
 
+// wait_word for two words at once, so that their round trips overlap.
+CULS_HD bool wait_words(const int *w0, const int *w1, int floor, int *status, int *v0, int *v1) {
+    int a = ld_relaxed(w0), b = ld_relaxed(w1);
+    if (a < floor || b < floor) {
+        const int64_t lim = spin_limit(status);
+        for (int64_t it = 1;; ++it) {
+            if ((it & 31) == 1 && ld_cg(status) != kDevOk) return false;
+            if (it >= lim) {
+                set_status(status, kDevWaitTimeout);
+                return false;
+            }
+            backoff(it);
+            a = ld_relaxed(w0);
+            b = ld_relaxed(w1);
+            if (a >= floor && b >= floor) break;
+        }
+    }
+    *v0 = a;
+    *v1 = b;
+    return true;
+}
+
 // MurmurHash3 64-bit finalizer (public domain, Austin Appleby).
 CULS_HD uint64_t mix64(uint64_t x) {
     x ^= x >> 33;

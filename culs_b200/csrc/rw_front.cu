@@ -13,6 +13,7 @@
 //    together with the PO references.
 #include <algorithm>
 
+#include "levels.cuh"
 #include "rw_work.cuh"
 #include "sched.cuh"
 
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(kBlock) k_front_levelize(ChunkSched S, const i
         int f0 = a0[p], f1 = a1[p];
         int u0 = f0 >> 1, u1 = f1 >> 1;
         int x0, x1;
-        if (!wait_word(&lp[u0], 0, status, &x0) || !wait_word(&lp[u1], 0, status, &x1)) continue;
+        if (!wait_words(&lp[u0], &lp[u1], 0, status, &x0, &x1)) continue;
         int lv = 1 + max(x0 >> 1, x1 >> 1);
         int ph = ((x0 & 1) ^ (f0 & 1)) & ((x1 & 1) ^ (f1 & 1));
         st_relaxed(&lp[p], 2 * lv + ph);
@@ -190,15 +191,24 @@ int rw_front(ExecCtx &X, Batch &b, RwWork &w) {
     int *cnt = X.counters;
     int rc;
     if ((rc = X.check(cudaMemsetAsync(cnt, 0, sizeof(int) * 8, s), "memset"))) return rc;
-    ChunkSched sched;
-    if ((rc = build_chunk_sched(X, b, kBlock, sched))) return rc;
     k_front_load<<<X.grid(N), kBlock, 0, s>>>(N, G, b.dg, b.F0, b.F1, gidIn, a0, a1, lp);
-    k_front_levelize<<<flow_blocks(w.width, kBlock, (unsigned)(X.sms * 8), X.sms), kBlock, 0, s>>>(sched, a0, a1, lp, cnt + 0, cnt + 1, X.status);
+    if (G == 1 && N <= kLevelsBlockMax) {
+        LevelsArgs A;
+        A.n = N, A.a0 = a0, A.a1 = a1, A.pre = lp, A.levelPhase = lp;
+        A.depth0 = cnt + 1, A.unsettled = cnt + 2, A.status = X.status;
+        if ((rc = X.check(levels_block(A, s), "levels"))) return rc;
+    } else {
+        ChunkSched sched;
+        if ((rc = build_chunk_sched(X, b, kBlock, sched))) return rc;
+        k_front_levelize<<<flow_blocks(w.width, kBlock, (unsigned)(X.sms * 8), X.sms), kBlock, 0, s>>>(
+            sched, a0, a1, lp, cnt + 0, cnt + 1, X.status);
+    }
     k_front_keys<<<X.grid(N), kBlock, 0, s>>>(N, lp, keys, vals);
     X.launched(3);
     if ((rc = X.check(cudaMemcpyAsync(X.hostSmall, cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h"))) return rc;
     if ((rc = X.sync())) return rc;
     if ((rc = X.status_check("rw levelize"))) return rc;
+    if (X.hostSmall[2]) return X.fail(CULS_E_INVALID, "rw levelize: fanins do not precede their node");
     w.maxLevel = X.hostSmall[1];
     int bits = 1;
     while ((1ll << bits) <= w.maxLevel) bits++;

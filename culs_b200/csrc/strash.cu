@@ -29,6 +29,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "levels.cuh"
 #include "rw_work.cuh"
 #include "sched.cuh"
 
@@ -181,6 +182,7 @@ __global__ void __launch_bounds__(kBlock) k_level_step(int L, int *items, int *r
     }
 }
 
+// done: 0 until an AND node's level is known, then level + 1
 __global__ void k_live_flags(int64_t M, const int *L0, const uint8_t *dead, uint8_t *liveFlag, int *done) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < M; v += stride) {
@@ -193,9 +195,8 @@ __global__ void k_live_flags(int64_t M, const int *L0, const uint8_t *dead, uint
 // Levels of a graph-major batch whose positions are topological (`st`):
 // the in-order dataflow of the rw front over the interleaved chunk schedule
 // (sched.cuh), instead of a worklist over a fanout CSR.  Every AND node gets
-// its ASAP level; only live nodes count towards a graph's depth.  An AND
-// node publishes its level (>= 1) in done[], the one word its fanouts wait
-// on and read.
+// its ASAP level; only live nodes count towards a graph's depth.  A node's
+// level + 1 in done[] is the one word its fanouts wait on and read.
 __global__ void __launch_bounds__(kBlock) k_st_levelize(ChunkSched S, const int *L0, const int *L1,
                                                          const uint8_t *liveFlag, const int *gid, int *level,
                                                          int *done, int *graphLevels, int *counter, int *maxLevel,
@@ -220,11 +221,10 @@ __global__ void __launch_bounds__(kBlock) k_st_levelize(ChunkSched S, const int 
         const int a = L0[p];
         if (a < 0) continue;  // constant or PI: level 0, done preset
         const int u0 = a >> 1, u1 = L1[p] >> 1;
-        int l0 = 0, l1 = 0;
-        if (L0[u0] >= 0 && !wait_word(&done[u0], 1, status, &l0)) continue;
-        if (L0[u1] >= 0 && !wait_word(&done[u1], 1, status, &l1)) continue;
-        const int lv = 1 + (l0 > l1 ? l0 : l1);
-        st_relaxed(&done[p], lv);
+        int d0, d1;
+        if (!wait_words(&done[u0], &done[u1], 1, status, &d0, &d1)) continue;
+        const int lv = d0 > d1 ? d0 : d1;
+        st_relaxed(&done[p], lv + 1);
         __stcg(&level[p], lv);
         if (liveFlag[p]) {
             agg_max(graphLevels, gid[p], lv);
@@ -295,6 +295,24 @@ __global__ void __launch_bounds__(kBlock) k_order_levelize(int64_t n, const int 
     }
     myMax = __reduce_max_sync(0xffffffffu, myMax);
     if ((threadIdx.x & 31) == 0 && myMax > 0) atomicMax(maxLevel, myMax);
+}
+
+// The same order as levels_block takes it: order index k's fanins as literals
+// over order indexes.
+__global__ void k_order_fanins(int64_t n, const int *list, const int *posOf, const int *L0, const int *L1,
+                               const uint8_t *liveFlag, int *a0, int *a1) {
+    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += stride) {
+        const int v = list[k];
+        const int a = v >= 0 ? L0[v] : 0;
+        if (v < 0 || a < 0 || !liveFlag[v]) {
+            a0[k] = v >= 0 && a < 0 ? kLevelZero : kLevelSkip;
+            continue;
+        }
+        const int b = L1[v];
+        a0[k] = 2 * posOf[a >> 1] + (a & 1);
+        a1[k] = 2 * posOf[b >> 1] + (b & 1);
+    }
 }
 
 __global__ void k_unresolved_flags(int64_t n, const int *list, const int *done, uint8_t *flag) {
@@ -698,17 +716,25 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         int *done = pending;  // reuse
         if (!liveIdx) return fail(CULS_E_OOM, "strash: scratch arena exhausted");
         ExecCtx X = ctx();
+        const bool inBlock = G == 1 && M <= kLevelsBlockMax;
         ChunkSched sched;
         int rc;
-        if ((rc = build_chunk_sched(X, b, kBlock, sched))) return rc;
+        if (!inBlock && (rc = build_chunk_sched(X, b, kBlock, sched))) return rc;
         check(cudaMemsetAsync(qc, 0, sizeof(int) * 8, s), "memset");
         check(cudaMemsetAsync(graphLevels, 0, sizeof(int) * (G + 1), s), "memset");
         check(cudaMemsetAsync(level, 0, sizeof(int) * (M + 1), s), "memset");
         k_live_flags<<<gridM, kBlock, 0, s>>>(M, L0, dead, liveFlag, done);
         check(compact_flags(liveFlag, M, liveIdx, qc + 3, ar_, s), "compact");  // live list and count
         if (prof_) this->mark(kMkLevelK0);
-        k_st_levelize<<<gridQ, kBlock, 0, s>>>(sched, L0, L1, liveFlag, gidA, level, done, graphLevels, qc + 5,
-                                               qc + 4, status_);
+        if (inBlock) {
+            LevelsArgs A;
+            A.n = M, A.a0 = L0, A.a1 = L1, A.level = level, A.counted = liveFlag;
+            A.depth0 = qc + 4, A.depth1 = graphLevels, A.unsettled = qc + 6, A.status = status_;
+            if ((rc = check(levels_block(A, s), "levels"))) return rc;
+        } else {
+            k_st_levelize<<<gridQ, kBlock, 0, s>>>(sched, L0, L1, liveFlag, gidA, level, done, graphLevels, qc + 5,
+                                                   qc + 4, status_);
+        }
         if (prof_) this->mark(kMkLevelK1);
         launches_ += 2;
     } else {
@@ -733,6 +759,18 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         if (prof_) this->mark(kMkLevelK0);
         const int *list = procInv;
         int64_t n = M;
+        if (G == 1 && M <= kLevelsBlockMax) {
+            int *a0 = cnt, *a1 = off;
+            k_order_fanins<<<gridM, kBlock, 0, s>>>(M, procInv, procPos, L0, L1, liveFlag, a0, a1);
+            LevelsArgs A;
+            A.n = M, A.a0 = a0, A.a1 = a1, A.posOf = procInv, A.level = level;
+            A.depth0 = qc + 4, A.depth1 = graphLevels, A.unsettled = qc + 6, A.status = qc + 7;
+            check(levels_block(A, s), "levels");
+            launches_ += 2;
+            check(cudaMemcpyAsync(hostSmall_, qc, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h");
+            if (int e = sync()) return e;
+            leveled = hostSmall_[6] == 0 && hostSmall_[7] == 0;
+        } else
         for (int pass = 0; pass < 64; pass++) {
             check(cudaMemsetAsync(qc + 5, 0, sizeof(int), s), "memset");
             k_order_levelize<<<gridQ, kBlock, 0, s>>>(n, list, procPos, L0, L1, liveFlag, gidA, level, done,
@@ -806,6 +844,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     if (int e = check_status("strash levels")) return e;
     int64_t nLive = hostSmall_[3];
     int maxLevel = hostSmall_[4];
+    if (topo && hostSmall_[6]) return fail(CULS_E_INVALID, "strash: fanins do not precede their node");
     if (!topo && hostSmall_[1] != nLive) return fail(CULS_E_INVALID, "strash: the AIG has a cycle");
     int *srt = ar_.get<int>(nLive + 1);
     uint32_t *keys = ar_.get<uint32_t>(nLive + 1);
