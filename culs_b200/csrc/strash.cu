@@ -497,30 +497,51 @@ __global__ void __launch_bounds__(kDedupChunk) k_dedup(DedupArgs A) {
 // The mapping k_dedup computes is the unique fixed point of one parallel
 // step: a node's key is its fanins' mapped literals (folded when trivial),
 // and it maps to the position of the lowest-ranked live node with the same
-// key.  (By induction over the levels: a node's key reads only lower
-// levels, so any fixed point equals the level-by-level result.)  Starting
-// from the identity, round r makes every node of level <= r final, and the
-// rounds stop at the first one that changes nothing -- after one round when
-// nothing merges, after a few when merges cascade, since a node's key
-// changes only when a fanin's mapping did.  Each round is two passes over
-// the live nodes with no dependency waits, so a deep, narrow graph costs a
-// few launches instead of one wait latency per level.
-
+// key.  (By induction over the levels: a node's key reads only lower levels,
+// so any fixed point equals the level-by-level result.)  Starting from the
+// identity, the first round keys and maps every node; a later round keys only
+// the nodes with a fanin whose mapping changed, and maps again only the nodes
+// of slots that received a key.  No thread waits on another, so a deep,
+// narrow graph costs a few launches instead of one wait latency per level.
+//
+// Keys a node had earlier stay in the table.  They do no harm: mappings are
+// equivalences that only grow (two nodes with equal keys under a part of the
+// final equivalence are equal under all of it), so every node ever inserted
+// with what is a final key has that key in the end, and a slot's lowest rank
+// is its lowest final member's.  For the same reason the mappings may be
+// read and written in place: a reader of an older one is visited again in
+// the round after.
+//
+// A round over all nodes moves their keys and table sectors (9.5M nodes: 1.1
+// ms, and merges cascade for 15 rounds on a 256-graph batch); a later round
+// reads their fanins and two bits each (0.15 ms).  That batch's
+// deduplication: 19.9 -> 6.6 ms; 2,000 graphs of up to 2,000 ANDs (14
+// rounds): 2.7 -> 1.75 ms.
 struct RoundArgs {
-    int64_t nLive;
-    const int *srt, *rankOf;
+    int64_t nLive, M;
+    const int *srt, *tOf, *rankOf;
+    const uint8_t *liveFlag;
     const int *L0, *L1;
     const int *gid;
     const DevGraph *dg;
     AndTable tab;
-    const int *cur;  // per position: the literal an AND node maps to this round
-    int *nxt;        // the same after this round
-    int *slotT;      // per processing index: table slot, -1 when folded
+    int *cur;    // per position: the literal an AND node maps to
+    int *slotT;  // per processing index: table slot, -1 when folded
     int *mapEnc, *kl0, *kl1;
     int foldTrivial, unique;
+    const uint32_t *chIn;  // per position: mapping changed in the round before
+    uint32_t *chOut;       //   in this round
+    uint32_t *slotBits;    // per slot: received a key in this round
+    const int *prev;       // whether the round before changed anything (null: first round)
     int *changed;
+    int *inserted;         // keys inserted by later rounds, at most `room`
+    int room;
+    int *full;             // a later round ran out of room: start again from all nodes
     int *status;
 };
+
+__device__ __forceinline__ bool bit_at(const uint32_t *b, int i) { return (b[i >> 5] >> (i & 31)) & 1u; }
+__device__ __forceinline__ void set_bit(uint32_t *b, int i) { atomicOr(&b[i >> 5], 1u << (i & 31)); }
 
 __global__ void k_round_init(int64_t n, const int *srt, int *cur) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -530,65 +551,112 @@ __global__ void k_round_init(int64_t n, const int *srt, int *cur) {
     }
 }
 
-// keys from this round's mapping: fold (as k_dedup does) or insert
+__device__ __forceinline__ void round_map(const RoundArgs &A, int v, int lit) {
+    if (A.cur[v] == lit) return;
+    A.cur[v] = lit;
+    set_bit(A.chOut, v);
+    *A.changed = 1;
+}
+
+// Node v's key from the current mappings, folded as k_dedup does: returns the
+// literal it folds to, or -1 with the key's literals in l0 <= l1.
+__device__ __forceinline__ int round_key(const RoundArgs &A, int v, int &l0, int &l1) {
+    l0 = A.L0[v], l1 = A.L1[v];
+    if (A.L0[l0 >> 1] >= 0) l0 = A.cur[l0 >> 1] ^ (l0 & 1);
+    if (A.L0[l1 >> 1] >= 0) l1 = A.cur[l1 >> 1] ^ (l1 & 1);
+    if (l0 > l1) {
+        const int x = l0;
+        l0 = l1;
+        l1 = x;
+    }
+    if (!A.foldTrivial) return -1;
+    const int T = 2 * A.dg[A.gid[v]].cpos;  // AIGMan: constant TRUE
+    const int F = T + 1;
+    if (l0 == l1) return l0;
+    if (l0 == (l1 ^ 1)) return F;
+    if (l0 == T) return l1;
+    if (l1 == T) return l0;
+    if (l0 == F || l1 == F) return F;
+    return -1;
+}
+
+__device__ __forceinline__ int round_insert(const RoundArgs &A, int v, int t, int l0, int l1) {
+    const unsigned long long key = A.unique ? (1ull << 63) | (unsigned long long)(uint32_t)v
+                                            : ((unsigned long long)(uint32_t)l0 << 32) | (uint32_t)l1;
+    const int slot = table_insert(A.tab, key, A.rankOf[v], v, A.status);
+    A.kl0[t] = l0;
+    A.kl1[t] = l1;
+    A.mapEnc[v] = slot >= 0 ? -(slot + 1) : 0;
+    A.slotT[t] = slot;
+    return slot;
+}
+
+// first round: every node's key
 __global__ void k_round_insert(RoundArgs A) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < A.nLive; t += stride) {
         const int v = A.srt[t];
-        int lits[2] = {A.L0[v], A.L1[v]};
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const int u = lits[k] >> 1;
-            if (A.L0[u] >= 0) lits[k] = A.cur[u] ^ (lits[k] & 1);
-        }
-        int l0 = lits[0], l1 = lits[1];
-        if (l0 > l1) {
-            const int x = l0;
-            l0 = l1;
-            l1 = x;
-        }
-        const int T = 2 * A.dg[A.gid[v]].cpos;  // AIGMan: constant TRUE
-        const int F = T + 1;
-        int triv = -1;
-        if (A.foldTrivial) {
-            if (l0 == l1)
-                triv = l0;
-            else if (l0 == (l1 ^ 1))
-                triv = F;
-            else if (l0 == T)
-                triv = l1;
-            else if (l1 == T)
-                triv = l0;
-            else if (l0 == F || l1 == F)
-                triv = F;
-        }
+        int l0, l1;
+        const int triv = round_key(A, v, l0, l1);
         if (triv >= 0) {
             A.mapEnc[v] = triv;
-            A.nxt[v] = triv;
             A.slotT[t] = -1;
-            if (triv != A.cur[v]) *A.changed = 1;
+            round_map(A, v, triv);
         } else {
-            const unsigned long long key = A.unique ? (1ull << 63) | (unsigned long long)(uint32_t)v
-                                                    : ((unsigned long long)(uint32_t)l0 << 32) | (uint32_t)l1;
-            const int slot = table_insert(A.tab, key, A.rankOf[v], v, A.status);
-            A.kl0[t] = l0;
-            A.kl1[t] = l1;
-            A.mapEnc[v] = slot >= 0 ? -(slot + 1) : 0;
-            A.slotT[t] = slot;
+            round_insert(A, v, (int)t, l0, l1);
         }
     }
 }
 
-// every key's lowest rank is known: the inserted nodes map to its position
+// first round: every key's lowest rank is known, and the inserted nodes map
+// to its position
 __global__ void k_round_resolve(RoundArgs A) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < A.nLive; t += stride) {
         const int slot = A.slotT[t];
-        if (slot < 0) continue;
-        const int v = A.srt[t];
-        const int m = 2 * slot_pos(A.tab.slots[slot].rp);
-        A.nxt[v] = m;
-        if (m != A.cur[v]) *A.changed = 1;
+        if (slot >= 0) round_map(A, A.srt[t], 2 * slot_pos(A.tab.slots[slot].rp));
+    }
+}
+
+// later round: new keys of the nodes with a fanin that maps elsewhere now
+__global__ void k_round_rekey(RoundArgs A) {
+    if (*A.prev == 0) return;
+    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < A.M; p += stride) {
+        const int v = (int)p, a = A.L0[v];
+        if (a < 0) continue;
+        const int b = A.L1[v];
+        if (!bit_at(A.chIn, a >> 1) && !bit_at(A.chIn, b >> 1)) continue;
+        if (!A.liveFlag[v]) continue;
+        const int t = A.tOf[v];
+        int l0, l1;
+        const int triv = round_key(A, v, l0, l1);
+        if (triv >= 0) {
+            A.mapEnc[v] = triv;
+            A.slotT[t] = -1;
+            round_map(A, v, triv);
+        } else if (A.slotT[t] < 0 || A.kl0[t] != l0 || A.kl1[t] != l1) {
+            const unsigned m = __activemask();
+            const int lane = threadIdx.x & 31, lead = __ffs(m) - 1;
+            int at = 0;
+            if (lane == lead) at = atomicAdd(A.inserted, __popc(m));
+            if (__shfl_sync(m, at, lead) + __popc(m) > A.room) {
+                *A.full = 1;
+                continue;
+            }
+            const int slot = round_insert(A, v, t, l0, l1);
+            if (slot >= 0) set_bit(A.slotBits, slot);
+        }
+    }
+}
+
+// later round: the nodes of the slots that received a key
+__global__ void k_round_remap(RoundArgs A) {
+    if (*A.prev == 0) return;
+    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < A.nLive; t += stride) {
+        const int slot = A.slotT[t];
+        if (slot >= 0 && bit_at(A.slotBits, slot)) round_map(A, A.srt[t], 2 * slot_pos(A.tab.slots[slot].rp));
     }
 }
 
@@ -898,15 +966,15 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     int *wl = ar_.get<int>(nLive + 1);
     if (!ts || !mapEnc || !kl0 || !kl1 || !wflags || !wl) return fail(CULS_E_OOM, "strash: arena exhausted");
     check(cudaMemsetAsync(qc + 5, 0, sizeof(int), s), "memset");
-    // Rounds (k_round_*) for batches of up to 16M live nodes, where a few
-    // full passes cost less than one wait latency per level (the 10M-AND
-    // single graph: each strash 22 -> 6 ms); the level dataflow (k_dedup)
-    // for larger ones, whose rounds each move gigabytes and whose merges
-    // can cascade for many rounds, and whenever the rounds do not settle
-    // within kMaxRounds.  CULS_DEDUP_MODE=levels|rounds forces either
+    // Rounds (k_round_*) for batches of up to 16M live nodes, where a full
+    // pass and a few light ones cost less than one wait latency per level
+    // (the 10M-AND single graph: each strash 22 -> 6 ms); the level dataflow
+    // (k_dedup) for larger ones, whose rounds each move gigabytes and whose
+    // merges can cascade for many rounds, and whenever the rounds do not
+    // settle within kMaxRounds.  CULS_DEDUP_MODE=levels|rounds forces either
     // (the tests run both on the same graphs).
     constexpr int64_t kRoundsMaxLive = 16ll << 20;
-    constexpr int kMaxRounds = 24;
+    constexpr int kMaxRounds = 64;
     bool useRounds = nLive > 0 && nLive <= kRoundsMaxLive;
     if (const char *env = getenv("CULS_DEDUP_MODE")) {
         if (!strcmp(env, "levels")) useRounds = false;
@@ -917,29 +985,52 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     int *slotT = ar_.get<int>(nLive + 1);
     if (!slotT) return fail(CULS_E_OOM, "strash: arena exhausted");
     if (useRounds) {
-        int *cur = ar_.get<int>(M + 1), *nxt = ar_.get<int>(M + 1);
-        if (!cur || !nxt) return fail(CULS_E_OOM, "strash: arena exhausted");
+        int *cur = ar_.get<int>(M + 1), *flag = ar_.get<int>(kMaxRounds + 2);  // changed per round; inserted, full
+        const size_t posWords = (size_t)M / 32 + 1, slotWords = (size_t)cap / 32 + 1;
+        uint32_t *ch[2] = {ar_.get<uint32_t>(posWords), ar_.get<uint32_t>(posWords)};
+        uint32_t *slotBits = ar_.get<uint32_t>(slotWords);
+        if (!cur || !flag || !ch[0] || !ch[1] || !slotBits) return fail(CULS_E_OOM, "strash: arena exhausted");
         const unsigned gl = grid_1d(nLive, kBlock, sms_ * 16);
         if (prof_) this->mark(kMkDedupK0);
         k_round_init<<<gl, kBlock, 0, s>>>(nLive, srt, cur);
         launches_ += 1;
-        for (int r = 0; r < kMaxRounds; r++) {
-            check(and_table_clear(ts, cap, s), "fill");
-            check(cudaMemsetAsync(qc + 16, 0, sizeof(int), s), "memset");
-            RoundArgs R{nLive,  srt,   rankOf, L0, L1, gidA, b.dg, AndTable{ts, cap - 1},
-                        cur,    nxt,   slotT,  mapEnc, kl0, kl1, foldTrivial ? 1 : 0, unique ? 1 : 0, qc + 16, status_};
-            k_round_insert<<<gl, kBlock, 0, s>>>(R);
-            k_round_resolve<<<gl, kBlock, 0, s>>>(R);
-            launches_ += 2;
-            check(cudaMemcpyAsync(hostSmall_ + 16, qc + 16, sizeof(int), cudaMemcpyDeviceToHost, s), "d2h");
+        RoundArgs R{nLive, M,   srt,    tOf, rankOf, liveFlag, L0, L1, gidA, b.dg, AndTable{ts, cap - 1}, cur, slotT,
+                    mapEnc, kl0, kl1,   foldTrivial ? 1 : 0, unique ? 1 : 0, nullptr, nullptr, slotBits, nullptr, nullptr,
+                    flag + kMaxRounds, (int)(cap / 4), flag + kMaxRounds + 1, status_};
+        check(cudaMemsetAsync(flag, 0, sizeof(int) * (kMaxRounds + 2), s), "memset");
+        bool all = true;  // the next round takes all nodes
+        for (int r = 0; r < kMaxRounds && !settled;) {
+            // all nodes: one round; later rounds three at a time (one that
+            // follows a round without a change does nothing)
+            const int first = r, last = all ? r + 1 : std::min(r + 3, kMaxRounds);
+            for (; r < last; r++) {
+                R.chIn = ch[(r + 1) & 1], R.chOut = ch[r & 1];
+                R.prev = r > 0 ? flag + r - 1 : nullptr;
+                R.changed = flag + r;
+                check(cudaMemsetAsync(R.chOut, 0, sizeof(uint32_t) * posWords, s), "memset");
+                if (all) {
+                    check(and_table_clear(ts, cap, s), "fill");
+                    check(cudaMemsetAsync(R.inserted, 0, sizeof(int) * 2, s), "memset");
+                    k_round_insert<<<gl, kBlock, 0, s>>>(R);
+                    k_round_resolve<<<gl, kBlock, 0, s>>>(R);
+                } else {
+                    check(cudaMemsetAsync(slotBits, 0, sizeof(uint32_t) * slotWords, s), "memset");
+                    k_round_rekey<<<gridM, kBlock, 0, s>>>(R);
+                    k_round_remap<<<gl, kBlock, 0, s>>>(R);
+                }
+                launches_ += 2;
+            }
+            check(cudaMemcpyAsync(hostSmall_ + 8, flag + first, sizeof(int) * (last - first), cudaMemcpyDeviceToHost, s),
+                  "d2h");
+            check(cudaMemcpyAsync(hostSmall_ + 16, R.full, sizeof(int), cudaMemcpyDeviceToHost, s), "d2h");
             if (int e = sync()) return e;
             if (int e = check_status("strash hashing")) return e;
-            std::swap(cur, nxt);
-            if (hostSmall_[16] == 0) {
-                settled = true;
-                hashRounds_ = r + 1;
-                break;
-            }
+            all = hostSmall_[16] != 0;
+            for (int k = first; k < last && !settled && !all; k++)
+                if (hostSmall_[8 + k - first] == 0) {
+                    settled = true;
+                    hashRounds_ = k + 1;
+                }
         }
         if (prof_) this->mark(kMkDedupK1);
     }
