@@ -232,8 +232,8 @@ class Engine {
     int ensure_arena(size_t bytes);
     int ensure_stage(size_t ints);  // pinned host staging of at least `ints` int32
     ExecCtx ctx();
-    int balance_graph(const int *F0, const int *F1, const int *PO, int nPIs, int nPO, int nObj, int *F0n, int *F1n,
-                      int *POn, int *nAndsOut);
+    // balances graphs [ga, gb) of b into its spare buffers (balance.cu)
+    int balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> &ng);
     void apply_spin_limit();
 
     // stage helpers

@@ -1,0 +1,91 @@
+"""The balance (CULS src/algorithms/balance.cu:912-1382) works on a graph
+with a block, a thread-block cluster or the whole grid, by its width, and on
+the graphs of a batch together as far as scratch allows.  Graphs whose levels
+are about as wide as each team, covers longer than a thread keeps (32 leaves)
+and than the reference's limits, constant covers, and a budget that takes the
+graphs one at a time must all give the oracle's graph."""
+import numpy as np
+import pytest
+
+import culs_b200 as C
+from oracle.oracle import Oracle
+from util import same_graph, to_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def oracle_b(g):
+    o = Oracle()
+    o.set_graph(to_oracle(g))
+    o.b()
+    return o.graph()
+
+
+def check(ctx, g):
+    d = ctx.upload(g)
+    ctx.b(d)
+    got, ref = d.download(), oracle_b(g)
+    assert same_graph(got, ref) and got.nLevels == ref.nLevels
+
+
+def products(seed, n_pis, sizes, contradict=False):
+    """Single-fanout AND chains of the given sizes over random PI literals,
+    their outputs paired up; with `contradict`, every third chain holds a
+    literal and its complement."""
+    rng = np.random.default_rng(seed)
+    f0, f1 = [-1] * (1 + n_pis), [-1] * (1 + n_pis)
+
+    def new(a, b):
+        f0.append(min(a, b))
+        f1.append(max(a, b))
+        return 2 * (len(f0) - 1)
+
+    tops = []
+    for k, size in enumerate(sizes):
+        lits = [int(2 * p + rng.integers(0, 2)) for p in rng.choice(np.arange(1, 1 + n_pis), size, replace=False)]
+        if contradict and k % 3 == 0:
+            lits[-1] = lits[0] ^ 1
+        x = lits[0]
+        for y in lits[1:]:
+            x = new(x, y)
+        tops.append(x)
+    outs = [new(a ^ 1, b ^ 1) for a, b in zip(tops, tops[1:])] + tops[:1]
+    return C.Aig(n_pis, np.array(f0, np.int32), np.array(f1, np.int32), np.array(outs, np.int32))
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    c = C.Context()
+    yield c
+    c.close()
+
+
+@pytest.mark.parametrize("ands,layers", [(4000, 10), (6000, 10), (11000, 10), (22000, 10), (45000, 10), (90000, 20),
+                                         (120000, 10)])
+def test_every_team_matches_oracle(ctx, ands, layers):
+    check(ctx, C.gen_layered(3, 600, 400, ands, layers, 3, 0.1, True))
+
+
+@pytest.mark.parametrize("contradict", [False, True])
+@pytest.mark.parametrize("longest", [31, 33, 120, 140, 1030])
+def test_long_covers_match_oracle(ctx, longest, contradict):
+    rng = np.random.default_rng(longest)
+    sizes = [int(s) for s in rng.integers(2, longest, 40)] + [longest, longest - 1, 2, 32]
+    check(ctx, products(longest, 1100, sizes, contradict))
+
+
+def test_batch_and_tight_budget_match_oracle(ctx):
+    gs = [C.gen_multiplier(20), C.gen_layered(3, 600, 400, 22000, 10, 3, 0.1, True), products(1, 200, [5, 60, 3, 150]),
+          C.gen_multiplier(3), *C.gen_batch(4, 10, 20, 200, 5000, 16, 64, threads=8)]
+    refs = [oracle_b(g) for g in gs]
+    largest = max(g.nObjs for g in gs)
+    tight = C.Context(hbm_budget=largest * 900 + (200 << 20))
+    try:
+        for c in [ctx, tight]:
+            d = c.upload_batch(gs)
+            c.b(d)
+            for i, ref in enumerate(refs):
+                got = d.download(i)
+                assert same_graph(got, ref) and got.nLevels == ref.nLevels, i
+    finally:
+        tight.close()
