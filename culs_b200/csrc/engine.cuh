@@ -30,7 +30,7 @@ struct ExecCtx;
 // Launch and schedule parameters that do not change results, only speed
 // (set by culs_set_param or culs_autotune).
 struct Tune {
-    int enumWideMin = 16384;   // levels this wide run one node per thread, narrower one per warp
+    int enumWideMin = 32768;   // levels this wide run one node per thread, narrower one per warp
     int enumBlocksPerSm = 8;   // persistent enumeration blocks per SM
     int evalGroupMSlots = 16;  // existence-table slots (millions) of a group of graphs built and evaluated together
 };

@@ -10,6 +10,9 @@
 // node reads nothing but its two fanins' 16 cut records.  Pairs whose 32-bit
 // signatures already exceed 4 leaves are rejected from the fanins' {sign,
 // packed} words before any leaf data is fetched.
+#include <algorithm>
+#include <vector>
+
 #include "enum_regs.cuh"
 #include "rw_work.cuh"
 
@@ -20,12 +23,10 @@ namespace {
 constexpr int kEnumBlock = 128;
 
 struct EnumArgs {
-    int64_t nL0, N;
-    const int *lvlCnt;      // AND nodes per level (level 0: none)
-    const int *lvlStart;    // first W position of each level
-    const int *chunkStart;  // first chunk of each level; maxLevel + 2 entries
-    int maxLevel;
-    int wideMin;            // levels at least this wide run thread-per-node
+    int64_t q0, q1;         // the W positions of the launch's levels
+    int nLevels;            // its levels,
+    const int *lvlStart;    //   the first W position of each and the end (nLevels + 1 entries), and
+    const int *chunkStart;  //   the first 32-node chunk of each and the end
     const int *w0, *w1;
     const int *ref;
     const uint8_t *lidLow;
@@ -493,22 +494,20 @@ __device__ __forceinline__ void enum_node_thread(const EnumArgs &A, int64_t q, b
     st_release(&A.done[q], 1);
 }
 
-// Levels are cut into chunks that never cross a level: a wide level into
-// 32-node chunks, each node on one thread (throughput), a narrow level into
-// one-node chunks, each node on a whole warp (latency: a narrow level's
-// time is the time of its slowest node).  Warps claim chunks in level
-// order, so every fanin of a claimed node lies in an earlier, claimed chunk.
+// A run of wide levels, each node on one thread (throughput): the levels are
+// cut into 32-node chunks that never cross a level, which warps claim in
+// level order, so every fanin of a claimed node lies in an earlier, claimed
+// chunk or below the run.
 __global__ void __launch_bounds__(kEnumBlock, 4) k_enumerate(EnumArgs A) {
-    __shared__ WarpCands s_cand[kEnumBlock / 32];
     const unsigned F = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    const int total = A.chunkStart[A.maxLevel + 1];
+    const int total = A.chunkStart[A.nLevels];
     while (true) {
         int c = 0;
         if (lane == 0) c = atomicAdd(A.counter, 1);
         c = __shfl_sync(F, c, 0);
         if (c >= total) break;
-        int lo = 1, hi = A.maxLevel;
+        int lo = 0, hi = A.nLevels - 1;
         while (lo < hi) {  // last level whose first chunk is <= c
             const int mid = (lo + hi + 1) >> 1;
             if (A.chunkStart[mid] <= c)
@@ -516,34 +515,58 @@ __global__ void __launch_bounds__(kEnumBlock, 4) k_enumerate(EnumArgs A) {
             else
                 hi = mid - 1;
         }
-        const int w = A.lvlCnt[lo];
-        const int64_t base = A.nL0 + A.lvlStart[lo];
-        const int64_t k = c - A.chunkStart[lo];
-        if (w >= A.wideMin) {
-            const int64_t q = base + k * 32 + lane;
-            enum_node_thread(A, q, q < base + w);
-        } else {
-            enum_node_warp(A, base + k, lane, s_cand[threadIdx.x >> 5]);
-        }
+        const int64_t q = (int64_t)A.lvlStart[lo] + (int64_t)(c - A.chunkStart[lo]) * 32 + lane;
+        enum_node_thread(A, q, q < A.lvlStart[lo + 1]);
     }
 }
 
-// lvlCnt has nBins counters (levels 0 .. nBins - 1)
-__global__ void k_level_count(int64_t nL0, int64_t N, const int *wlev, int *lvlCnt, int nBins) {
-    __shared__ int h[kHistBins];
-    hist_begin(h, nBins);
-    int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t q = nL0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += stride)
-        hist_add(h, nBins, lvlCnt, wlev[q]);
-    hist_end(h, nBins, lvlCnt);
+// A run of narrower levels, each node on a warp (latency: a level's time is
+// that of its slowest node), claimed in W order.  A kernel of its own for its
+// smaller register need: six resident blocks an SM instead of the four of one
+// kernel for both forms (1M-AND layered graph, 3,800 nodes a level: 2.80 ->
+// 1.94 ms).
+//
+// Where the forms meet (Tune::enumWideMin): a wide level takes about 40 us
+// however few nodes it has, one warp's 32 replays; a warp per node takes 2 ns
+// a node and 8 us at least.  128 graphs of up to 100k ANDs: 9.9 ms with the
+// line at 4,096 nodes a level, 5.7 at 16,384, 5.0 at 32,768, 5.05 at 65,536
+// and 5.5 with no wide levels; 256 graphs of up to 200k: 19.0, 17.2, 16.6,
+// 19.6, 21.4.
+__global__ void __launch_bounds__(kEnumBlock, 6) k_enumerate_warp(EnumArgs A) {
+    __shared__ WarpCands s_cand[kEnumBlock / 32];
+    const int lane = threadIdx.x & 31;
+    while (true) {
+        int c = 0;
+        if (lane == 0) c = atomicAdd(A.counter, 1);
+        c = __shfl_sync(0xffffffffu, c, 0);
+        if (c >= A.q1 - A.q0) break;
+        enum_node_warp(A, A.q0 + c, lane, s_cand[threadIdx.x >> 5]);
+    }
 }
 
-__global__ void k_level_chunks(int n, const int *lvlCnt, int wideMin, int *cc) {
-    int stride = gridDim.x * blockDim.x;
-    for (int l = blockIdx.x * blockDim.x + threadIdx.x; l < n; l += stride) {
-        const int w = lvlCnt[l];
-        cc[l] = w >= wideMin ? (w + 31) / 32 : w;
+// Runs of levels that take the same form.  Every run is a launch, which waits
+// for the one before it: a profile that changes too often takes the form of
+// most of its nodes throughout.
+struct EnumRun {
+    bool wide;
+    int l0, l1;  // levels [l0, l1)
+};
+
+std::vector<EnumRun> enum_runs(const std::vector<int> &cnt, int wideMin) {
+    constexpr size_t kMaxRuns = 8;
+    std::vector<EnumRun> runs;
+    int64_t wide = 0, all = 0;
+    for (int l = 1; l < (int)cnt.size(); l++) {
+        const bool w = cnt[l] >= wideMin;
+        all += cnt[l];
+        if (w) wide += cnt[l];
+        if (runs.empty() || runs.back().wide != w)
+            runs.push_back(EnumRun{w, l, l + 1});
+        else
+            runs.back().l1 = l + 1;
     }
+    if (runs.size() > kMaxRuns) runs = {EnumRun{2 * wide > all, 1, (int)cnt.size()}};
+    return runs;
 }
 
 }  // namespace
@@ -560,29 +583,49 @@ int rw_enumerate(ExecCtx &X, RwWork &w) {
         return X.fail(CULS_E_OOM, "rw: scratch arena exhausted (cuts)");
     int rc;
     if ((rc = X.check(cudaMemsetAsync(w.cutM, 0, sizeof(int2) * N * 8, s), "memset"))) return rc;
-    if ((rc = X.check(cudaMemsetAsync(X.counters, 0, sizeof(int) * 4, s), "memset"))) return rc;
     if ((rc = X.check(cudaMemsetAsync(w.warpPairs, 0, sizeof(unsigned long long), s), "memset"))) return rc;
-    // per-level widths, starts and chunk offsets
-    const int L = w.maxLevel + 2;
-    int *lvlCnt = X.ar->get<int>(L), *lvlStart = X.ar->get<int>(L), *cc = X.ar->get<int>(L),
-        *chunkStart = X.ar->get<int>(L);
-    if (!lvlCnt || !lvlStart || !cc || !chunkStart) return X.fail(CULS_E_OOM, "rw: scratch arena exhausted (levels)");
-    if ((rc = X.check(cudaMemsetAsync(lvlCnt, 0, sizeof(int) * L, s), "memset"))) return rc;
-    k_level_count<<<X.grid(N - w.nL0), kBlock, 0, s>>>(w.nL0, N, w.wlev, lvlCnt, w.maxLevel + 1);
-    k_level_chunks<<<grid_1d(L, kBlock, X.sms * 16), kBlock, 0, s>>>(L - 1, lvlCnt, X.tune->enumWideMin, cc);
-    if ((rc = X.check(scan_exclusive(lvlCnt, lvlStart, L - 1, nullptr, *X.ar, s), "scan"))) return rc;
-    if ((rc = X.check(scan_exclusive(cc, chunkStart, L - 1, chunkStart + L - 1, *X.ar, s), "scan"))) return rc;
+    const std::vector<EnumRun> runs = enum_runs(w.lvlCnt, X.tune->enumWideMin);
+    // per run: its claim counter and, if wide, its levels' starts and chunks
+    const int nRuns = (int)runs.size();
+    std::vector<int> host(nRuns, 0);
+    std::vector<int64_t> lvlStart(w.lvlCnt.size() + 1, w.nL0);  // W position of each level's first AND node
+    for (size_t l = 1; l < w.lvlCnt.size(); l++) lvlStart[l + 1] = lvlStart[l] + w.lvlCnt[l];
+    for (const EnumRun &r : runs) {
+        if (!r.wide) continue;
+        for (int l = r.l0; l <= r.l1; l++) host.push_back((int)lvlStart[l]);
+        int chunks = 0;
+        for (int l = r.l0; l <= r.l1; l++) {
+            host.push_back(chunks);
+            if (l < r.l1) chunks += (w.lvlCnt[l] + 31) / 32;
+        }
+    }
+    int *dev = X.ar->get<int>(host.size() + 1);
+    if (!dev) return X.fail(CULS_E_OOM, "rw: scratch arena exhausted (levels)");
+    if (nRuns && (rc = X.check(cudaMemcpyAsync(dev, host.data(), sizeof(int) * host.size(), cudaMemcpyHostToDevice, s), "h2d")))
+        return rc;
     k_enum_init<<<X.grid(N), kBlock, 0, s>>>(N, w.wlev, w.wl, w.lidLow, w.ref, w.cutL, w.cutM, w.cutA, done);
-    // lvlStart counts AND nodes only: the AND positions of W start at nL0
-    EnumArgs A{w.nL0, N,       lvlCnt, lvlStart, chunkStart, w.maxLevel, X.tune->enumWideMin, w.w0, w.w1,
-               w.ref, w.lidLow, w.cutL, w.cutM, w.cutA,     done,       X.counters, w.warpPairs, X.status};
+    X.launched(1);
     X.mark(kMkEnumK0);
-    // a wide batch fills the GPU; a narrow one runs about sixteen levels'
-    // worth of chunks at a time (32 nodes a warp on wide levels, 1 on narrow)
-    const int perBlock = (kEnumBlock / 32) * (w.width >= X.tune->enumWideMin ? 32 : 1);
-    k_enumerate<<<flow_blocks(w.width, perBlock, (unsigned)(X.sms * X.tune->enumBlocksPerSm), X.sms), kEnumBlock, 0, s>>>(A);
+    const int *table = dev + nRuns;
+    for (int k = 0; k < nRuns; k++) {
+        const EnumRun &r = runs[k];
+        const int n = r.l1 - r.l0;
+        EnumArgs A{lvlStart[r.l0], lvlStart[r.l1], n,        table,    table + n + 1, w.w0, w.w1, w.ref,
+                   w.lidLow,       w.cutL,         w.cutM,   w.cutA,   done,          dev + k, w.warpPairs, X.status};
+        const int64_t width = (A.q1 - A.q0) / n + 1;
+        // a wide run fills the GPU; a narrow one runs about sixteen levels'
+        // worth of nodes at a time
+        if (r.wide) {
+            table += 2 * (n + 1);
+            k_enumerate<<<flow_blocks(width, kEnumBlock, (unsigned)(X.sms * X.tune->enumBlocksPerSm), X.sms), kEnumBlock, 0,
+                          s>>>(A);
+        } else {
+            k_enumerate_warp<<<flow_blocks(width, kEnumBlock / 32, (unsigned)(X.sms * std::min(X.tune->enumBlocksPerSm, 6)),
+                                           X.sms), kEnumBlock, 0, s>>>(A);
+        }
+        X.launched(1);
+    }
     X.mark(kMkEnumK1);
-    X.launched(6);
     if ((rc = X.check(cudaGetLastError(), "enumerate launch"))) return rc;
     return 0;
 }

@@ -125,6 +125,16 @@ __global__ void k_front_permute(int64_t N, const int *order, const int *newPos, 
     }
 }
 
+// AND nodes per level; lvlCnt has nBins counters (levels 0 .. nBins - 1)
+__global__ void k_front_level_count(int64_t nL0, int64_t N, const int *wlev, int *lvlCnt, int nBins) {
+    __shared__ int h[kHistBins];
+    hist_begin(h, nBins);
+    int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t q = nL0 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < N; q += stride)
+        hist_add(h, nBins, lvlCnt, wlev[q]);
+    hist_end(h, nBins, lvlCnt);
+}
+
 __global__ void k_front_local_ids(int64_t N, const int *byGraph, const int *wg, const DevGraph *dg, int *wl,
                                   uint8_t *lidLow) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -216,7 +226,11 @@ int rw_front(ExecCtx &X, Batch &b, RwWork &w) {
     k_front_inverse<<<X.grid(N), kBlock, 0, s>>>(N, order, newPos);
     k_front_permute<<<X.grid(N), kBlock, 0, s>>>(N, order, newPos, gidIn, a0, a1, lp, b.dg, w.w0, w.w1, w.wg, w.wlev,
                                                   w.wph);
-    X.launched(2);
+    int *lvlCnt = ar.get<int>(w.maxLevel + 1);
+    if (!lvlCnt) return X.fail(CULS_E_OOM, "rw: scratch arena exhausted (front)");
+    if ((rc = X.check(cudaMemsetAsync(lvlCnt, 0, sizeof(int) * (w.maxLevel + 1), s), "memset"))) return rc;
+    k_front_level_count<<<X.grid(N - w.nL0), kBlock, 0, s>>>(w.nL0, N, w.wlev, lvlCnt, w.maxLevel + 1);
+    X.launched(3);
     // local ids: rank of each W position among its graph's positions
     int *byGraph = done;  // reuse
     if (G == 1) {
@@ -235,6 +249,10 @@ int rw_front(ExecCtx &X, Batch &b, RwWork &w) {
     if ((rc = X.check(cudaMemsetAsync(w.ref, 0, sizeof(int) * N, s), "memset"))) return rc;
     k_front_refs<<<X.grid(std::max<int64_t>(N, b.nPO)), kBlock, 0, s>>>(N, w.w0, w.w1, w.wlev, b.nPO, w.wpo, w.ref);
     X.launched(3);
+    w.lvlCnt.resize(w.maxLevel + 1);
+    if ((rc = X.check(cudaMemcpyAsync(w.lvlCnt.data(), lvlCnt, sizeof(int) * (w.maxLevel + 1), cudaMemcpyDeviceToHost, s),
+                      "d2h")))
+        return rc;
     // graph table now carries the constant positions of W
     if ((rc = X.check(cudaMemcpyAsync(b.hg.data(), b.dg, sizeof(DevGraph) * G, cudaMemcpyDeviceToHost, s), "d2h")))
         return rc;

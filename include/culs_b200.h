@@ -225,7 +225,7 @@ int culs_fetch_aiger(culs_ctx *ctx, int64_t job, uint8_t *buf, size_t cap, size_
  * Launch and schedule parameters: they change speed only, never results.
  * CULS_PARAM_ENUM_WIDE_MIN: cut-enumeration levels with at least this many
  * AND nodes run one node per thread, narrower ones one node per warp
- * (default 16384).  CULS_PARAM_ENUM_BLOCKS_PER_SM: persistent enumeration
+ * (default 32768).  CULS_PARAM_ENUM_BLOCKS_PER_SM: persistent enumeration
  * blocks per SM (default 8).  CULS_PARAM_SM_SHARE: size every grid of the
  * context for 1/value of the device's SMs (default 1), for contexts that run
  * at once on one GPU (the served workers use their share); setting it also
