@@ -430,8 +430,7 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
     if (nAnd > 0)
         k_aig_ands<<<X.grid(nAnd), kBlock, 0, s>>>(nAnd, count, dAnd, dTerm, b.dg, nums, b.F0, b.F1, status_);
     launches_ += 4;
-    if ((rc = sync())) return rc;
-    if ((rc = check_status("upload (AIGER)"))) return rc;
+    if ((rc = fetch("upload (AIGER)"))) return rc;
     b.G = count;
     b.nObj = nObj;
     b.nPO = nPO;
@@ -454,8 +453,9 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
     ar_.reset();
     int64_t *dAnd = ar_.get<int64_t>(G + 1);
     long long *lenA = ar_.get<long long>(nAnd + 1), *offA = ar_.get<long long>(nAnd + 1),
-              *gOff = ar_.get<long long>(G + 1), *tot = ar_.get<long long>(1);
-    if (!dAnd || !lenA || !offA || !gOff || !tot) return fail(CULS_E_OOM, "download: arena exhausted (AIGER)");
+              *gOff = ar_.get<long long>(G + 1);
+    long long *tot = reinterpret_cast<long long *>(counters_);
+    if (!dAnd || !lenA || !offA || !gOff) return fail(CULS_E_OOM, "download: arena exhausted (AIGER)");
     cudaStream_t s = s_;
     ExecCtx X = ctx();
     if ((rc = check(cudaMemcpyAsync(dAnd, andBase.data(), sizeof(int64_t) * (G + 1), cudaMemcpyHostToDevice, s), "h2d")))
@@ -464,10 +464,7 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
     if (nAnd > 0) {
         k_aig_enc_len<<<X.grid(nAnd), kBlock, 0, s>>>(nAnd, G, dAnd, b.dg, b.F0, b.F1, lenA, status_);
         if ((rc = check(scan_exclusive(lenA, offA, nAnd, tot, ar_, s), "scan"))) return rc;
-        if ((rc = check(cudaMemcpyAsync(&hostSmall_[0], tot, sizeof(long long), cudaMemcpyDeviceToHost, s), "d2h")))
-            return rc;
-        if ((rc = sync())) return rc;
-        if ((rc = check_status("download (AIGER)"))) return rc;
+        if ((rc = fetch("download (AIGER)"))) return rc;
         memcpy(&total, hostSmall_, sizeof total);
     }
     uint8_t *dB = ar_.get<uint8_t>(total + 1);

@@ -798,16 +798,15 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
     launches_ += 1;
     // ---- covers by (graph, last level, id); per level: count and longest cover
     uint8_t *flags = ar_.get<uint8_t>(nObj);
-    int *ids = ar_.get<int>(nObj), *sorted = ar_.get<int>(nObj), *ncov = ar_.get<int>(1);
+    int *ids = ar_.get<int>(nObj), *sorted = ar_.get<int>(nObj);
     // the sort's keys, in the place of arrays that are not read any more
     uint32_t *keys = reinterpret_cast<uint32_t *>(A.lists[0]), *keys2 = reinterpret_cast<uint32_t *>(A.lists[1]);
-    if (!flags || !ids || !sorted || !ncov) return fail(CULS_E_OOM, "balance: arena exhausted");
+    if (!flags || !ids || !sorted) return fail(CULS_E_OOM, "balance: arena exhausted");
     k_bal_cover_flags<<<grid_1d(nObj, kBlock, sms_ * 8), kBlock, 0, s>>>(nObj, A.covLen, flags);
-    check(compact_flags(flags, nObj, ids, ncov, ar_, s), "compact");
+    check(compact_flags(flags, nObj, ids, counters_, ar_, s), "compact");
     std::vector<int> hc((size_t)G * kBcSize);
-    check(cudaMemcpyAsync(hostSmall_, ncov, sizeof(int), cudaMemcpyDeviceToHost, s), "d2h");
     check(cudaMemcpyAsync(hc.data(), A.cnt, sizeof(int) * (size_t)G * kBcSize, cudaMemcpyDeviceToHost, s), "d2h");
-    if ((rc = sync()) || (rc = check_status("balance covers"))) return rc;
+    if ((rc = fetch("balance covers"))) return rc;
     const int nCov = hostSmall_[0];
     int64_t nLv = 0, nTab = 0;
     for (int i = 0; i < G; i++) {
@@ -840,7 +839,7 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
         return rc;
     launches_ += 4;
     check(cudaMemcpyAsync(hc.data(), A.cnt, sizeof(int) * (size_t)G * kBcSize, cudaMemcpyDeviceToHost, s), "d2h");
-    if ((rc = sync()) || (rc = check_status("balance reconstruction"))) return rc;
+    if ((rc = fetch("balance reconstruction"))) return rc;
     // ---- phase 3: renumbering in id order
     int64_t nB = 0, out = ng[ga].base;
     int maxId = 0;
@@ -856,14 +855,14 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
         out += 1 + (int64_t)g.nPIs + g.nBuilt;
     }
     uint8_t *used = ar_.get<uint8_t>(nTab);
-    int *slots = ar_.get<int>(nB + 1), *slots2 = ar_.get<int>(nB + 1), *nBuilt = ar_.get<int>(1);
+    int *slots = ar_.get<int>(nB + 1), *slots2 = ar_.get<int>(nB + 1);
     uint32_t *bk = ar_.get<uint32_t>(nB + 1), *bk2 = ar_.get<uint32_t>(nB + 1);
-    if (!used || !slots || !slots2 || !nBuilt || !bk || !bk2) return fail(CULS_E_OOM, "balance: arena exhausted");
+    if (!used || !slots || !slots2 || !bk || !bk2) return fail(CULS_E_OOM, "balance: arena exhausted");
     check(cudaMemcpyAsync(dg, bg.data(), sizeof(BalGraph) * G, cudaMemcpyHostToDevice, s), "h2d");
     if (nB > 0) {
         const unsigned gs = grid_1d(nB, kBlock, sms_ * 8);
         k_bal_used<<<grid_1d(nTab, kBlock, sms_ * 16), kBlock, 0, s>>>(nTab, A.tab, used);
-        check(compact_flags(used, nTab, slots, nBuilt, ar_, s), "compact");
+        check(compact_flags(used, nTab, slots, counters_, ar_, s), "compact");
         k_bal_ids<<<gs, kBlock, 0, s>>>(nB, slots, A.tab, bk);
         if ((rc = check(radix_sort_pairs(bk, slots, bk2, slots2, nB, bits_for((int64_t)maxId + 1), ar_, s), "sort")))
             return rc;
@@ -909,7 +908,7 @@ int Engine::balance(Batch &b, bool updateLevel) {
         if (rc) return rc;
         ga = gb;
     }
-    if ((rc = sync()) || (rc = check_status("balance output"))) return rc;
+    if ((rc = fetch("balance output"))) return rc;
     ar_.reset();
     const int64_t nObj = b.G > 0 ? (int64_t)ng[b.G - 1].base + 1 + ng[b.G - 1].nPIs + ng[b.G - 1].nAnds : 0;
     if ((rc = check(cudaMemcpyAsync(b.dg, ng.data(), sizeof(DevGraph) * b.G, cudaMemcpyHostToDevice, s_), "h2d")))

@@ -229,6 +229,7 @@ class Engine {
     int fail(int code, const std::string &msg);
     int check(cudaError_t e, const char *what);
     int check_status(const char *what);
+    int fetch(const char *what);  // ExecCtx::fetch
     int ensure_arena(size_t bytes);
     int ensure_stage(size_t ints);  // pinned host staging of at least `ints` int32
     ExecCtx ctx();
@@ -263,10 +264,10 @@ class Engine {
     std::string err_;
     cudaStream_t s_ = nullptr;
     RwLib *lib_ = nullptr;
-    int *status_ = nullptr;     // device status word and spin bound (2 ints)
+    int *status_ = nullptr;     // device status word and spin bound (2 ints of counters_)
     int spinLimit_ = 0;         // the bound last written to status_[1]
-    int *counters_ = nullptr;   // device scratch counters
-    int *hostSmall_ = nullptr;  // pinned host scratch
+    int *counters_ = nullptr;   // device scratch counters (kCounters ints, see rw_work.cuh)
+    int *hostSmall_ = nullptr;  // their pinned host copy
     int32_t *stage_ = nullptr;  // pinned staging for uploads and downloads
     size_t stageCap_ = 0;       // in int32
     size_t budget_ = 0;

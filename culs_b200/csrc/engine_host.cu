@@ -11,12 +11,12 @@ extern "C" const size_t culs_rwlib_blob_size;
 
 namespace culs {
 
-int ExecCtx::status_check(const char *what) {
-    int st = 0;
-    cudaError_t e = cudaMemcpy(&st, status, sizeof(int), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return check(e, what);
+int ExecCtx::fetch(const char *what) {
+    int rc = check(cudaMemcpyAsync(hostSmall, counters, sizeof(int) * kCounters, cudaMemcpyDeviceToHost, s), "d2h");
+    if (rc || (rc = sync())) return rc;
+    const int st = hostSmall[kCtStatus];
     if (st == kDevOk) return 0;
-    cudaMemset(status, 0, sizeof(int));
+    if ((rc = check(cudaMemsetAsync(status, 0, sizeof(int), s), "memset")) || (rc = sync())) return rc;
     static const char *names[] = {"ok", "dependency wait timed out", "hash table full", "traversal stack overflow",
                                   "malformed graph", "work buffer too small", "malformed binary AIGER"};
     if (err) *err = std::string(what) + ": " + (st >= 0 && st <= 6 ? names[st] : "device error");
@@ -266,7 +266,6 @@ Engine::Engine() = default;
 Engine::~Engine() {
     if (s_) cudaStreamSynchronize(s_);
     cudaFree(lib_);
-    cudaFree(status_);
     cudaFree(counters_);
     if (hostSmall_) cudaFreeHost(hostSmall_);
     if (stage_) cudaFreeHost(stage_);
@@ -288,10 +287,12 @@ int Engine::check(cudaError_t e, const char *what) {
 
 int Engine::sync() { return check(cudaStreamSynchronize(s_), "stream sync"); }
 
-int Engine::check_status(const char *what) {
+int Engine::fetch(const char *what) {
     ExecCtx X = ctx();
-    return X.status_check(what);
+    return X.fetch(what);
 }
+
+int Engine::check_status(const char *what) { return fetch(what); }
 
 // CULS_SPIN_LIMIT (spin iterations, 0 or unset = the built-in bound of about
 // one second) bounds every dependency wait of the next calls; the tests lower
@@ -342,11 +343,12 @@ int Engine::init(size_t hbmBudget) {
     if (!rc) rc = check(cudaMemcpy(lib_, h, sizeof(RwLib), cudaMemcpyHostToDevice), "library upload");
     delete h;
     if (rc) return rc;
-    // status word and the spin bound of dependency waits (see common.cuh)
-    if ((rc = check(cudaMalloc(&status_, sizeof(int) * 2), "cudaMalloc"))) return rc;
-    if ((rc = check(cudaMemset(status_, 0, sizeof(int) * 2), "memset"))) return rc;
-    if ((rc = check(cudaMalloc(&counters_, sizeof(int) * 64), "cudaMalloc"))) return rc;
-    if ((rc = check(cudaMallocHost(&hostSmall_, sizeof(int) * 64), "cudaMallocHost"))) return rc;
+    // the counters hold the status word and the spin bound of dependency
+    // waits (see common.cuh), so that one copy reads both
+    if ((rc = check(cudaMalloc(&counters_, sizeof(int) * kCounters), "cudaMalloc"))) return rc;
+    if ((rc = check(cudaMemset(counters_, 0, sizeof(int) * kCounters), "memset"))) return rc;
+    status_ = counters_ + kCtStatus;
+    if ((rc = check(cudaMallocHost(&hostSmall_, sizeof(int) * kCounters), "cudaMallocHost"))) return rc;
     for (auto &e : ev_)
         if ((rc = check(cudaEventCreate(&e), "event"))) return rc;
     size_t freeB = 0, totalB = 0;

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <climits>
 #include <cstdlib>
+#include <cstring>
 
 #include "rw_work.cuh"
 
@@ -42,7 +43,8 @@ struct ChoiceArgs {
     int4 *rec;                // per node {L0, L1, ref, del}
     int *mark;                // per node: lowest window place that changes it (INT_MAX: none)
     const int4 *recA, *recB;  // per candidate in graph order: {c, q, rep, -}, leaves
-    const int *gStart, *gCount;
+    const int *gStart, *gCount;  // a graph's candidates (several graphs)
+    int n;                       // all candidates
     int useZeros;
     int serial;  // replay every candidate alone
     int4 *stack;
@@ -362,8 +364,8 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
     const int t = (tid & 31) * kWarps + (tid >> 5);  // place in the window
     const int64_t nL0 = A.nL0;
     const int trueLit = 2 * A.dg[g].cpos + 1;
-    int base = A.gStart[g];
-    const int end = base + A.gCount[g];
+    int base = gridDim.x > 1 ? A.gStart[g] : 0;
+    const int end = gridDim.x > 1 ? base + A.gCount[g] : A.n;
     if (tid < 2) s_stop[tid] = INT_MAX;
     __syncthreads();
     int nDone[kChReverted + 1] = {}, nPos = 0, expected = 0;
@@ -529,7 +531,7 @@ cudaError_t launch_choice(const ChoiceArgs &A, int G, cudaStream_t s) {
 
 }  // namespace
 
-int rw_choice(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats) {
+int rw_choice(ExecCtx &X, Batch &b, RwWork &w) {
     const int G = w.G;
     const int64_t nCand = w.nCand, nRep = w.nRep;
     const int64_t M = w.N + w.nNew;  // extent of L0, L1, ref, del
@@ -541,7 +543,7 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats) {
     int *vals = ar.get<int>(nRep + 1);
     int4 *recA = ar.get<int4>(nRep + 1), *recB = ar.get<int4>(nRep + 1);
     w.choice = ar.get<int>(nCand + 1);
-    unsigned long long *dstats = ar.get<unsigned long long>(8);
+    unsigned long long *dstats = reinterpret_cast<unsigned long long *>(X.counters + kCtStats);
     // explicit recursion stacks: deep enough for any chain through the
     // levels plus the new nodes
     int64_t stackCap = (int64_t)w.maxLevel + 64;
@@ -558,29 +560,29 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats) {
         rec = ar.get<int4>(M);
         mark = ar.get<int>(M);
     }
-    if (!gCount || !gStart || !candByG || !keys || !keys2 || !vals || !recA || !recB || !w.choice || !dstats || !stack ||
+    if (!gCount || !gStart || !candByG || !keys || !keys2 || !vals || !recA || !recB || !w.choice || !stack ||
         !rec || !mark)
         return X.fail(CULS_E_OOM, "rw: arena exhausted (choice)");
-    if ((rc = X.check(cudaMemsetAsync(gCount, 0, sizeof(int) * (G + 1), s), "memset"))) return rc;
+    if (G > 1 && (rc = X.check(cudaMemsetAsync(gCount, 0, sizeof(int) * (G + 1), s), "memset"))) return rc;
     if ((rc = X.check(cudaMemsetAsync(dstats, 0, sizeof(unsigned long long) * 8, s), "memset"))) return rc;
     if ((rc = X.check(fill_i32(w.choice, kChNoReplace, nCand, s), "fill"))) return rc;
     if (nRep > 0) {
-        k_cand_gid<<<X.grid(nRep), kBlock, 0, s>>>(nRep, w.withRep, w.cand, w.wg, keys, vals, gCount);
-        X.launched(1);
         if (G > 1) {
+            k_cand_gid<<<X.grid(nRep), kBlock, 0, s>>>(nRep, w.withRep, w.cand, w.wg, keys, vals, gCount);
+            X.launched(1);
             int bits = 1;
             while ((1ll << bits) < G) bits++;
             if ((rc = X.check(radix_sort_pairs(keys, vals, keys2, candByG, nRep, bits, ar, s), "sort"))) return rc;
+            if ((rc = X.check(scan_exclusive(gCount, gStart, G, nullptr, ar, s), "scan"))) return rc;
         } else {
             candByG = w.withRep;
         }
         k_cand_records<<<X.grid(nRep), kBlock, 0, s>>>(nRep, candByG, w.cand, w.repW, w.bestCut, w.cutL, w.cutM, w.wg,
                                                        w.dg, recA, recB);
-        if ((rc = X.check(scan_exclusive(gCount, gStart, G, nullptr, ar, s), "scan"))) return rc;
         k_choice_pack<<<X.grid(M), kBlock, 0, s>>>(M, w.L0, w.L1, w.ref, w.del, rec, mark);
         // CULS_CHOICE_GLOBAL replays every candidate alone (the tests compare
         // the two)
-        ChoiceArgs A{w.nL0,  w.dg,  rec,           mark,     recA,   recB,    gStart, gCount, w.useZeros ? 1 : 0,
+        ChoiceArgs A{w.nL0,  w.dg,  rec,           mark,     recA,   recB,    gStart, gCount, (int)nRep, w.useZeros ? 1 : 0,
                      getenv("CULS_CHOICE_GLOBAL") ? 1 : 0, stack, (int)stackCap, w.choice, dstats, X.status};
         // Threads per graph: a window as wide as an SM's shared memory allows
         // while there is an SM for every graph, narrower ones so that more
@@ -596,28 +598,6 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats) {
         if (rc) return rc;
         k_choice_unpack<<<X.grid(M), kBlock, 0, s>>>(M, rec, w.L0, w.L1, w.del);
         X.launched(4);
-    }
-    unsigned long long hs[8], warpPairs = 0;
-    if ((rc = X.check(cudaMemcpyAsync(hs, dstats, sizeof hs, cudaMemcpyDeviceToHost, s), "d2h"))) return rc;
-    if (w.warpPairs &&
-        (rc = X.check(cudaMemcpyAsync(&warpPairs, w.warpPairs, sizeof warpPairs, cudaMemcpyDeviceToHost, s), "d2h")))
-        return rc;
-    if ((rc = X.sync())) return rc;
-    if ((rc = X.status_check("rw choice"))) return rc;
-    if (stats) {
-        int64_t nAnd = w.N - w.nL0;
-        stats->replaced = (long long)hs[0];
-        stats->replacedPos = (long long)hs[1];
-        stats->replacedZero = (long long)hs[2];
-        stats->reverted = (long long)hs[3];
-        stats->compromised = (long long)hs[4];
-        stats->newIdx = nCand - nRep;
-        stats->expected = (long long)hs[6];
-        stats->preEval = nAnd - nCand;
-        stats->smallCut = 0;
-        stats->newNodes = w.nNew;
-        stats->candidates = nCand;
-        stats->warpPairs = (long long)warpPairs;
     }
     (void)b;
     return 0;
@@ -710,7 +690,7 @@ __global__ void k_redundancy_finish(RedArgs A, int *L0, int *L1, uint8_t *delOut
 
 }  // namespace
 
-int rw_redundancy(ExecCtx &X, Batch &b, RwWork &w) {
+int rw_redundancy(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats) {
     (void)b;
     const int64_t M = w.N + w.nNew;
     cudaStream_t s = X.s;
@@ -727,30 +707,48 @@ int rw_redundancy(ExecCtx &X, Batch &b, RwWork &w) {
     X.launched(1);
     int *changed = X.counters + 24;
     // sweep state: (post1, nred) of the chased nodes; state 0 (no chase
-    // yet) is (pre1, 0), read from pre1 itself
+    // yet) is (pre1, 0), read from pre1 itself.  Two sweeps per host check:
+    // the second one usually finds nothing left to change.
     const int *in1 = pre1;
     const uint8_t *inR = NR[0];
     int cur = 1;
-    for (int it = 0;; it++) {
+    for (int it = 0;; it += 2) {
         if (it >= 64) return X.fail(CULS_E_INVALID, "rw: redundancy sweep did not converge");
-        RedArgs A{M, w.gidAll, w.dg, w.L0, pre1, st, in1, inR, P1[cur], NR[cur], changed, X.status};
-        if ((rc = X.check(cudaMemsetAsync(changed, 0, sizeof(int), s), "memset"))) return rc;
-        k_redundancy<<<X.grid(M), kBlock, 0, s>>>(A);
-        X.launched(1);
-        if ((rc = X.check(cudaMemcpyAsync(X.hostSmall + 24, changed, sizeof(int), cudaMemcpyDeviceToHost, s), "d2h")))
-            return rc;
-        if ((rc = X.sync())) return rc;
-        in1 = P1[cur];
-        inR = NR[cur];
-        cur ^= 1;
-        if (!X.hostSmall[24]) break;
+        if ((rc = X.check(cudaMemsetAsync(changed, 0, sizeof(int) * 2, s), "memset"))) return rc;
+        for (int k = 0; k < 2; k++) {
+            RedArgs A{M, w.gidAll, w.dg, w.L0, pre1, st, in1, inR, P1[cur], NR[cur], changed + k, X.status};
+            k_redundancy<<<X.grid(M), kBlock, 0, s>>>(A);
+            in1 = P1[cur];
+            inR = NR[cur];
+            cur ^= 1;
+        }
+        X.launched(2);
+        if ((rc = X.fetch("rw choice and redundancy"))) return rc;
+        if (!X.hostSmall[25]) break;
     }
     // (in1, inR) is a fix-point: sweeping it again reproduces it
     RedArgs F{M, w.gidAll, w.dg, w.L0, pre1, st, in1, inR, nullptr, nullptr, changed, X.status};
     k_redundancy_finish<<<X.grid(std::max<int64_t>(M, w.nPO)), kBlock, 0, s>>>(F, w.L0, w.L1, w.del, w.nPO, w.wpo);
     X.launched(1);
-    if ((rc = X.sync())) return rc;
-    return X.status_check("rw redundancy");
+    if (stats) {
+        const int64_t nAnd = w.N - w.nL0, nCand = w.nCand, nRep = w.nRep;
+        unsigned long long hs[8], warpPairs;
+        memcpy(hs, X.hostSmall + kCtStats, sizeof hs);
+        memcpy(&warpPairs, X.hostSmall + kCtPairs, sizeof warpPairs);
+        stats->replaced = (long long)hs[0];
+        stats->replacedPos = (long long)hs[1];
+        stats->replacedZero = (long long)hs[2];
+        stats->reverted = (long long)hs[3];
+        stats->compromised = (long long)hs[4];
+        stats->newIdx = nCand - nRep;
+        stats->expected = (long long)hs[6];
+        stats->preEval = nAnd - nCand;
+        stats->smallCut = 0;
+        stats->newNodes = w.nNew;
+        stats->candidates = nCand;
+        stats->warpPairs = (long long)warpPairs;
+    }
+    return 0;
 }
 
 }  // namespace culs

@@ -221,9 +221,11 @@ __device__ __forceinline__ void fetch_slot(int src, int4 L, int2 M, int2 X, RCut
 // a mask in every lane, FindCut is its first clear bit or a min over the
 // slots, CutFilter two ballots of precomputed bits.
 //
-// Bound: the node's latency on a narrow level.  Comparing the leaves inside
-// the policy loop took 0.38 us a pair and the 64x64 multiplier (15 pairs a
-// node, 501 levels) 15.9 us a level.
+// Bound: the node's latency on a narrow level, of which building the
+// candidates takes 1.9 us, comparing them 1.0, the policy 1.6 (0.11 a pair)
+// and publishing 1.2.  With the leaves compared inside the policy loop a pair
+// took 0.18 us (0.38 while acquire polls slowed it) and the 64x64 multiplier
+// (15 pairs a node, 501 levels) 15.9 us a level; now 8.4.
 __device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int lane, WarpCands &W) {
     const unsigned F = 0xffffffffu;
     constexpr int kTrivial = 64 + 63;  // the trivial cut's index: bit 63 of the relations
@@ -578,12 +580,12 @@ int rw_enumerate(ExecCtx &X, RwWork &w) {
     w.cutM = X.ar->get<int2>(N * 8);
     w.cutA = X.ar->get<int2>(N * 8);
     int *done = X.ar->get<int>(N);
-    w.warpPairs = X.ar->get<unsigned long long>(1);
-    if (!w.cutL || !w.cutM || !w.cutA || !done || !w.warpPairs)
+    unsigned long long *warpPairs = reinterpret_cast<unsigned long long *>(X.counters + kCtPairs);
+    if (!w.cutL || !w.cutM || !w.cutA || !done)
         return X.fail(CULS_E_OOM, "rw: scratch arena exhausted (cuts)");
     int rc;
     if ((rc = X.check(cudaMemsetAsync(w.cutM, 0, sizeof(int2) * N * 8, s), "memset"))) return rc;
-    if ((rc = X.check(cudaMemsetAsync(w.warpPairs, 0, sizeof(unsigned long long), s), "memset"))) return rc;
+    if ((rc = X.check(cudaMemsetAsync(warpPairs, 0, sizeof(unsigned long long), s), "memset"))) return rc;
     const std::vector<EnumRun> runs = enum_runs(w.lvlCnt, X.tune->enumWideMin);
     // per run: its claim counter and, if wide, its levels' starts and chunks
     const int nRuns = (int)runs.size();
@@ -611,7 +613,7 @@ int rw_enumerate(ExecCtx &X, RwWork &w) {
         const EnumRun &r = runs[k];
         const int n = r.l1 - r.l0;
         EnumArgs A{lvlStart[r.l0], lvlStart[r.l1], n,        table,    table + n + 1, w.w0, w.w1, w.ref,
-                   w.lidLow,       w.cutL,         w.cutM,   w.cutA,   done,          dev + k, w.warpPairs, X.status};
+                   w.lidLow,       w.cutL,         w.cutM,   w.cutA,   done,          dev + k, warpPairs, X.status};
         const int64_t width = (A.q1 - A.q0) / n + 1;
         // a wide run fills the GPU; a narrow one runs about sixteen levels'
         // worth of nodes at a time

@@ -324,10 +324,7 @@ int rw_evaluate(ExecCtx &X, RwWork &w, const Batch &b) {
         X.launched(1);
     }
     if ((rc = X.check(compact_flags(candFlag, N, w.cand, X.counters + 8, *X.ar, s), "compact"))) return rc;
-    if ((rc = X.check(cudaMemcpyAsync(X.hostSmall + 8, X.counters + 8, sizeof(int), cudaMemcpyDeviceToHost, s), "d2h")))
-        return rc;
-    if ((rc = X.sync())) return rc;
-    if ((rc = X.status_check("rw evaluate"))) return rc;
+    if ((rc = X.fetch("rw evaluate"))) return rc;
     w.nCand = X.hostSmall[8];
     return 0;
 }

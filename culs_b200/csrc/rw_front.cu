@@ -215,9 +215,7 @@ int rw_front(ExecCtx &X, Batch &b, RwWork &w) {
     }
     k_front_keys<<<X.grid(N), kBlock, 0, s>>>(N, lp, keys, vals);
     X.launched(3);
-    if ((rc = X.check(cudaMemcpyAsync(X.hostSmall, cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h"))) return rc;
-    if ((rc = X.sync())) return rc;
-    if ((rc = X.status_check("rw levelize"))) return rc;
+    if ((rc = X.fetch("rw levelize"))) return rc;
     if (X.hostSmall[2]) return X.fail(CULS_E_INVALID, "rw levelize: fanins do not precede their node");
     w.maxLevel = X.hostSmall[1];
     int bits = 1;

@@ -68,6 +68,7 @@ __global__ void k_proc_order(int64_t N, int64_t M, const int *wlev, const int *o
         const int64_t pos = x < N ? x + newStart[wlev[x]] : lvEnd[ownLev[x - N]] + (x - N);
         if (pos < 0 || pos >= M) {
             set_status(status, kDevBadGraph);
+            posOf[x] = 0;  // in range for the passes until the status is read
             continue;
         }
         inv[pos] = (int)x;
@@ -164,9 +165,10 @@ int Engine::rw(Batch &b, bool useZeros, bool gpuDedup, RwStats *stats, RwDump *d
             cudaMemcpy(dump->newF1.data(), w.L1 + N, sizeof(int) * w.nNew, cudaMemcpyDeviceToHost);
         }
     }
-    if ((rc = rw_choice(X, b, w, stats))) return rc;
+    if ((rc = rw_choice(X, b, w))) return rc;
     X.mark(kMkChoice);
     if (wantDump) {
+        if ((rc = X.sync())) return rc;
         std::vector<int> cand(w.nCand), ch(w.nCand), lev(N);
         if (w.nCand) {
             cudaMemcpy(cand.data(), w.cand, sizeof(int) * w.nCand, cudaMemcpyDeviceToHost);
@@ -178,7 +180,7 @@ int Engine::rw(Batch &b, bool useZeros, bool gpuDedup, RwStats *stats, RwDump *d
             if (lev[q] > 0) dump->choice[q] = kChNoCut;
         for (int64_t c = 0; c < w.nCand; c++) dump->choice[cand[c]] = ch[c];
     }
-    if ((rc = rw_redundancy(X, b, w))) return rc;
+    if ((rc = rw_redundancy(X, b, w, stats))) return rc;
     X.mark(kMkRedund);
     const int64_t M = N + w.nNew;
     int *o0 = ar_.get<int>(M), *o1 = ar_.get<int>(M), *opo = ar_.get<int>(b.nPO + 1);
@@ -194,7 +196,6 @@ int Engine::rw(Batch &b, bool useZeros, bool gpuDedup, RwStats *stats, RwDump *d
     k_new_starts<<<X.grid(w.nNew + 1), kBlock, 0, s_>>>(w.nNew, w.newOwnLev, w.maxLevel, newStart);
     k_proc_order<<<X.grid(M), kBlock, 0, s_>>>(N, M, w.wlev, w.newOwnLev, lvEnd, newStart, procInv, procPos, status_);
     launches_ += 3;
-    if ((rc = X.sync()) || (rc = X.status_check("rw dedup order"))) return rc;
     if (gpuDedup) {
         // updateFromRewriteManager(2): GPU strash, which also ends the
         // rewrite manager's state (src/aig_manager.cu:523-546)

@@ -44,7 +44,8 @@ struct RepArgs {
 };
 
 // Recomputes the match of ReplaceSubgr for candidate c and walks BuildSubgr's
-// visit order.  With fill == false only the count is written.
+// visit order.  With fill == false only the count and the greatest depth are
+// written.
 __device__ void rep_candidate(const RepArgs &A, int c, bool fill) {
     const int q = A.cand[c];
     const int slot = A.bestCut[q];
@@ -95,7 +96,7 @@ __device__ void rep_candidate(const RepArgs &A, int c, bool fill) {
     // a built node's match becomes -(2 + post-order index).
     int stk[56], st[56];
     int depth[54];
-    int sp = 0, nb = 0;
+    int sp = 0, nb = 0, deepest = 0;
     const int T0 = fill ? A.koff[c] : 0;
     stk[0] = rt;
     st[0] = 0;
@@ -124,19 +125,19 @@ __device__ void rep_candidate(const RepArgs &A, int c, bool fill) {
         int in0 = ln_f0(w), in1 = ln_f1(w);
         int idx = nb++;
         match[cur] = -(2 + idx);
+        const int m0 = match[in0], m1 = match[in1];
+        const int d0 = m0 <= -2 ? depth[-m0 - 2] : 0;
+        const int d1 = m1 <= -2 ? depth[-m1 - 2] : 0;
+        depth[idx] = 1 + (d0 > d1 ? d0 : d1);
+        deepest = depth[idx] > deepest ? depth[idx] : deepest;
         if (fill) {
             int T = T0 + idx;
-            int m0 = match[in0], m1 = match[in1];
-            int d0 = m0 <= -2 ? depth[-m0 - 2] : 0;
-            int d1 = m1 <= -2 ? depth[-m1 - 2] : 0;
-            depth[idx] = 1 + (d0 > d1 ? d0 : d1);
             A.recCand[T] = c;
             A.r0[T] = m0 >= 0 ? m0 : -(T0 + (-m0 - 2)) - 1;
             A.r1[T] = m1 >= 0 ? m1 : -(T0 + (-m1 - 2)) - 1;
             A.rc0[T] = (uint8_t)((in0 < 4 ? ((isC >> in0) & 1) : 0) ^ ln_c0(w));
             A.rc1[T] = (uint8_t)((in1 < 4 ? ((isC >> in1) & 1) : 0) ^ ln_c1(w));
             A.depth[T] = depth[idx];
-            atomicMax(A.maxDepth, depth[idx]);
         }
         sp--;
     }
@@ -145,6 +146,7 @@ __device__ void rep_candidate(const RepArgs &A, int c, bool fill) {
         A.rootRef[c] = m >= 0 ? m : -(T0 + (-m - 2)) - 1;
     } else {
         A.kcnt[c] = nb;
+        agg_max(A.maxDepth, 0, deepest);
     }
 }
 
@@ -377,10 +379,9 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
     k_rep_count<<<X.grid(nCand, 64), 64, 0, s>>>(nCand, A);
     X.launched(1);
     if ((rc = X.check(scan_exclusive(kcnt, koff, nCand, cnt + 0, ar, s), "scan"))) return rc;
-    if ((rc = X.check(cudaMemcpyAsync(X.hostSmall + 16, cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h")))
-        return rc;
-    if ((rc = X.sync())) return rc;
+    if ((rc = X.fetch("rw replace match"))) return rc;
     const int64_t K = X.hostSmall[16];
+    const int maxDepth = X.hostSmall[17];
     if (N + K >= (1ll << 29)) return X.fail(CULS_E_INVALID, "rw: batch too large for 30-bit node positions");
     int *recCand = ar.get<int>(K + 1), *r0 = ar.get<int>(K + 1), *r1 = ar.get<int>(K + 1), *depth = ar.get<int>(K + 1);
     uint8_t *rc0 = ar.get<uint8_t>(K + 1), *rc1 = ar.get<uint8_t>(K + 1);
@@ -402,11 +403,6 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
     A.rc1 = rc1;
     k_rep_fill<<<X.grid(nCand, 64), 64, 0, s>>>(nCand, A);
     X.launched(1);
-    if ((rc = X.check(cudaMemcpyAsync(X.hostSmall + 16, cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h")))
-        return rc;
-    if ((rc = X.sync())) return rc;
-    if ((rc = X.status_check("rw replace match"))) return rc;
-    const int maxDepth = X.hostSmall[17];
     if ((rc = X.check(and_table_clear(ts, cap, s), "fill"))) return rc;
     MergeArgs Mg{N, K, r0, r1, depth, rc0, rc1, w.wph, canon, nph, f0, f1, c0, c1, slot, AndTable{ts, cap - 1},
                  X.status};
@@ -422,16 +418,14 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
                                                      X.status);
     X.launched(3);
     if ((rc = X.check(scan_exclusive(kp, kpo, nCand, cnt + 2, ar, s), "scan"))) return rc;
-    if ((rc = X.check(cudaMemcpyAsync(X.hostSmall + 16, cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h")))
-        return rc;
-    if ((rc = X.sync())) return rc;
-    const int64_t nNew = X.hostSmall[18];
     if ((rc = X.check(fill_i32(newPos, -1, K, s), "fill"))) return rc;
     k_rep_rebuild<<<X.grid(nCand, 64), 64, 0, s>>>(nCand, N, rootRef, canon, f0, f1, owner, nullptr, kpo, newPos,
                                                      X.status);
     X.launched(1);
-    if ((rc = rep_extend_only(X, w, nNew))) return rc;
-    w.newOwnLev = ar.get<int>(nNew + 1);
+    // the new nodes' number is read with the last fetch: their arrays get
+    // room for all K, of which they are the first nNew
+    if ((rc = rep_extend_only(X, w, K))) return rc;
+    w.newOwnLev = ar.get<int>(K + 1);
     if (!w.newOwnLev) return X.fail(CULS_E_OOM, "rw: arena exhausted (replace)");
     if (K > 0)
         k_rep_newnodes<<<X.grid(K), kBlock, 0, s>>>(K, N, canon, f0, f1, c0, c1, newPos, owner, w.cand, w.wg, w.wlev,
@@ -439,11 +433,10 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
     k_rep_final<<<X.grid(nCand), kBlock, 0, s>>>(nCand, N, repT, newPos, w.repW, hasRep);
     X.launched(2);
     if ((rc = X.check(compact_flags(hasRep, nCand, w.withRep, cnt + 3, ar, s), "compact"))) return rc;
-    if ((rc = X.check(cudaMemcpyAsync(X.hostSmall + 16, cnt, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h")))
-        return rc;
-    if ((rc = X.sync())) return rc;
+    if ((rc = X.fetch("rw replace"))) return rc;
+    w.nNew = X.hostSmall[18];
     w.nRep = X.hostSmall[19];
-    return X.status_check("rw replace");
+    return 0;
 }
 
 }  // namespace culs

@@ -13,12 +13,26 @@
 
 namespace culs {
 
+// The context's device counters, copied to the host together by fetch().
+enum CounterIndex : int {
+    kCtFree = 0,      // [0, 64): each stage's own
+    kCtStatus = 64,   // status word and spin bound
+    kCtRound = 72,    // the strash's hashing rounds: changed, by round (kMaxHashRounds), then
+    kCtInserted = 136,
+    kCtFull = 137,
+    kCtStats = 144,   // the choice's statistics: eight 64-bit counters
+    kCtPairs = 160,   // RwStats::warpPairs, 64 bits
+    kCounters = 176,
+};
+constexpr int kMaxHashRounds = 64;
+static_assert(kCtRound + kMaxHashRounds <= kCtInserted, "hashing rounds");
+
 struct ExecCtx {
     cudaStream_t s = nullptr;
     Arena *ar = nullptr;
     int *status = nullptr;    // device status word
-    int *counters = nullptr;  // 64 device ints of scratch
-    int *hostSmall = nullptr; // 64 pinned host ints
+    int *counters = nullptr;  // kCounters device ints
+    int *hostSmall = nullptr; // their host copy as of the last fetch
     const RwLib *lib = nullptr;
     int sms = 148;
     int *launches = nullptr;
@@ -43,8 +57,9 @@ struct ExecCtx {
         return CULS_E_DEVICE;
     }
     int sync() { return check(cudaStreamSynchronize(s), "stream sync"); }
-    // Reads the device status word (after a sync) and maps it to an error.
-    int status_check(const char *what);
+    // Copies the counters to the host, waits for the stream and maps the
+    // device status word to an error.
+    int fetch(const char *what);
     void launched(int k = 1) {
         if (launches) *launches += k;
     }
@@ -63,7 +78,6 @@ struct RwWork {
     int maxLevel = 0;
     std::vector<int> lvlCnt;  // AND nodes per level
     int64_t width = 1;  // Batch::flow_width of the batch: nodes a level-ordered pass can work on at once
-    unsigned long long *warpPairs = nullptr;  // device counter (RwStats::warpPairs)
     bool useZeros = false;
     DevGraph *dg = nullptr;  // device graph table (cpos = constant's W position)
 
@@ -113,7 +127,7 @@ int rw_front(ExecCtx &X, Batch &b, RwWork &w);     // levelize, reorder, refs
 int rw_enumerate(ExecCtx &X, RwWork &w);           // cut enumeration
 int rw_evaluate(ExecCtx &X, RwWork &w, const Batch &b);  // table + evaluation + candidates
 int rw_replace(ExecCtx &X, Batch &b, RwWork &w);   // subgraph build + rebuild ids
-int rw_choice(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats);  // sequential choice per graph
-int rw_redundancy(ExecCtx &X, Batch &b, RwWork &w);  // buffer chasing
+int rw_choice(ExecCtx &X, Batch &b, RwWork &w);    // sequential choice per graph
+int rw_redundancy(ExecCtx &X, Batch &b, RwWork &w, RwStats *stats);  // buffer chasing; the choice's statistics
 
 }  // namespace culs

@@ -694,7 +694,7 @@ __global__ void k_winner_local(int64_t n, const int *wlByG, const int *srt, cons
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
         int t = wlByG[i];
         int g = gid[srt[t]];
-        newLocalT[t] = dg[g].nPIs + 1 + (int)(i - gStart[g]);
+        newLocalT[t] = dg[g].nPIs + 1 + (int)(i - (gStart ? gStart[g] : 0));
     }
 }
 
@@ -704,8 +704,7 @@ struct OutArgs {
     const int *po;
     const DevGraph *dgNew;
     int *F0, *F1, *PO;
-    int64_t nPO;
-    int G;
+    int64_t nPO, M;
 };
 
 __device__ __forceinline__ int local_lit(const OutArgs &A, int lit) {
@@ -726,6 +725,12 @@ __global__ void k_strash_out(int64_t nW, const int *wl, OutArgs A) {
         int a = local_lit(A, A.kl0[t]), b = local_lit(A, A.kl1[t]);
         A.F0[p] = a < b ? a : b;
         A.F1[p] = a < b ? b : a;
+    }
+    // the constants and PIs
+    for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < A.M; v += stride) {
+        if (A.L0[v] >= 0) continue;
+        const int p = A.dgNew[A.gid[v]].base + A.lidIn[v];
+        A.F0[p] = A.F1[p] = -1;
     }
     for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < A.nPO; k += stride) {
         int lit = A.po[k];
@@ -748,7 +753,6 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     const int G = b.G;
     const int64_t nPO = b.nPO;
     cudaStream_t s = s_;
-    size_t mark = ar_.used();
     int *cnt = ar_.get<int>(M + 1);
     uint8_t *dead = ar_.get<uint8_t>(M + 1);
     uint8_t *flags = ar_.get<uint8_t>(M + 1);
@@ -835,8 +839,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
             A.depth0 = qc + 4, A.depth1 = graphLevels, A.unsettled = qc + 6, A.status = qc + 7;
             check(levels_block(A, s), "levels");
             launches_ += 2;
-            check(cudaMemcpyAsync(hostSmall_, qc, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h");
-            if (int e = sync()) return e;
+            if (int e = fetch("strash levels")) return e;
             leveled = hostSmall_[6] == 0 && hostSmall_[7] == 0;
         } else
         for (int pass = 0; pass < 64; pass++) {
@@ -846,8 +849,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
             k_unresolved_flags<<<grid_1d(n, kBlock, sms_ * 16), kBlock, 0, s>>>(n, list, done, flags);
             launches_ += 2;
             check(compact_flags(flags, n, idx, qc + 6, ar_, s), "compact");
-            check(cudaMemcpyAsync(hostSmall_, qc, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h");
-            if (int e = sync()) return e;
+            if (int e = fetch("strash levels")) return e;
             const int64_t nu = hostSmall_[6];
             if (hostSmall_[7] != 0) break;  // a wait timed out
             if (nu == 0) {
@@ -861,11 +863,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
             list = next;
             n = nu;
         }
-        if (leveled) {
-            // every live node has its level
-            check(cudaMemcpyAsync(qc + 1, qc + 3, sizeof(int), cudaMemcpyDeviceToDevice, s), "copy");
-            if (prof_) this->mark(kMkLevelK1);
-        }
+        if (leveled && prof_) this->mark(kMkLevelK1);
     }
     if (!leveled) {
     check(cudaMemsetAsync(off, 0, sizeof(int) * (M + 2), s), "memset");
@@ -904,16 +902,17 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     }
     check(cudaMemcpyAsync(qc + 1, ring + 3 + L % 3, sizeof(int), cudaMemcpyDeviceToDevice, s), "copy");
     if (prof_) this->mark(kMkLevelK1);
+    if (int e = fetch("strash levels")) return e;
+    if (hostSmall_[1] != hostSmall_[3]) return fail(CULS_E_INVALID, "strash: the AIG has a cycle");
     }
     }
     // 3. processing order (level, position) and tentative ranks
-    check(cudaMemcpyAsync(hostSmall_, qc, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h");
-    if (int e = sync()) return e;
-    if (int e = check_status("strash levels")) return e;
-    int64_t nLive = hostSmall_[3];
-    int maxLevel = hostSmall_[4];
-    if (topo && hostSmall_[6]) return fail(CULS_E_INVALID, "strash: fanins do not precede their node");
-    if (!topo && hostSmall_[1] != nLive) return fail(CULS_E_INVALID, "strash: the AIG has a cycle");
+    if (topo) {
+        if (int e = fetch("strash levels")) return e;
+        if (hostSmall_[6]) return fail(CULS_E_INVALID, "strash: fanins do not precede their node");
+    }
+    const int64_t nLive = hostSmall_[3];
+    const int maxLevel = hostSmall_[4];
     int *srt = ar_.get<int>(nLive + 1);
     uint32_t *keys = ar_.get<uint32_t>(nLive + 1);
     uint32_t *keys2 = ar_.get<uint32_t>(nLive + 1);
@@ -928,7 +927,6 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     if (!srt || !keys || !keys2 || !vals2 || !lvlCnt || !lvlDone || !lvlStart || !chunkCnt || !chunkStart)
         return fail(CULS_E_OOM, "strash: arena exhausted");
     check(cudaMemsetAsync(lvlCnt, 0, sizeof(int) * (maxLevel + 2), s), "memset");
-    check(cudaMemsetAsync(lvlDone, 0, sizeof(int) * (maxLevel + 2), s), "memset");
     if (nLive > 0) {
         unsigned gl = grid_1d(nLive, kBlock, sms_ * 16);
         k_gather_levels<<<gl, kBlock, 0, s>>>(nLive, liveIdx, level, keys, lvlCnt, maxLevel + 1);
@@ -939,11 +937,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         k_inverse<<<gl, kBlock, 0, s>>>(nLive, srt, tOf);
         // tentative rank: processing order, or id order for the CPU variants
         k_inverse<<<gl, kBlock, 0, s>>>(nLive, idOrder ? liveIdx : srt, rankOf);
-        // level-aligned chunks for the hashing dataflow
-        k_level_chunks<<<grid_1d(maxLevel + 1, kBlock, sms_ * 16), kBlock, 0, s>>>(maxLevel + 1, lvlCnt, chunkCnt);
-        launches_ += 4;
-        check(scan_exclusive(lvlCnt, lvlStart, maxLevel + 1, nullptr, ar_, s), "scan");
-        check(scan_exclusive(chunkCnt, chunkStart, maxLevel + 1, chunkStart + maxLevel + 1, ar_, s), "scan");
+        launches_ += 3;
     }
     // 4. hash: fixed-point rounds or the level dataflow (below)
     uint32_t cap = 1024;
@@ -965,7 +959,6 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     uint8_t *wflags = ar_.get<uint8_t>(nLive + 1);
     int *wl = ar_.get<int>(nLive + 1);
     if (!ts || !mapEnc || !kl0 || !kl1 || !wflags || !wl) return fail(CULS_E_OOM, "strash: arena exhausted");
-    check(cudaMemsetAsync(qc + 5, 0, sizeof(int), s), "memset");
     // Rounds (k_round_*) for batches of up to 16M live nodes, where a full
     // pass and a few light ones cost less than one wait latency per level
     // (the 10M-AND single graph: each strash 22 -> 6 ms); the level dataflow
@@ -974,7 +967,6 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     // settle within kMaxRounds.  CULS_DEDUP_MODE=levels|rounds forces either
     // (the tests run both on the same graphs).
     constexpr int64_t kRoundsMaxLive = 16ll << 20;
-    constexpr int kMaxRounds = 64;
     bool useRounds = nLive > 0 && nLive <= kRoundsMaxLive;
     if (const char *env = getenv("CULS_DEDUP_MODE")) {
         if (!strcmp(env, "levels")) useRounds = false;
@@ -985,24 +977,25 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     int *slotT = ar_.get<int>(nLive + 1);
     if (!slotT) return fail(CULS_E_OOM, "strash: arena exhausted");
     if (useRounds) {
-        int *cur = ar_.get<int>(M + 1), *flag = ar_.get<int>(kMaxRounds + 2);  // changed per round; inserted, full
+        int *cur = ar_.get<int>(M + 1), *flag = counters_ + kCtRound;
         const size_t posWords = (size_t)M / 32 + 1, slotWords = (size_t)cap / 32 + 1;
         uint32_t *ch[2] = {ar_.get<uint32_t>(posWords), ar_.get<uint32_t>(posWords)};
         uint32_t *slotBits = ar_.get<uint32_t>(slotWords);
-        if (!cur || !flag || !ch[0] || !ch[1] || !slotBits) return fail(CULS_E_OOM, "strash: arena exhausted");
+        if (!cur || !ch[0] || !ch[1] || !slotBits) return fail(CULS_E_OOM, "strash: arena exhausted");
         const unsigned gl = grid_1d(nLive, kBlock, sms_ * 16);
         if (prof_) this->mark(kMkDedupK0);
         k_round_init<<<gl, kBlock, 0, s>>>(nLive, srt, cur);
         launches_ += 1;
         RoundArgs R{nLive, M,   srt,    tOf, rankOf, liveFlag, L0, L1, gidA, b.dg, AndTable{ts, cap - 1}, cur, slotT,
                     mapEnc, kl0, kl1,   foldTrivial ? 1 : 0, unique ? 1 : 0, nullptr, nullptr, slotBits, nullptr, nullptr,
-                    flag + kMaxRounds, (int)(cap / 4), flag + kMaxRounds + 1, status_};
-        check(cudaMemsetAsync(flag, 0, sizeof(int) * (kMaxRounds + 2), s), "memset");
+                    counters_ + kCtInserted, (int)(cap / 4), counters_ + kCtFull, status_};
+        check(cudaMemsetAsync(flag, 0, sizeof(int) * kMaxHashRounds, s), "memset");
         bool all = true;  // the next round takes all nodes
-        for (int r = 0; r < kMaxRounds && !settled;) {
-            // all nodes: one round; later rounds three at a time (one that
-            // follows a round without a change does nothing)
-            const int first = r, last = all ? r + 1 : std::min(r + 3, kMaxRounds);
+        for (int r = 0; r < kMaxHashRounds && !settled;) {
+            // per host check three rounds, or one over all nodes where
+            // nothing is expected to merge (a round that follows one without
+            // a change does nothing)
+            const int first = r, last = std::min(all && topo ? r + 1 : r + 3, kMaxHashRounds);
             for (; r < last; r++) {
                 R.chIn = ch[(r + 1) & 1], R.chOut = ch[r & 1];
                 R.prev = r > 0 ? flag + r - 1 : nullptr;
@@ -1013,6 +1006,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
                     check(cudaMemsetAsync(R.inserted, 0, sizeof(int) * 2, s), "memset");
                     k_round_insert<<<gl, kBlock, 0, s>>>(R);
                     k_round_resolve<<<gl, kBlock, 0, s>>>(R);
+                    all = false;
                 } else {
                     check(cudaMemsetAsync(slotBits, 0, sizeof(uint32_t) * slotWords, s), "memset");
                     k_round_rekey<<<gridM, kBlock, 0, s>>>(R);
@@ -1020,14 +1014,10 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
                 }
                 launches_ += 2;
             }
-            check(cudaMemcpyAsync(hostSmall_ + 8, flag + first, sizeof(int) * (last - first), cudaMemcpyDeviceToHost, s),
-                  "d2h");
-            check(cudaMemcpyAsync(hostSmall_ + 16, R.full, sizeof(int), cudaMemcpyDeviceToHost, s), "d2h");
-            if (int e = sync()) return e;
-            if (int e = check_status("strash hashing")) return e;
-            all = hostSmall_[16] != 0;
+            if (int e = fetch("strash hashing")) return e;
+            all = hostSmall_[kCtFull] != 0;
             for (int k = first; k < last && !settled && !all; k++)
-                if (hostSmall_[8 + k - first] == 0) {
+                if (hostSmall_[kCtRound + k] == 0) {
                     settled = true;
                     hashRounds_ = k + 1;
                 }
@@ -1035,6 +1025,13 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         if (prof_) this->mark(kMkDedupK1);
     }
     if (nLive > 0 && !settled) {
+        // level-aligned chunks for the hashing dataflow
+        check(cudaMemsetAsync(lvlDone, 0, sizeof(int) * (maxLevel + 2), s), "memset");
+        check(cudaMemsetAsync(qc + 5, 0, sizeof(int), s), "memset");
+        k_level_chunks<<<grid_1d(maxLevel + 1, kBlock, sms_ * 16), kBlock, 0, s>>>(maxLevel + 1, lvlCnt, chunkCnt);
+        check(scan_exclusive(lvlCnt, lvlStart, maxLevel + 1, nullptr, ar_, s), "scan");
+        check(scan_exclusive(chunkCnt, chunkStart, maxLevel + 1, chunkStart + maxLevel + 1, ar_, s), "scan");
+        launches_ += 1;
         check(and_table_clear(ts, cap, s), "fill");
         DedupArgs A{nLive,      srt,      rankOf,
                     L0,         L1,       level,   lvlCnt,
@@ -1054,10 +1051,8 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     check(compact_flags(wflags, nLive, wl, qc + 6, ar_, s), "compact");
     // In id order (CPU variants) the winners are ranked by position, not by
     // processing order: sort the winner list by rank.
-    check(cudaMemcpyAsync(hostSmall_, qc, sizeof(int) * 8, cudaMemcpyDeviceToHost, s), "d2h");
-    if (int e = sync()) return e;
-    if (int e = check_status("strash hashing")) return e;
-    int64_t nW = hostSmall_[6];
+    if (int e = fetch("strash hashing")) return e;
+    const int64_t nW = hostSmall_[6];
     int *newLocalT = ar_.get<int>(nLive + 1);
     int *cntG = ar_.get<int>(G + 1);
     int *gStart = ar_.get<int>(G + 1);
@@ -1075,25 +1070,28 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         check(radix_sort_pairs(wk, wv, wk2, wl, nW, bits, ar_, s), "sort");
         launches_ += 1;
     }
-    check(cudaMemsetAsync(cntG, 0, sizeof(int) * (G + 1), s), "memset");
-    if (nW > 0) {
-        unsigned gw = grid_1d(nW, kBlock, sms_ * 16);
-        k_winner_keys<<<gw, kBlock, 0, s>>>(nW, wl, srt, gidA, wk, cntG);
-        launches_ += 1;
-        if (G > 1) {
+    std::vector<int> hCnt(G), hLev(G);
+    if (G == 1) {
+        hCnt[0] = (int)nW;
+        hLev[0] = maxLevel;
+        wlByG = wl;
+        gStart = nullptr;
+    } else {
+        check(cudaMemsetAsync(cntG, 0, sizeof(int) * (G + 1), s), "memset");
+        if (nW > 0) {
+            unsigned gw = grid_1d(nW, kBlock, sms_ * 16);
+            k_winner_keys<<<gw, kBlock, 0, s>>>(nW, wl, srt, gidA, wk, cntG);
+            launches_ += 1;
             int bits = 1;
             while ((1ll << bits) < G) bits++;
             check(cudaMemcpyAsync(wv, wl, sizeof(int) * nW, cudaMemcpyDeviceToDevice, s), "copy");
             check(radix_sort_pairs(wk, wv, wk2, wlByG, nW, bits, ar_, s), "sort");
-        } else {
-            check(cudaMemcpyAsync(wlByG, wl, sizeof(int) * nW, cudaMemcpyDeviceToDevice, s), "copy");
         }
+        check(scan_exclusive(cntG, gStart, G, nullptr, ar_, s), "scan");
+        check(cudaMemcpyAsync(hCnt.data(), cntG, sizeof(int) * G, cudaMemcpyDeviceToHost, s), "d2h");
+        check(cudaMemcpyAsync(hLev.data(), graphLevels, sizeof(int) * G, cudaMemcpyDeviceToHost, s), "d2h");
+        if (int e = sync()) return e;
     }
-    check(scan_exclusive(cntG, gStart, G, nullptr, ar_, s), "scan");
-    std::vector<int> hCnt(G), hLev(G);
-    check(cudaMemcpyAsync(hCnt.data(), cntG, sizeof(int) * G, cudaMemcpyDeviceToHost, s), "d2h");
-    check(cudaMemcpyAsync(hLev.data(), graphLevels, sizeof(int) * G, cudaMemcpyDeviceToHost, s), "d2h");
-    if (int e = sync()) return e;
     // new graph table
     std::vector<DevGraph> ng = b.hg;
     int64_t base = 0;
@@ -1113,25 +1111,21 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     if (int e = check(b.reserve_spare(nObjNew + 1, nPO + 1), "cudaMalloc")) return e;
     int *F0n = b.F0s, *F1n = b.F1s, *POn = b.POs;
     check(cudaMemcpyAsync(dgNew, ng.data(), sizeof(DevGraph) * G, cudaMemcpyHostToDevice, s), "h2d");
-    check(fill_i32(F0n, -1, nObjNew, s), "fill");
-    check(fill_i32(F1n, -1, nObjNew, s), "fill");
     if (nW > 0) {
         unsigned gw = grid_1d(nW, kBlock, sms_ * 16);
         k_winner_local<<<gw, kBlock, 0, s>>>(nW, wlByG, srt, gidA, gStart, b.dg, newLocalT);
         launches_ += 1;
     }
-    OutArgs O{srt, tOf, gidA, lidIn, L0, kl0, kl1, newLocalT, mapEnc, ts, po, dgNew, F0n, F1n, POn, nPO, G};
-    k_strash_out<<<grid_1d(std::max<int64_t>(std::max<int64_t>(nW, nPO), 1), kBlock, sms_ * 16), kBlock, 0, s>>>(nW, wl,
-                                                                                                             O);
+    OutArgs O{srt, tOf, gidA, lidIn, L0, kl0, kl1, newLocalT, mapEnc, ts, po, dgNew, F0n, F1n, POn, nPO, M};
+    k_strash_out<<<gridM, kBlock, 0, s>>>(nW, wl, O);
     launches_ += 1;
     check(cudaMemcpyAsync(b.dg, ng.data(), sizeof(DevGraph) * G, cudaMemcpyHostToDevice, s), "h2d");
-    if (int e = sync()) return e;
+    if (int e = fetch("strash output")) return e;
     b.swap_spare();
     b.hg = ng;
     b.nObj = nObjNew;
     ar_.reset();
-    (void)mark;
-    return check_status("strash output");
+    return 0;
 }
 
 namespace {
@@ -1189,8 +1183,7 @@ int Engine::batch_depth(Batch &b) {
     std::vector<int> hl(G);
     if ((rc = check(cudaMemcpyAsync(hl.data(), graphLevels, sizeof(int) * G, cudaMemcpyDeviceToHost, s), "d2h")))
         return rc;
-    if ((rc = sync())) return rc;
-    if ((rc = check_status("depth"))) return rc;
+    if ((rc = fetch("depth"))) return rc;
     for (int g = 0; g < G; g++) b.hg[g].nLevels = hl[g];
     rc = check(cudaMemcpyAsync(b.dg, b.hg.data(), sizeof(DevGraph) * G, cudaMemcpyHostToDevice, s), "h2d");
     ar_.reset();
