@@ -84,15 +84,17 @@ __global__ void __launch_bounds__(kAigThreads) k_aig_count(const uint8_t *buf, i
     }
 }
 
-// 2. index of each graph's first number: terminators before its region
+// 2. index of each graph's first number: terminators before its region.  A
+// warp per graph, since up to a tile of bytes is counted one by one.
 __global__ void k_aig_term_base(int G, const uint8_t *buf, int64_t n, const int64_t *regOff, const int64_t *tileBase,
                                 int64_t *termBase) {
-    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g <= G; g += gridDim.x * blockDim.x) {
-        const int64_t off = regOff[g];
-        const int64_t tile = off / kAigTile;
-        int64_t c = tileBase[tile];
-        for (int64_t i = tile * kAigTile; i < off && i < n; i++) c += !(buf[i] & 0x80);
-        termBase[g] = c;
+    const int lane = threadIdx.x & 31, warps = gridDim.x * (blockDim.x >> 5);
+    for (int g = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g <= G; g += warps) {
+        const int64_t off = regOff[g], tile = off / kAigTile;
+        int c = 0;
+        for (int64_t i = tile * kAigTile + lane; i < off && i < n; i += 32) c += !(buf[i] & 0x80);
+        c = __reduce_add_sync(0xffffffffu, c);
+        if (lane == 0) termBase[g] = tileBase[tile] + c;
     }
 }
 
@@ -233,14 +235,15 @@ __global__ void k_gather_i64(int n, const int64_t *idx, const long long *src, lo
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) dst[k] = src[idx[k]];
 }
 
-// Graphs [0, G) in at most `parts` contiguous runs of about equal weight,
-// each run on its own host thread (the first on the caller's).
+// Graphs [0, G) in contiguous runs of about equal weight, each run on its own
+// host thread (the first on the caller's); `grain`: the weight that is worth a
+// thread (starting one costs about 15 us).
 template <class W, class F>
-void for_runs(int G, W weight, F fn) {
+void for_runs(int G, int64_t grain, W weight, F fn) {
     int64_t total = 0;
     for (int g = 0; g < G; g++) total += weight(g);
     const unsigned hw = std::thread::hardware_concurrency();
-    const int parts = total < (1 << 20) ? 1 : (int)std::max(1u, std::min({hw ? hw : 1u, 32u, (unsigned)G}));
+    const int parts = (int)std::max<int64_t>(1, std::min({(int64_t)(hw ? hw : 1u), (int64_t)32, (int64_t)G, total / grain}));
     std::vector<int> cut{0};
     int64_t acc = 0;
     for (int g = 0; g < G; g++) {
@@ -307,8 +310,7 @@ bool read_dec(const uint8_t *&p, const uint8_t *end, long long &v) {
     return true;
 }
 
-bool parse_head(const uint8_t *data, size_t len, int &nPIs, int &nPOs, int &nAnds, std::vector<int> &outs,
-                size_t &body) {
+bool parse_head(const uint8_t *data, size_t len, int &nPIs, int &nPOs, int &nAnds, size_t &text) {
     const uint8_t *p = data, *end = data + len;
     if (len < 4 || memcmp(p, "aig ", 4) != 0) return false;
     p += 4;
@@ -322,16 +324,27 @@ bool parse_head(const uint8_t *data, size_t len, int &nPIs, int &nPOs, int &nAnd
     nPIs = (int)I;
     nPOs = (int)O;
     nAnds = (int)A;
+    text = (size_t)(p - data);
+    return true;
+}
+
+// The output lines from `text` on; body: where the numbers start.
+bool parse_outs(const uint8_t *data, size_t len, int nObjs, int nPOs, size_t text, std::vector<int> &outs, size_t &body) {
+    const uint8_t *p = data + text, *end = data + len;
+    if ((size_t)nPOs > len / 2) return false;  // an output line has at least two bytes
     outs.resize(nPOs);
     for (int i = 0; i < nPOs; i++) {
         long long lit;
         if (!read_dec(p, end, lit) || p >= end || *p++ != '\n') return false;
-        if (lit >= 2 * (M + 1)) return false;
+        if (lit >= 2 * (long long)nObjs) return false;
         outs[i] = aig_inv_const((int)lit);
     }
     body = (size_t)(p - data);
     return true;
 }
+
+// Work of one host thread: output lines (9 ns to parse, 3 ns to size), bytes.
+constexpr int64_t kLinesPerThread = 1 << 14, kBytesPerThread = 1 << 20;
 
 }  // namespace
 
@@ -341,17 +354,21 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
     std::vector<std::vector<int>> outs(count);
     std::vector<int64_t> regOff(count + 1), andBase(count + 1);
     int64_t nObj = 0, nPO = 0, nAnd = 0, bytes = 0;
-    std::vector<size_t> body(count);
+    std::vector<size_t> text(count), body(count);
     std::vector<int> head(3 * (size_t)count);
     std::atomic<int> bad{-1};
-    for_runs(count, [&](int g) { return (int64_t)len[g] / 64 + 1; }, [&](int g0, int g1) {
-        for (int g = g0; g < g1; g++)
-            if (!data[g] || !parse_head(data[g], len[g], head[3 * g], head[3 * g + 1], head[3 * g + 2], outs[g], body[g])) {
-                int none = -1;
-                bad.compare_exchange_strong(none, g);
-                return;
-            }
-    });
+    for (int g = 0; g < count && bad.load() < 0; g++)
+        if (!data[g] || !parse_head(data[g], len[g], head[3 * g], head[3 * g + 1], head[3 * g + 2], text[g])) bad = g;
+    if (bad.load() < 0)
+        for_runs(count, kLinesPerThread, [&](int g) { return (int64_t)head[3 * g + 1] + 1; }, [&](int g0, int g1) {
+            for (int g = g0; g < g1; g++)
+                if (!parse_outs(data[g], len[g], 1 + head[3 * g] + head[3 * g + 2], head[3 * g + 1], text[g], outs[g],
+                                body[g])) {
+                    int none = -1;
+                    bad.compare_exchange_strong(none, g);
+                    return;
+                }
+        });
     if (bad.load() >= 0) return fail(CULS_E_IO, "upload: not binary AIGER (graph " + std::to_string(bad.load()) + ")");
     for (int g = 0; g < count; g++) {
         const int nPIs = head[3 * g], nPOs = head[3 * g + 1], nAnds = head[3 * g + 2];
@@ -371,12 +388,6 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
     if ((rc = ensure_stage((size_t)(bytes + 3) / 4 + (size_t)nPO + 1))) return rc;
     uint8_t *sB = reinterpret_cast<uint8_t *>(stage_);
     int32_t *sPO = stage_ + (bytes + 3) / 4;
-    for_runs(count, [&](int g) { return regOff[g + 1] - regOff[g] + 1; }, [&](int g0, int g1) {
-        for (int g = g0; g < g1; g++) {
-            memcpy(sB + regOff[g], data[g] + body[g], len[g] - body[g]);
-            if (!outs[g].empty()) memcpy(sPO + hg[g].poOff, outs[g].data(), sizeof(int32_t) * outs[g].size());
-        }
-    });
     if (!b.pool) b.pool = pool_;
     if ((rc = check(b.reserve(nObj, nPO, count), "cudaMalloc"))) return rc;
     const int64_t nTiles = (bytes + kAigTile - 1) / kAigTile;
@@ -393,9 +404,18 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
         return fail(CULS_E_OOM, "upload: arena exhausted (AIGER)");
     cudaStream_t s = s_;
     ExecCtx X = ctx();
-    if ((rc = check(cudaMemcpyAsync(dB, sB, (size_t)bytes, cudaMemcpyHostToDevice, s), "h2d"))) return rc;
-    if (nPO && (rc = check(cudaMemcpyAsync(b.PO, sPO, sizeof(int32_t) * nPO, cudaMemcpyHostToDevice, s), "h2d")))
-        return rc;
+    // a run's copies follow its staging and overlap the other runs'
+    for_runs(count, kBytesPerThread, [&](int g) { return regOff[g + 1] - regOff[g] + 1; }, [&](int g0, int g1) {
+        for (int g = g0; g < g1; g++) {
+            memcpy(sB + regOff[g], data[g] + body[g], len[g] - body[g]);
+            if (!outs[g].empty()) memcpy(sPO + hg[g].poOff, outs[g].data(), sizeof(int32_t) * outs[g].size());
+        }
+        const int64_t p0 = hg[g0].poOff, p1 = g1 < count ? (int64_t)hg[g1].poOff : nPO;
+        if (regOff[g1] > regOff[g0])
+            cudaMemcpyAsync(dB + regOff[g0], sB + regOff[g0], (size_t)(regOff[g1] - regOff[g0]), cudaMemcpyHostToDevice, s);
+        if (p1 > p0) cudaMemcpyAsync(b.PO + p0, sPO + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyHostToDevice, s);
+    });
+    if ((rc = check(cudaGetLastError(), "h2d"))) return rc;
     if ((rc = check(cudaMemcpyAsync(dReg, regOff.data(), sizeof(int64_t) * (count + 1), cudaMemcpyHostToDevice, s),
                     "h2d")))
         return rc;
@@ -423,7 +443,7 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
     } else if ((rc = check(cudaMemsetAsync(tileBase, 0, sizeof(int64_t) * 2, s), "memset"))) {
         return rc;
     }
-    k_aig_term_base<<<grid_1d(count + 1, kBlock, sms_ * 4), kBlock, 0, s>>>(count, dB, bytes, dReg, tileBase, dTerm);
+    k_aig_term_base<<<grid_1d(32 * (count + 1), kBlock, sms_ * 4), kBlock, 0, s>>>(count, dB, bytes, dReg, tileBase, dTerm);
     if (nTiles > 0)
         k_aig_numbers<<<(unsigned)nTiles, kAigThreads, 0, s>>>(
             AigDecode{dB, bytes, tileBase, count, dReg, dTerm, dAnd, nums, status_});
@@ -501,11 +521,13 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
     if ((rc = ensure_stage((size_t)(total + 3) / 4 + (size_t)b.nPO + 1))) return rc;
     uint8_t *sB = reinterpret_cast<uint8_t *>(stage_);
     int32_t *sPO = stage_ + (total + 3) / 4;
-    if (buf && total && (rc = check(cudaMemcpyAsync(sB, dB, (size_t)total, cudaMemcpyDeviceToHost, s), "d2h")))
-        return rc;  // (the sizes need the numbers' lengths and the output literals only)
     if (b.nPO && (rc = check(cudaMemcpyAsync(sPO, b.PO, sizeof(int32_t) * b.nPO, cudaMemcpyDeviceToHost, s), "d2h")))
         return rc;
     if ((rc = sync())) return rc;
+    // the numbers land while the output lines are measured (the sizes need
+    // their lengths only)
+    if (buf && total && (rc = check(cudaMemcpyAsync(sB, dB, (size_t)total, cudaMemcpyDeviceToHost, s), "d2h")))
+        return rc;
     // file g = header, output lines, numbers, "c\n"; files back to back
     std::vector<int> headLen(G);
     std::vector<int64_t> textLen(G);
@@ -514,7 +536,7 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
         const DevGraph &d = b.hg[g];
         headLen[g] = snprintf(hline, sizeof hline, "aig %d %d 0 %d %d\n", d.nPIs + d.nAnds, d.nPIs, d.nPOs, d.nAnds);
     }
-    for_runs(G, [&](int g) { return (int64_t)b.hg[g].nPOs + 1; }, [&](int g0, int g1) {
+    for_runs(G, 4 * kLinesPerThread, [&](int g) { return (int64_t)b.hg[g].nPOs + 1; }, [&](int g0, int g1) {
         for (int g = g0; g < g1; g++) {
             int64_t t = 0;
             for (int o = 0; o < b.hg[g].nPOs; o++) t += line_len(aig_inv_const(sPO[b.hg[g].poOff + o]));
@@ -525,8 +547,9 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
     for (int g = 0; g < G; g++)
         offsets[g + 1] = offsets[g] + (size_t)headLen[g] + (size_t)textLen[g] + (size_t)(hOff[g + 1] - hOff[g]) + 2;
     if (!buf) return 0;  // sizes only
+    if ((rc = sync())) return rc;
     if (cap < offsets[G]) return fail(CULS_E_INVALID, "download: AIGER buffer too small");
-    for_runs(G, [&](int g) { return (int64_t)(offsets[g + 1] - offsets[g]); }, [&](int g0, int g1) {
+    for_runs(G, kBytesPerThread, [&](int g) { return (int64_t)(offsets[g + 1] - offsets[g]); }, [&](int g0, int g1) {
         char line[96];
         for (int g = g0; g < g1; g++) {
             const DevGraph &d = b.hg[g];
