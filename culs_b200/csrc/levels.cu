@@ -4,15 +4,18 @@
 // hop's latency.  Through L2 a hop takes 1.8 us (a published word has to
 // reach L2 and a poll to come back): the 64x64 multiplier's 501 levels 0.92
 // ms, three times in one `rw; st`.  A graph of up to 57,000 nodes has its
-// words in one block's shared memory instead: 1,024 threads take the nodes in
-// order, a row at a time, and poll their two fanins' words there.
+// words in one block's shared memory instead: the threads take the nodes in
+// order, a row at a time, and poll their two fanins' words there.  The polls
+// of waiting warps bound the hop: 512 threads are faster than 1,024 (those
+// 501 levels 0.13 ms against 0.16), and so is one node a thread than two or
+// four (0.14, 0.17).
 #include "levels.cuh"
 
 namespace culs {
 
 namespace {
 
-constexpr int kLevelsThreads = 1024;
+constexpr int kLevelsThreads = 512;
 constexpr int kUnresolved = -1;  // word of a node whose fanins are not all known; 0: pending, else 2 * level + phase + 1
 
 // Every warp takes its rows in order and waits only for nodes earlier in the

@@ -8,10 +8,12 @@
 // step as the reference's recursion does (its order of reference-count
 // updates matters when a cone reaches a node along two paths: a node can be
 // deleted twice) -- against the committed graph, with its own changes kept in
-// a small overlay.  A candidate whose overlay holds a node that an earlier
-// candidate of the window changes has seen a stale graph; everything before
-// the first such candidate is exactly what the sequential loop would have
-// done, is committed at once, and the next window starts there.
+// a small overlay.  A candidate that read something which an earlier candidate
+// of the window changes -- a deletion flag, a fanin, or a reference count that
+// may now be zero where it was not, or the other way round -- has seen a stale
+// graph; everything before the first such candidate is exactly what the
+// sequential loop would have done, is committed at once, and the next window
+// starts there.
 //
 // Redundancy removal chases buffer chains.  The reference does it in one
 // sequential sweep in which a node's fanins, once rewritten, can make it
@@ -24,7 +26,11 @@
 #include <cstdlib>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "rw_work.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace culs {
 
@@ -34,14 +40,15 @@ namespace {
 // stack.  On the 1M-AND layered graph (rw -z) candidates touch 5 nodes above
 // the inputs on average and at most 53 reads of 24 traversed nodes; a
 // candidate that needs more is replayed alone on the committed graph.
-constexpr int kOverlay = 32;  // a multiple of 4
+constexpr int kOverlay = 32;  // a multiple of 8
 constexpr int kSpecFrames = 16;
 
 struct ChoiceArgs {
     int64_t nL0;  // W positions [0, nL0) are constants and PIs
     const DevGraph *dg;
     int4 *rec;                // per node {L0, L1, ref, del}
-    int *mark;                // per node: lowest window place that changes it (INT_MAX: none)
+    int4 *mark;               // per node, by the window's candidates: lowest place that changes its flag, its count
+                              // (INT_MAX: none), what is taken from its count in all, lowest place that changes its fanins
     const int4 *recA, *recB;  // per candidate in graph order: {c, q, rep, -}, leaves
     const int *gStart, *gCount;  // a graph's candidates (several graphs)
     int n;                       // all candidates
@@ -64,18 +71,21 @@ struct ChoiceArgs {
 struct GraphMem {
     int4 *rec;
     int64_t nL0;
-    __device__ __forceinline__ int4 ld(int x) const { return rec[x]; }
+    __device__ __forceinline__ int4 ld(int x) const { return __ldcg(rec + x); }
     __device__ __forceinline__ int append(int x, const int4 &) const { return x >= nL0 ? x : -1; }
     __device__ __forceinline__ void slots(int x0, const int4 &, int x1, const int4 &, int &k0, int &k1) const {
         k0 = x0 >= nL0 ? x0 : -1;
         k1 = x1 >= nL0 ? x1 : -1;
     }
-    __device__ __forceinline__ int del(int k) const { return k >= 0 ? rec[k].w : 0; }
-    __device__ __forceinline__ int ref(int k, int base) const { return k >= 0 ? rec[k].z : base; }
+    __device__ __forceinline__ int del(int k) const { return k >= 0 ? __ldcg(&rec[k].w) : 0; }
+    __device__ __forceinline__ int ref(int k, int base) const { return k >= 0 ? __ldcg(&rec[k].z) : base; }
     __device__ __forceinline__ void add(int k, int d) {
-        if (k >= 0) rec[k].z += d;
+        if (k >= 0) rec[k].z = __ldcg(&rec[k].z) + d;
     }
     __device__ __forceinline__ void set_del(int k, int v) { rec[k].w = v; }
+    __device__ __forceinline__ void use_del(int) {}
+    __device__ __forceinline__ void use_fanins(int) {}
+    __device__ __forceinline__ void decide(int, int) {}
     __device__ __forceinline__ void set_fanins(int k, int a, int b) {
         rec[k].x = a;
         rec[k].y = b;
@@ -85,9 +95,14 @@ struct GraphMem {
 
 // The committed graph under one candidate's changes; a node's handle is its
 // entry in the thread's overlay.  Entry k: node id and {deleted before: bit
-// 0, deleted now: bit 1, fanins rewritten: bit 2, change of ref: bits 16-31}.
-// The ids lie four to a 16-byte word, words and states thread-minor in shared
-// memory.
+// 0, deleted now: bit 1, fanins rewritten: bit 2, flag mattered: bit 3, a count
+// that was zero or below mattered: bit 4, fanins mattered: bit 5, lowest
+// positive count that mattered: bits 6-15 (kNoLow: none), change of ref: bits
+// 16-31}.  The ids lie four to a 16-byte word, words and states thread-minor
+// in shared memory.
+constexpr int kNoLow = 1023;
+// OneSm: all threads that change the graph are on one SM, whose L1 may hold it.
+template <bool OneSm>
 struct OverlayMem {
     const int4 *rec;
     int64_t nL0;
@@ -96,7 +111,7 @@ struct OverlayMem {
     int stride;
     int n;
     bool full;
-    __device__ __forceinline__ int4 ld(int x) const { return rec[x]; }
+    __device__ __forceinline__ int4 ld(int x) const { return OneSm ? rec[x] : __ldcg(rec + x); }
     __device__ __forceinline__ int id(int k) const { return reinterpret_cast<const int *>(ids + (k >> 2) * stride)[k & 3]; }
     // new entry of node x with record r; x has none
     __device__ __forceinline__ int append(int x, const int4 &r) {
@@ -106,7 +121,7 @@ struct OverlayMem {
             return 0;  // the candidate is abandoned, so any entry will do
         }
         reinterpret_cast<int *>(ids + (n >> 2) * stride)[n & 3] = x;
-        sts[n * stride] = r.w ? 3 : 0;
+        sts[n * stride] = (r.w ? 3 : 0) | (kNoLow << 6);
         return n++;
     }
     // the entries of x0 and x1, made when absent (places beyond n hold
@@ -131,16 +146,45 @@ struct OverlayMem {
         }
         if (k1 < 0) k1 = append(x1, r1);
     }
-    __device__ __forceinline__ int del(int k) const { return k >= 0 ? (sts[k * stride] >> 1) & 1 : 0; }
+    __device__ __forceinline__ int del(int k) {
+        if (k < 0) return 0;
+        const int s = sts[k * stride];
+        sts[k * stride] = s | 8;
+        return (s >> 1) & 1;
+    }
+    // the node's flag, or its fanins, matter to the candidate
+    __device__ __forceinline__ void use_del(int k) {
+        if (k >= 0) sts[k * stride] |= 8;
+    }
+    __device__ __forceinline__ void use_fanins(int k) {
+        if (k >= 0) sts[k * stride] |= 32;
+    }
+    // whether the node's count, now v, is zero matters
+    __device__ __forceinline__ void decide(int k, int v) {
+        if (k < 0) return;
+        const int s = sts[k * stride];
+        if (v <= 0)
+            sts[k * stride] = s | 16;
+        else if (v < ((s >> 6) & kNoLow) || ((s >> 6) & kNoLow) == kNoLow)
+            sts[k * stride] = (s & ~(kNoLow << 6)) | (min(v, kNoLow - 1) << 6);
+    }
     __device__ __forceinline__ int ref(int k, int base) const { return k >= 0 ? base + (sts[k * stride] >> 16) : base; }
     __device__ __forceinline__ void add(int k, int d) {
         if (k >= 0) sts[k * stride] += d * 65536;
     }
-    __device__ __forceinline__ void set_del(int k, int v) { sts[k * stride] = (sts[k * stride] & ~2) | (v << 1); }
+    __device__ __forceinline__ void set_del(int k, int v) { sts[k * stride] = (sts[k * stride] & ~2) | (v << 1) | 8; }
     __device__ __forceinline__ void set_fanins(int k, int, int) { sts[k * stride] |= 4; }
     __device__ __forceinline__ bool failed() const { return full; }
-    // whether the node of state st ends up changed
-    static __device__ __forceinline__ bool changed(int st) { return (st >> 16) != 0 || (st & 4) || ((st ^ (st >> 1)) & 1); }
+    // whether the flag of the node of state st ends up changed
+    static __device__ __forceinline__ bool flipped(int st) { return (st ^ (st >> 1)) & 1; }
+    // Whether a candidate at place t that holds state st of a node saw it stale,
+    // given the node's marks.  A count that mattered as positive still is when
+    // it exceeds all that the window's other candidates take away.
+    static __device__ __forceinline__ bool stale(int st, const int4 &mark, int t) {
+        const int low = (st >> 6) & kNoLow, own = st >> 16;
+        return ((st & 8) && mark.x < t) || ((st & 32) && mark.w < t) ||
+               (mark.y < t && ((st & 16) || (low < kNoLow && low <= mark.z - (own < 0 ? -own : 0))));
+    }
 };
 
 // Traversal stacks.  Frames: FastDelete's {handle, count << 2 | where to
@@ -233,11 +277,13 @@ struct Replay {
         gain = 0;
         n0 = rn.x, n1 = rn.y, nRef = rn.z, q0 = rq.x, q1 = rq.y;
         // the leaves are distinct nodes below q; the replacement may be one
-        m.append(lv.x, r0);
-        m.append(lv.y, r1);
-        m.append(lv.z, r2);
-        m.append(lv.w, r3);
+        m.use_del(m.append(lv.x, r0));
+        m.use_del(m.append(lv.y, r1));
+        m.use_del(m.append(lv.z, r2));
+        m.use_del(m.append(lv.w, r3));
         m.slots(q, rq, x, rn, kq, kn);
+        m.use_fanins(kq);
+        m.use_fanins(kn);
         if (x == q || (n1 >> 1) == q) return done(kChSelfRef);
         if (r0.w | r1.w | r2.w | r3.w) return done(kChCompromised);
         phase = 0;
@@ -270,7 +316,9 @@ struct Replay {
         if (phase == 2) {  // the node is back: drop the replacement
             m.add(kq, 1);
             phase = 3;
-            if (kn >= 0 && m.ref(kn, nRef) == 0) return begin_delete(kn, n0, n1);
+            const int v = m.ref(kn, nRef);
+            m.decide(kn, v);
+            if (kn >= 0 && v == 0) return begin_delete(kn, n0, n1);
         }
         m.add(kq, -1);
         done(kChReverted);
@@ -289,10 +337,12 @@ struct Replay {
             m.add(k1, 1);
             if (d1 && c1 != c0) {
                 m.set_del(k1, 0);
+                m.use_fanins(k1);
                 st.push(sp, make_int4(k1, 0, r1.x, r1.y));
             }
             if (d0) {
                 m.set_del(k0, 0);
+                m.use_fanins(k0);
                 k = k0, l0 = r0.x, l1 = r0.y;
             } else if (sp > 0) {
                 const int4 f = st.pop(sp);
@@ -309,14 +359,18 @@ struct Replay {
                 v1 = m.ref(k1, r1.z) - 1;
                 m.add(k1, -1);
                 v0 = c0 == c1 ? v1 : o0 - 1;  // one node twice: both decrements precede the first check
+                m.decide(k0, v0);
             } else {
                 v1 = m.ref(k1, r1.z);
             }
+            m.decide(k1, v1);
             if (v0 == 0 && k0 >= 0) {
                 st.push(sp, make_int4(k, (cnt << 2) | 1, l0, l1));
+                m.use_fanins(k0);
                 mode = kOpen, k = k0, l0 = r0.x, l1 = r0.y;
             } else if (v1 == 0 && k1 >= 0) {
                 st.push(sp, make_int4(k, (cnt << 2) | 2, l0, l1));
+                m.use_fanins(k1);
                 mode = kOpen, k = k1, l0 = r1.x, l1 = r1.y;
             } else {
                 while (true) {
@@ -340,43 +394,53 @@ struct Replay {
 };
 
 // Rounds of a window of candidates, one per thread (see the top of the
-// file); T threads, the window's places dealt to the warps in turn.  A round
-// is three block barriers: every thread replays its candidate and lowers the
-// mark of each node it changes to its place in the window (one red per node);
-// a thread whose overlay holds a node marked by a lower place must wait, and
-// the lowest such place ends the part that is committed; committing adds the
-// overlay's changes to the records, which no other committed candidate has
-// read.  A candidate that outgrows its overlay ends the window and, at its
+// file); T threads on each of B blocks (a cluster when B > 1), the window's
+// places dealt to the warps in turn.  A round
+// is three barriers: every thread replays its candidate and marks each
+// node it changes with its place in the window; a thread that saw one of its
+// nodes stale must wait, and the lowest such place ends the part that is
+// committed; committing adds the overlay's changes to the records.  Flags and
+// fanins that a committed candidate changes, no later committed one has used;
+// counts change by sums.  A candidate that outgrows its overlay ends the window and, at its
 // start, is replayed by thread 0 on the committed graph.  The next window is
 // up to four times the part committed, at least two places a warp.
 //
-// Bound: the latency of a replay's dependent record loads (about ten), 9 us a
-// round.  One thread walking the candidates took 2.3-2.5 us for each.  64x64
-// multiplier (4,157 candidates, 25 committed at a time): 9.6 -> 1.5 ms;
-// 1M-AND layered graph with rw -z (80,251 tried, 295 at a time): 202 -> 4.5
-// ms; 256 graphs of up to 200k ANDs: 15.1 -> 2.6 ms.
-template <int T>
+// Bound: the latency of a replay's dependent record loads (about ten), 10-16
+// us a round.  One thread walking the candidates took 2.3-2.5 us for each.
+// 64x64 multiplier (4,157 candidates, 61 committed at a time; 25 when every
+// change of a node made it stale): 9.6 -> 0.76 ms; 1M-AND layered graph with
+// rw -z (80,251 tried, 345 at a time): 202 -> 3.7 ms; 256 graphs of up to 200k
+// ANDs: 15.1 -> 2.5 ms.
+template <int T, int B>
 __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
+    using Overlay = OverlayMem<B == 1>;
     extern __shared__ int4 s_overlay[];
     __shared__ int s_stop[2];
-    constexpr int kWarps = T / 32;
-    const int tid = threadIdx.x, g = blockIdx.x;
-    const int t = (tid & 31) * kWarps + (tid >> 5);  // place in the window
+    constexpr int kWarps = T / 32 * B;
+    const int tid = threadIdx.x, g = blockIdx.x / B, rank = blockIdx.x % B;
+    const int t = (tid & 31) * kWarps + rank * (T / 32) + (tid >> 5);  // place in the window
+    auto barrier = [] {
+        if (B == 1)
+            __syncthreads();
+        else
+            cg::this_cluster().sync();
+    };
+    int *stops = B == 1 ? s_stop : cg::this_cluster().map_shared_rank(s_stop, 0);
     const int64_t nL0 = A.nL0;
     const int trueLit = 2 * A.dg[g].cpos + 1;
-    int base = gridDim.x > 1 ? A.gStart[g] : 0;
-    const int end = gridDim.x > 1 ? base + A.gCount[g] : A.n;
+    int base = gridDim.x > B ? A.gStart[g] : 0;
+    const int end = gridDim.x > B ? base + A.gCount[g] : A.n;
     if (tid < 2) s_stop[tid] = INT_MAX;
-    __syncthreads();
+    barrier();
     int nDone[kChReverted + 1] = {}, nPos = 0, expected = 0;
-    int window = A.serial ? 1 : T;
+    int window = A.serial ? 1 : T * B;
     for (int round = 0; base < end; round++) {
         const int nAct = min(window, end - base);
         const bool act = t < nAct;
-        int *stop = &s_stop[round & 1];
-        Replay<OverlayMem, SpecStack> R;
+        int *stop = &stops[round & 1];
+        Replay<Overlay, SpecStack> R;
         int4 frames[kSpecFrames];
-        R.m = OverlayMem{A.rec, nL0, s_overlay + tid, reinterpret_cast<int *>(s_overlay + kOverlay / 4 * T) + tid, T, 0, false};
+        R.m = Overlay{A.rec, nL0, s_overlay + tid, reinterpret_cast<int *>(s_overlay + kOverlay / 4 * T) + tid, T, 0, false};
         R.st = SpecStack{frames, false};
         R.trueLit = trueLit;
         R.nL0 = nL0;
@@ -392,46 +456,62 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
             __syncwarp();
         }
         const bool alone = R.m.full || R.st.full || A.serial;
-        if (act && !alone)
-            for (int k = 0; k < R.m.n; k++)
-                if (OverlayMem::changed(R.m.sts[k * T])) atomicMin(&A.mark[R.m.id(k)], t);
-        if (tid == 0) s_stop[(round + 1) & 1] = INT_MAX;
-        __syncthreads();
+        // the overlay's entries four at a time, so that their accesses overlap
+        const int n = act && !alone ? R.m.n : 0;
+        for (int k = 0; k < n; k += 4) {
+            const int4 x = R.m.ids[(k >> 2) * T];
+            const int node[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (k + j >= n) continue;
+                const int st = R.m.sts[(k + j) * T], d = st >> 16;
+                int4 *mark = &A.mark[node[j]];
+                if (Overlay::flipped(st)) atomicMin(&mark->x, t);
+                if (d) atomicMin(&mark->y, t);
+                if (d < 0) atomicAdd(&mark->z, -d);
+                if (st & 4) atomicMin(&mark->w, t);
+            }
+        }
+        if (rank == 0 && tid == 0) s_stop[(round + 1) & 1] = INT_MAX;
+        barrier();
         if (act) {
             bool wait = alone;
-            if (!wait) {
-                int low = INT_MAX;  // four marks in flight at a time
-                for (int k = 0; k < R.m.n; k += 4) {
-                    const int4 x = R.m.ids[(k >> 2) * T];
-                    const int left = R.m.n - k;
-                    const int m0 = __ldcg(&A.mark[x.x]), m1 = left > 1 ? __ldcg(&A.mark[x.y]) : INT_MAX,
-                              m2 = left > 2 ? __ldcg(&A.mark[x.z]) : INT_MAX,
-                              m3 = left > 3 ? __ldcg(&A.mark[x.w]) : INT_MAX;
-                    low = min(min(low, min(m0, m1)), min(m2, m3));
-                }
-                wait = low < t;
+            for (int k = 0; k < n; k += 8) {
+                int4 m[8];
+                const int4 x = R.m.ids[(k >> 2) * T], y = R.m.ids[((k >> 2) + 1) * T];
+                const int node[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    m[j] = k + j < n ? __ldcg(&A.mark[node[j]]) : make_int4(INT_MAX, INT_MAX, 0, INT_MAX);
+#pragma unroll
+                for (int j = 0; j < 8; j++) wait |= k + j < n && Overlay::stale(R.m.sts[(k + j) * T], m[j], t);
             }
             if (wait) atomicMin(stop, t);
         }
-        __syncthreads();
+        barrier();
         int done = min(*stop, nAct);
-        if (act && !alone) {
-            for (int k = 0; k < R.m.n; k++) {
-                const int st = R.m.sts[k * T], x = R.m.id(k);
-                if (!OverlayMem::changed(st)) continue;
-                A.mark[x] = INT_MAX;
+        for (int k = 0; k < n; k += 4) {
+            const int4 x = R.m.ids[(k >> 2) * T];
+            const int node[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (k + j >= n) continue;
+                const int st = R.m.sts[(k + j) * T];
+                if (!Overlay::flipped(st) && !(st >> 16) && !(st & 4)) continue;
+                A.mark[node[j]] = make_int4(INT_MAX, INT_MAX, 0, INT_MAX);
                 if (t >= done) continue;
-                if (st >> 16) atomicAdd(&A.rec[x].z, st >> 16);
-                if ((st ^ (st >> 1)) & 1) A.rec[x].w = (st >> 1) & 1;
+                int4 *rec = A.rec + node[j];
+                if (st >> 16) atomicAdd(&rec->z, st >> 16);
+                if (Overlay::flipped(st)) rec->w = (st >> 1) & 1;
                 if (st & 4) {
-                    A.rec[x].x = trueLit;
-                    A.rec[x].y = a.z;
+                    rec->x = trueLit;
+                    rec->y = a.z;
                 }
             }
         }
         int code = R.code, gain = R.gain;
         if (done == 0) {  // the first candidate alone
-            __syncthreads();
+            barrier();
             if (t == 0) {
                 Replay<GraphMem, GraphStack> S;
                 S.m = GraphMem{A.rec, nL0};
@@ -456,8 +536,8 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
             }
         }
         base += done;
-        window = A.serial ? 1 : min(T, max(2 * kWarps, 4 * done));
-        __syncthreads();
+        window = A.serial ? 1 : min(T * B, max(2 * kWarps, 4 * done));
+        barrier();
     }
     const int tot[7] = {nDone[kChCommitted],   nPos,     nDone[kChCommitted] - nPos, nDone[kChReverted],
                         nDone[kChCompromised], nDone[kChSelfRef], expected};
@@ -470,11 +550,11 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
 
 // Gathers the nodes' records and clears their marks.
 __global__ void k_choice_pack(int64_t M, const int *L0, const int *L1, const int *ref, const uint8_t *del, int4 *rec,
-                              int *mark) {
+                              int4 *mark) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < M; x += stride) {
         rec[x] = make_int4(L0[x], L1[x], ref[x], del[x]);
-        mark[x] = INT_MAX;
+        mark[x] = make_int4(INT_MAX, INT_MAX, 0, INT_MAX);
     }
 }
 
@@ -520,13 +600,24 @@ __global__ void k_cand_gid(int64_t n, const int *withRep, const int *cand, const
     }
 }
 
-template <int T>
+template <int T, int B>
 cudaError_t launch_choice(const ChoiceArgs &A, int G, cudaStream_t s) {
     const int smem = 2 * kOverlay * T * (int)sizeof(int);  // ids and states
-    cudaError_t e = cudaFuncSetAttribute(k_choice<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = cudaFuncSetAttribute(k_choice<T, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k_choice<T><<<G, T, smem, s>>>(A);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(G * B));
+    cfg.blockDim = dim3(T);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = B;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = B > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, k_choice<T, B>, A);
 }
 
 }  // namespace
@@ -551,14 +642,13 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w) {
     int4 *stack = ar.get<int4>((size_t)stackCap * G);
     // the records and marks take the place of the enumeration's cut
     // attributes (64 bytes per original node), which nothing reads any more
-    int4 *rec;
-    int *mark;
-    if (20 * M <= 64 * w.N) {
+    int4 *rec, *mark;
+    if (32 * M <= 64 * w.N) {
         rec = reinterpret_cast<int4 *>(w.cutA);
-        mark = reinterpret_cast<int *>(rec + M);
+        mark = rec + M;
     } else {
         rec = ar.get<int4>(M);
-        mark = ar.get<int>(M);
+        mark = ar.get<int4>(M);
     }
     if (!gCount || !gStart || !candByG || !keys || !keys2 || !vals || !recA || !recB || !w.choice || !stack ||
         !rec || !mark)
@@ -584,17 +674,24 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w) {
         // the two)
         ChoiceArgs A{w.nL0,  w.dg,  rec,           mark,     recA,   recB,    gStart, gCount, (int)nRep, w.useZeros ? 1 : 0,
                      getenv("CULS_CHOICE_GLOBAL") ? 1 : 0, stack, (int)stackCap, w.choice, dstats, X.status};
-        // Threads per graph: a window as wide as an SM's shared memory allows
-        // while there is an SM for every graph, narrower ones so that more
+        // Threads per graph: a cluster of eight SMs for few graphs of many
+        // candidates (not on an SM partition, whose SMs need not hold a whole
+        // cluster), so that the replays of a window share no SM's load path
+        // (1M-AND rw -z 4.6 -> 3.7 ms, 64x64 multiplier 0.87 -> 0.76; its
+        // barriers cost more where 95 candidates are all there are: 0.28 ->
+        // 0.31); else a window as wide
+        // as an SM's shared memory allows while there is an SM for every graph, narrower ones so that more
         // graphs are resident when there are more (a batch's graphs have
         // short windows: 7 candidates are committed at a time on the c4
         // family's, 340 on the 1M-AND graph).
-        if (G <= X.sms)
-            rc = X.check(launch_choice<512>(A, G, s), "choice launch");
+        if (X.clusters && 8 * G <= X.sms && nRep >= 1024 * (int64_t)G)
+            rc = X.check(launch_choice<128, 8>(A, G, s), "choice launch");
+        else if (G <= X.sms)
+            rc = X.check(launch_choice<512, 1>(A, G, s), "choice launch");
         else if (G <= 3 * X.sms)
-            rc = X.check(launch_choice<256>(A, G, s), "choice launch");
+            rc = X.check(launch_choice<256, 1>(A, G, s), "choice launch");
         else
-            rc = X.check(launch_choice<64>(A, G, s), "choice launch");
+            rc = X.check(launch_choice<64, 1>(A, G, s), "choice launch");
         if (rc) return rc;
         k_choice_unpack<<<X.grid(M), kBlock, 0, s>>>(M, rec, w.L0, w.L1, w.del);
         X.launched(4);

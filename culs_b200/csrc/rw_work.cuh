@@ -35,6 +35,7 @@ struct ExecCtx {
     int *hostSmall = nullptr; // their host copy as of the last fetch
     const RwLib *lib = nullptr;
     int sms = 148;
+    bool clusters = true;  // thread-block clusters may be launched on s (not on an SM-partition stream)
     int *launches = nullptr;
     std::string *err = nullptr;
     const Tune *tune = nullptr;  // launch and schedule parameters
