@@ -11,10 +11,10 @@
 
 namespace culs {
 
-// A cut in registers.  aux0 = ref of leaf 0 | ref of leaf 1 << 11 |
-// (ref of leaf 2 & 0x3FF) << 22; aux1 = ref of leaf 2 >> 10 | ref of leaf 3
-// << 1 | lid5 of leaves 0..3 << 12 + 5*i.  Refs are clamped to 1001, which
-// leaves CutFindValue's result unchanged (it caps the sum at 1000).
+// A cut in registers.  Each leaf's attributes, its reference count (11 bits)
+// and local-id bits (5), are a halfword: aux0 = leaves 0 and 1, aux1 = leaves
+// 2 and 3.  Refs are clamped to 1001, which leaves CutFindValue's result
+// unchanged (it caps the sum at 1000).  Unused places hold zeros.
 struct RCut {
     int l[4];
     uint32_t sign, tt, value, n, used;
@@ -22,32 +22,29 @@ struct RCut {
     uint32_t lid[4];
 };
 
+__device__ __forceinline__ uint32_t rc_attr(const RCut &c, int i) { return (c.ref[i] & 0x7FFu) | ((c.lid[i] & 31u) << 11); }
+__device__ __forceinline__ void rc_set_attr(RCut &c, int i, uint32_t a) {
+    c.ref[i] = a & 0x7FFu;
+    c.lid[i] = (a >> 11) & 31u;
+}
+
 __device__ __forceinline__ void rc_unpack_aux(uint32_t a0, uint32_t a1, RCut &c) {
-    c.ref[0] = a0 & 0x7FFu;
-    c.ref[1] = (a0 >> 11) & 0x7FFu;
-    c.ref[2] = ((a0 >> 22) & 0x3FFu) | ((a1 & 1u) << 10);
-    c.ref[3] = (a1 >> 1) & 0x7FFu;
-#pragma unroll
-    for (int i = 0; i < 4; i++) c.lid[i] = (a1 >> (12 + 5 * i)) & 31u;
+    rc_set_attr(c, 0, a0 & 0xFFFFu);
+    rc_set_attr(c, 1, a0 >> 16);
+    rc_set_attr(c, 2, a1 & 0xFFFFu);
+    rc_set_attr(c, 3, a1 >> 16);
 }
 
 __device__ __forceinline__ void rc_pack_aux(const RCut &c, uint32_t &a0, uint32_t &a1) {
-    a0 = (c.ref[0] & 0x7FFu) | ((c.ref[1] & 0x7FFu) << 11) | ((c.ref[2] & 0x3FFu) << 22);
-    a1 = ((c.ref[2] >> 10) & 1u) | ((c.ref[3] & 0x7FFu) << 1);
-#pragma unroll
-    for (int i = 0; i < 4; i++) a1 |= (c.lid[i] & 31u) << (12 + 5 * i);
+    a0 = rc_attr(c, 0) | (rc_attr(c, 1) << 16);
+    a1 = rc_attr(c, 2) | (rc_attr(c, 3) << 16);
 }
 
 // CutFindValue from the carried refs.
 __device__ __forceinline__ uint32_t rc_value(const RCut &c) {
     if (c.n < 2) return 1001u;
-    uint32_t v = 0, ones = 0;
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-        if ((uint32_t)i < c.n) {
-            v += c.ref[i];
-            ones += c.ref[i] == 1u;
-        }
+    const uint32_t v = c.ref[0] + c.ref[1] + c.ref[2] + c.ref[3];
+    const uint32_t ones = (c.ref[0] == 1u) + (c.ref[1] == 1u) + (c.ref[2] == 1u) + (c.ref[3] == 1u);
     int value = v > 1000u ? 1000 : (int)v;
     if (ones > 3) value = 5 - (int)ones;
     return (uint32_t)value & 0x7FFu;
@@ -59,41 +56,52 @@ __device__ __forceinline__ T pick4(const T (&v)[4], int i) {
 }
 
 // MergeCutOrdered / MergeCut with the leaf attributes carried along: four
-// merge steps, each taking the smaller head leaf (both when equal), without
-// branches -- the lanes of the warp-wide enumeration merge different cuts.
-// Bit s of pa0 (pb0) is set when a0 (b0) has the merged leaf s: CutTruthPhase
+// merge steps, each taking the smaller head leaf (both when equal) and moving
+// the lists up, without branches -- the lanes of the warp-wide enumeration
+// merge different cuts.  Places past a list's end are larger than every leaf.
+// Bit s of pa (pb) is set when a (b) has the merged leaf s: CutTruthPhase
 // (rewrite.cu:195-201).
-__device__ __forceinline__ bool rc_merge(const RCut &a0, const RCut &b0, RCut &o, int &pa0, int &pb0) {
-    const bool sw = a0.n < b0.n;
-    const RCut &a = sw ? b0 : a0;
-    const RCut &b = sw ? a0 : b0;
-    int i = 0, k = 0, c = 0, pa = 0, pb = 0;
-    const int na = (int)a.n, nb = (int)b.n;
+__device__ __forceinline__ bool rc_merge(const RCut &a, const RCut &b, RCut &o, int &pa, int &pb) {
+    constexpr int kEnd = 0x7FFFFFFF;
+    int x[4], y[4];
+    uint32_t xa[4], ya[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        x[i] = (uint32_t)i < a.n ? a.l[i] : kEnd;
+        y[i] = (uint32_t)i < b.n ? b.l[i] : kEnd;
+        xa[i] = rc_attr(a, i);
+        ya[i] = rc_attr(b, i);
+    }
+    const bool first = a.n >= b.n;  // whose attributes an equal leaf takes
+    int c = 0;
+    pa = pb = 0;
 #pragma unroll
     for (int s = 0; s < 4; s++) {
-        const bool ea = i >= na, eb = k >= nb;
-        const bool act = !(ea && eb);
-        const int ai = ea ? 0x7FFFFFFF : pick4(a.l, i);
-        const int bk = eb ? 0x7FFFFFFF : pick4(b.l, k);
-        const int take = eb ? 0 : (ea ? 1 : (ai < bk ? 0 : (ai > bk ? 1 : 2)));  // 0 = a, 1 = b, 2 = equal
-        o.l[s] = act ? (take == 1 ? bk : ai) : 0;
-        o.ref[s] = act ? (take == 1 ? pick4(b.ref, k) : pick4(a.ref, i)) : 0u;
-        o.lid[s] = act ? (take == 1 ? pick4(b.lid, k) : pick4(a.lid, i)) : 0u;
-        const int ta = (act && take != 1) ? 1 : 0, tb = (act && take != 0) ? 1 : 0;
-        i += ta;
-        k += tb;
-        pa |= ta << s;
-        pb |= tb << s;
-        c = act ? s + 1 : c;
+        const bool ta = x[0] <= y[0], tb = y[0] <= x[0];
+        const int leaf = ta ? x[0] : y[0];
+        const bool act = leaf != kEnd;
+        o.l[s] = act ? leaf : 0;
+        rc_set_attr(o, s, act ? (ta && (first || !tb) ? xa[0] : ya[0]) : 0u);
+        pa |= act && ta ? 1 << s : 0;
+        pb |= act && tb ? 1 << s : 0;
+        c += act ? 1 : 0;
+        // what is still looked at: the heads of the steps left, and the last
+        // one's successor
+#pragma unroll
+        for (int i = 0; i < 4 - s; i++) {
+            x[i] = ta ? (i < 3 ? x[i + 1] : kEnd) : x[i];
+            y[i] = tb ? (i < 3 ? y[i + 1] : kEnd) : y[i];
+            if (i < 3 - s) {
+                xa[i] = ta && i < 3 ? xa[i + 1] : xa[i];
+                ya[i] = tb && i < 3 ? ya[i + 1] : ya[i];
+            }
+        }
     }
     o.n = (uint32_t)c;
-    o.sign = a0.sign | b0.sign;
+    o.sign = a.sign | b.sign;
     o.used = 1;
-    pa0 = sw ? pb : pa;
-    pb0 = sw ? pa : pb;
-    return i >= na && k >= nb;
+    return x[0] == kEnd && y[0] == kEnd;
 }
-
 __device__ __forceinline__ bool rc_merge(const RCut &a, const RCut &b, RCut &o) {
     int pa, pb;
     return rc_merge(a, b, o, pa, pb);
@@ -126,6 +134,11 @@ __device__ __forceinline__ bool rc_minimize(RCut &c) {
     if (nl == (int)c.n) return false;
     c.tt = tt_shrink_flat(t, ph) & 0xFFFFu;
     RCut o = c;
+#pragma unroll
+    for (int s = 0; s < 4; s++) {
+        o.l[s] = 0;
+        rc_set_attr(o, s, 0);
+    }
     int k = 0;
     uint32_t sign = 0;
 #pragma unroll
@@ -136,8 +149,7 @@ __device__ __forceinline__ bool rc_minimize(RCut &c) {
             for (int s = 0; s < 4; s++)
                 if (s == k) {
                     o.l[s] = c.l[i];
-                    o.ref[s] = c.ref[i];
-                    o.lid[s] = c.lid[i];
+                    rc_set_attr(o, s, rc_attr(c, i));
                 }
             sign |= 1u << c.lid[i];
             k++;

@@ -39,7 +39,9 @@ struct EnumArgs {
     int *status;
 };
 
-__device__ __forceinline__ uint32_t clamp_ref(int r) { return r > 1001 ? 1001u : (uint32_t)r; }
+__device__ __forceinline__ uint32_t leaf_attr(int ref, uint32_t lid) {
+    return (ref > 1001 ? 1001u : (uint32_t)ref) | ((lid & 31u) << 11);
+}
 
 __global__ void k_enum_init(int64_t N, const int *wlev, const int *wl, const uint8_t *lidLow, const int *ref,
                             int4 *cutL, int2 *cutM, int2 *cutA, int *done) {
@@ -56,7 +58,7 @@ __global__ void k_enum_init(int64_t N, const int *wlev, const int *wl, const uin
             c.value = 1001u;  // CutFindValue of a one-leaf cut
             cutL[q * 8] = make_int4((int)q, 0, 0, 0);
             cutM[q * 8] = make_int2((int)c.sign, (int)cut_pack(c));
-            cutA[q * 8] = make_int2((int)clamp_ref(ref[q]), (int)((uint32_t)lidLow[q] << 12));
+            cutA[q * 8] = make_int2((int)leaf_attr(ref[q], lidLow[q]), 0);
         }
     }
 }
@@ -120,12 +122,14 @@ __device__ __forceinline__ void load_rcut(const EnumArgs &A, int64_t idx, int2 m
 }
 
 // ------------------------------------------------- warp-per-node variant
-// A warp's scratch: its node's candidates, one per admissible pair.
+// A warp's scratch: its node's fanin cuts and candidates, one per admissible
+// pair.
 struct WarpCands {
     int4 leaves[64];  // final leaves
     int4 rec[64];     // final {sign, packed tt / value / nLeaves / used, cutA words}
     uint4 rel[64];    // the merged cut against earlier candidates' final cuts
     uint4 relMin[64]; // the same for the final cut, where minimisation removed leaves
+    int4 inL[16], inR[16];  // the fanins' cuts: leaves, {sign, packed, cutA words}
     uint8_t pair[64]; // the k-th admissible pair
 };
 
@@ -194,20 +198,18 @@ __device__ __forceinline__ uint32_t slot_key(uint32_t pk) {
     return ((n > 2 ? 0u : (n == 2 ? 1u : 2u)) << 20) | (((pk >> 16) & 0x7FFu) << 3);
 }
 
-// Fanin cut record held by lane src.
-__device__ __forceinline__ void fetch_slot(int src, int4 L, int2 M, int2 X, RCut &c) {
-    const unsigned F = 0xffffffffu;
-    c.l[0] = __shfl_sync(F, L.x, src);
-    c.l[1] = __shfl_sync(F, L.y, src);
-    c.l[2] = __shfl_sync(F, L.z, src);
-    c.l[3] = __shfl_sync(F, L.w, src);
-    const uint32_t sign = (uint32_t)__shfl_sync(F, M.x, src), pk = (uint32_t)__shfl_sync(F, M.y, src);
-    const uint32_t x0 = (uint32_t)__shfl_sync(F, X.x, src), x1 = (uint32_t)__shfl_sync(F, X.y, src);
-    c.sign = sign;
-    c.tt = pk & 0xFFFFu;
-    c.n = packed_nleaves(pk);
+// The fanin cut in place i.
+__device__ __forceinline__ void fetch_slot(const WarpCands &W, int i, RCut &c) {
+    const int4 L = W.inL[i], R = W.inR[i];
+    c.l[0] = L.x;
+    c.l[1] = L.y;
+    c.l[2] = L.z;
+    c.l[3] = L.w;
+    c.sign = (uint32_t)R.x;
+    c.tt = (uint32_t)R.y & 0xFFFFu;
+    c.n = packed_nleaves((uint32_t)R.y);
     c.used = 1;
-    rc_unpack_aux(x0, x1, c);
+    rc_unpack_aux((uint32_t)R.z, (uint32_t)R.w, c);
 }
 
 // A warp enumerates one node at a time: lanes 0-7 hold u0's cut slots and
@@ -240,7 +242,7 @@ __device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int
         c.used = 1;
         c.value = 1001u;
         sl.x = (int)q;
-        sr = make_int4((int)c.sign, (int)cut_pack(c), (int)clamp_ref(A.ref[q]), (int)((uint32_t)A.lidLow[q] << 12));
+        sr = make_int4((int)c.sign, (int)cut_pack(c), (int)leaf_attr(A.ref[q], A.lidLow[q]), 0);
     }
     int ok = 1;
     if (lane < 2) ok = wait_ge(&A.done[lane ? u1 : u0], 1, A.status);
@@ -255,16 +257,15 @@ __device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int
             M = __ldcg(&A.cutM[idx]);
             L = __ldcg(&A.cutL[idx]);
             X = __ldcg(&A.cutA[idx]);
+            W.inL[lane] = L;
+            W.inR[lane] = make_int4(M.x, M.y, X.x, X.y);
         }
         // admissible pairs from the signatures: pair lane (i = lane / 8)
         // and pair lane + 32 (i = 4 + lane / 8), both with j = lane % 8
-        const uint32_t sA = (uint32_t)__shfl_sync(F, M.x, lane >> 3), pA = (uint32_t)__shfl_sync(F, M.y, lane >> 3);
-        const uint32_t sB = (uint32_t)__shfl_sync(F, M.x, 4 + (lane >> 3)),
-                       pB = (uint32_t)__shfl_sync(F, M.y, 4 + (lane >> 3));
-        const uint32_t sJ = (uint32_t)__shfl_sync(F, M.x, 8 + (lane & 7)),
-                       pJ = (uint32_t)__shfl_sync(F, M.y, 8 + (lane & 7));
-        const bool adm0 = packed_used(pA) && packed_used(pJ) && popc32(sA | sJ) <= 4;
-        const bool adm1 = packed_used(pB) && packed_used(pJ) && popc32(sB | sJ) <= 4;
+        const uint32_t sign = packed_used((uint32_t)M.y) ? (uint32_t)M.x : 0xFFFFFFFFu;  // unused: never admissible
+        const uint32_t sA = __shfl_sync(F, sign, lane >> 3), sB = __shfl_sync(F, sign, 4 + (lane >> 3)),
+                       sJ = __shfl_sync(F, sign, 8 + (lane & 7));
+        const bool adm0 = popc32(sA | sJ) <= 4, adm1 = popc32(sB | sJ) <= 4;
         const uint32_t b0 = __ballot_sync(F, adm0), b1 = __ballot_sync(F, adm1);
         const uint32_t below = (1u << lane) - 1u;
         const int n0 = __popc(b0), nPairs = n0 + __popc(b1);
@@ -281,8 +282,8 @@ __device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int
             const int k = r * 32 + (nPairs <= 16 ? lane & 15 : lane);
             const int p = W.pair[k < nPairs ? k : 0];
             RCut a, b, m;
-            fetch_slot(p >> 3, L, M, X, a);
-            fetch_slot(8 + (p & 7), L, M, X, b);
+            fetch_slot(W, p >> 3, a);
+            fetch_slot(W, 8 + (p & 7), b);
             int pa, pb;
             const bool merged = rc_merge(a, b, m, pa, pb);
 #pragma unroll
@@ -299,8 +300,7 @@ __device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int
                 pc.value = rc_value(m);
                 uint32_t x0, x1;
                 rc_pack_aux(m, x0, x1);
-                W.leaves[k] = make_int4(m.n > 0 ? m.l[0] : 0, m.n > 1 ? m.l[1] : 0, m.n > 2 ? m.l[2] : 0,
-                                        m.n > 3 ? m.l[3] : 0);
+                W.leaves[k] = make_int4(m.l[0], m.l[1], m.l[2], m.l[3]);
                 W.rec[k] = make_int4((int)m.sign, (int)cut_pack(pc), (int)x0, (int)x1);
             }
         }
@@ -387,7 +387,7 @@ __device__ __forceinline__ void enum_node_thread(const EnumArgs &A, int64_t q, b
         S[0].l[0] = (int)q;
         S[0].sign = c.sign;
         S[0].pk = cut_pack(c);
-        A.cutA[q * 8] = make_int2((int)clamp_ref(A.ref[q]), (int)((uint32_t)A.lidLow[q] << 12));
+        A.cutA[q * 8] = make_int2((int)leaf_attr(A.ref[q], A.lidLow[q]), 0);
     }
     const int f0 = valid ? A.w0[q] : 0, f1 = valid ? A.w1[q] : 0;
     const int u0 = f0 >> 1, u1 = f1 >> 1, c0 = f0 & 1, c1 = f1 & 1;
