@@ -524,17 +524,16 @@ __global__ void __launch_bounds__(kEnumBlock, 4) k_enumerate(EnumArgs A) {
 
 // A run of narrower levels, each node on a warp (latency: a level's time is
 // that of its slowest node), claimed in W order.  A kernel of its own for its
-// smaller register need: six resident blocks an SM instead of the four of one
-// kernel for both forms (1M-AND layered graph, 3,800 nodes a level: 2.80 ->
-// 1.94 ms).
+// smaller register need: eight resident blocks an SM instead of the four of
+// one kernel for both forms (1M-AND layered graph, 3,800 nodes a level: 1.56
+// ms, with six 1.64, with four 2.3).
 //
-// Where the forms meet (Tune::enumWideMin): a wide level takes about 40 us
-// however few nodes it has, one warp's 32 replays; a warp per node takes 2 ns
-// a node and 8 us at least.  128 graphs of up to 100k ANDs: 9.9 ms with the
-// line at 4,096 nodes a level, 5.7 at 16,384, 5.0 at 32,768, 5.05 at 65,536
-// and 5.5 with no wide levels; 256 graphs of up to 200k: 19.0, 17.2, 16.6,
-// 19.6, 21.4.
-__global__ void __launch_bounds__(kEnumBlock, 6) k_enumerate_warp(EnumArgs A) {
+// Where the forms meet (Tune::enumWideMin): a wide level takes about 30 us
+// however few nodes it has, one warp's 32 replays; a warp per node takes 1.7
+// ns a node and 7 us at least.  128 graphs of up to 100k ANDs: 4.3 ms with the
+// line at 16,384 nodes a level, 3.77 at 32,768, 3.80 at 65,536 and 4.1 with no
+// wide levels; 256 graphs of up to 200k: 12.9 at 16,384, 12.8, 14.7, 15.9.
+__global__ void __launch_bounds__(kEnumBlock, 8) k_enumerate_warp(EnumArgs A) {
     __shared__ WarpCands s_cand[kEnumBlock / 32];
     const int lane = threadIdx.x & 31;
     while (true) {
@@ -622,7 +621,7 @@ int rw_enumerate(ExecCtx &X, RwWork &w) {
             k_enumerate<<<flow_blocks(width, kEnumBlock, (unsigned)(X.sms * X.tune->enumBlocksPerSm), X.sms), kEnumBlock, 0,
                           s>>>(A);
         } else {
-            k_enumerate_warp<<<flow_blocks(width, kEnumBlock / 32, (unsigned)(X.sms * std::min(X.tune->enumBlocksPerSm, 6)),
+            k_enumerate_warp<<<flow_blocks(width, kEnumBlock / 32, (unsigned)(X.sms * std::min(X.tune->enumBlocksPerSm, 8)),
                                            X.sms), kEnumBlock, 0, s>>>(A);
         }
         X.launched(1);
