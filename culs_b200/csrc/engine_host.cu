@@ -206,7 +206,12 @@ static bool decode_lib(const unsigned char *b, size_t n, RwLib &L) {
     memcpy(L.nRoots, nr, kNumClasses);
     memset(L.node, 0, sizeof L.node);
     memset(L.roots, 0, sizeof L.roots);
-    memset(L.batch, 0xFF, sizeof L.batch);
+    memset(L.uses, 0, sizeof L.uses);
+    memset(L.pairNode, 0, sizeof L.pairNode);
+    memset(L.pairMask, 0, sizeof L.pairMask);
+    memset(L.pairRest, 0, sizeof L.pairRest);
+    memset(L.rootPairs, 0, sizeof L.rootPairs);
+    memset(L.rootDepth, 0, sizeof L.rootDepth);
     memset(L.rootCone, 0, sizeof L.rootCone);
     for (int c = 0; c < kNumClasses; c++) {
         if (L.nNodes[c] > kMaxLibNodes - 4 || L.nRoots[c] > 16) return false;
@@ -221,30 +226,23 @@ static bool decode_lib(const unsigned char *b, size_t n, RwLib &L) {
         cur += L.nRoots[c];
         for (int i = 0; i < L.nNodes[c]; i++)  // fanins precede their node
             if (ln_f0(L.node[c][i]) >= i + 4 || ln_f1(L.node[c][i]) >= i + 4) return false;
-        // evaluation batches: nodes by depth (inputs at depth 0), index order
-        // within a depth, at most kLibBatch per batch
-        int depth[kMaxLibNodes], maxDepth = 0;
-        for (int i = 0; i < 4; i++) depth[i] = 0;
+        // readers, and the nodes over two inputs by pair and complements
+        const int pairBase[4][4] = {{0, 0, 4, 8}, {0, 0, 12, 16}, {0, 0, 0, 20}, {0, 0, 0, 0}};
         for (int i = 0; i < L.nNodes[c]; i++) {
-            const int d0 = depth[ln_f0(L.node[c][i])], d1 = depth[ln_f1(L.node[c][i])];
-            depth[i + 4] = 1 + (d0 > d1 ? d0 : d1);
-            maxDepth = depth[i + 4] > maxDepth ? depth[i + 4] : maxDepth;
-        }
-        int nb = 0;
-        for (int d = 1; d <= maxDepth; d++) {
-            uint32_t ent[kLibBatch];
-            int k = 0;
-            for (int i = 0; i <= L.nNodes[c]; i++) {
-                const bool flush = k == kLibBatch || (i == L.nNodes[c] && k > 0);
-                if (flush) {
-                    for (int e = k; e < kLibBatch; e++) ent[e] = kNoLibNode;
-                    L.batch[c][nb++] = uint4{ent[0], ent[1], ent[2], ent[3]};
-                    k = 0;
-                }
-                if (i < L.nNodes[c] && depth[i + 4] == d) ent[k++] = L.node[c][i] | ((uint32_t)i << 18);
+            const uint32_t w = L.node[c][i];
+            int f0 = ln_f0(w), f1 = ln_f1(w), c0 = ln_c0(w), c1 = ln_c1(w);
+            L.uses[c][f0] |= 1ull << (i + 4);
+            L.uses[c][f1] |= 1ull << (i + 4);
+            if (f0 >= 4 || f1 >= 4) continue;
+            if (f0 > f1) std::swap(f0, f1), std::swap(c0, c1);
+            const int e = pairBase[f0][f1] + 2 * c0 + c1;
+            if (f0 == f1 || L.pairNode[c][e]) {
+                L.pairRest[c] |= 1ull << (i + 4);
+            } else {
+                L.pairNode[c][e] = (uint8_t)(i + 4);
+                L.pairMask[c] |= 1u << e;
             }
         }
-        L.nBatches[c] = (uint8_t)nb;
         // root cones over the internal nodes
         unsigned long long cone[kMaxLibNodes] = {0, 0, 0, 0};
         for (int i = 0; i < L.nNodes[c]; i++)
@@ -253,11 +251,24 @@ static bool decode_lib(const unsigned char *b, size_t n, RwLib &L) {
             if (L.roots[c][r] >= 4 + L.nNodes[c]) return false;
             L.rootCone[c][r] = cone[L.roots[c][r]];
         }
+        for (int r = 0; r < L.nRoots[c]; r++) {
+            uint32_t p = 0;
+            for (int e = 0; e < 24; e++)
+                if (L.pairNode[c][e] && ((L.rootCone[c][r] >> L.pairNode[c][e]) & 1)) p |= 1u << e;
+            if (__builtin_popcountll(L.rootCone[c][r]) > 1) p |= 1u << 31;
+            L.rootPairs[c][r] = p;
+        }
+        // longest paths from each input
+        for (int in = 0; in < 4; in++) {
+            int far[kMaxLibNodes] = {0, 0, 0, 0};
+            far[in] = 1;
+            for (int i = 0; i < L.nNodes[c]; i++) {
+                const int f = std::max(far[ln_f0(L.node[c][i])], far[ln_f1(L.node[c][i])]);
+                far[i + 4] = f ? f + 1 : 0;
+            }
+            for (int r = 0; r < L.nRoots[c]; r++) L.rootDepth[c][r] |= (uint32_t)far[L.roots[c][r]] << (8 * in);
+        }
     }
-    int order[kNumClasses];
-    for (int c = 0; c < kNumClasses; c++) order[c] = c;
-    std::stable_sort(order, order + kNumClasses, [&](int a, int b) { return L.nBatches[a] < L.nBatches[b]; });
-    for (int i = 0; i < kNumClasses; i++) L.classSlot[order[i]] = (uint8_t)i;
     return cur == n;
 }
 

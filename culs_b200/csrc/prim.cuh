@@ -28,6 +28,7 @@ class Arena {
         return static_cast<T *>(alloc(n * sizeof(T)));
     }
     void reset() { used_ = 0; }
+    void release(size_t used) { used_ = used; }  // gives back what was taken since used() returned this
     size_t used() const { return used_; }
     size_t capacity() const { return cap_; }
     size_t high_water() const { return high_; }

@@ -31,24 +31,27 @@ struct RwLib {
     // fanin0 (bits 0-7) | fanin1 (bits 8-15) | compl0 (bit 16) | compl1 (bit 17)
     uint32_t node[kNumClasses][kMaxLibNodes];
     uint8_t roots[kNumClasses][16];
-    // The same internal nodes regrouped for evaluation: batches of up to
-    // kLibBatch nodes of equal depth (every fanin in an earlier batch), in
-    // order of depth.  Entry = node word | index j (bits 18-23), or
-    // kNoLibNode for an unused entry.  Nodes of one batch never read each
-    // other, so their table probes are issued together.
-    uint4 batch[kNumClasses][kMaxLibNodes];
-    uint8_t nBatches[kNumClasses];
+    // Evaluation reaches a library node through a matched fanin, or, when
+    // both its fanins are inputs, through the pair's filter bits:
+    // uses[j]: the nodes that read node j;
+    // pairNode[4 * pair + 2 * c_lo + c_hi]: the node that ANDs inputs lo < hi
+    // with these complements, pairs in the order 01 02 03 12 13 23, 0 when
+    // there is none, and pairMask its non-zero entries;
+    // pairRest: nodes over two inputs that have no entry of their own.
+    unsigned long long uses[kNumClasses][kMaxLibNodes];
+    uint8_t pairNode[kNumClasses][24];
+    uint32_t pairMask[kNumClasses];
+    unsigned long long pairRest[kNumClasses];
+    // Per class and root: the pair entries in its cone (bits 0-23), and bit 31
+    // when the root itself is not one of them.
+    uint32_t rootPairs[kNumClasses][16];
     // Per class and root: bit j set for every internal node j (j >= 4) in
     // the root's cone, the root included.
     unsigned long long rootCone[kNumClasses][16];
-    // Evaluation order of the classes: by number of batches, then class, so
-    // that cut items sorted by this slot put forests of equal batch count
-    // side by side.
-    uint8_t classSlot[kNumClasses];
+    // Per class and root: byte i = 1 + the longest path from input i to the
+    // root, 0 when the root does not depend on it.
+    uint32_t rootDepth[kNumClasses][16];
 };
-constexpr int kLibBatch = 4;
-constexpr uint32_t kNoLibNode = 0xFFFFFFFFu;
-static_assert(kLibBatch == 4, "a batch is one uint4");
 
 CULS_HD int npn_phase(uint32_t w) { return (int)(w & 31u); }
 CULS_HD int npn_perm(uint32_t w) { return (int)((w >> 8) & 31u); }
@@ -422,7 +425,7 @@ CULS_HD int and_lookup(const AndTable &t, int in0, int in1, int c0, int c1, int 
 struct alignas(16) TabSlot {
     unsigned long long key;
     int val;  // smallest position with this key
-    int lvl;  // its level (equal for all nodes with one key: same fanins)
+    int pad;
 };
 
 struct RegionTable {
@@ -449,13 +452,12 @@ CULS_HD uint32_t region_home(unsigned long long key, uint32_t size) {
     return (uint32_t)(((unsigned long long)(h ^ (h >> 15)) * size) >> 32);
 }
 
-CULS_HD int region_insert(const TabRegion &t, unsigned long long key, int val, int lvl, int *status) {
+CULS_HD int region_insert(const TabRegion &t, unsigned long long key, int val, int *status) {
     uint32_t h = region_home(key, t.size);
     for (uint32_t probe = 0; probe < t.size; probe++) {
         unsigned long long prev = at_cas(&t.slots[h].key, kEmptyKey, key);
         if (prev == kEmptyKey || prev == key) {
             at_min(&t.slots[h].val, val);
-            t.slots[h].lvl = lvl;
             return (int)h;
         }
         if (++h == t.size) h = 0;
@@ -483,34 +485,6 @@ CULS_HD int region_find(const TabRegion &t, unsigned long long key, int *status)
     return -1;
 }
 
-CULS_HD int4 region_load(const TabRegion &t, uint32_t h) {
-#if defined(__CUDA_ARCH__)
-    return *reinterpret_cast<const int4 *>(&t.slots[h]);
-#else
-    const TabSlot &x = t.slots[h];
-    return int4{(int)(uint32_t)x.key, (int)(uint32_t)(x.key >> 32), x.val, x.lvl};
-#endif
-}
-
-// Finishes a lookup whose home slot was already loaded into s: returns
-// {position, level} of the key, or {-1, 0} when absent.  The home index is
-// recomputed only when the probe goes on past it.
-CULS_HD int2 region_resolve(const TabRegion &t, unsigned long long key, int4 s, int *status) {
-    uint32_t h = 0;
-    for (uint32_t probe = 0; probe < t.size; probe++) {
-        if (probe > 0) {
-            if (probe == 1) h = region_home(key, t.size);
-            if (++h == t.size) h = 0;
-            s = region_load(t, h);
-        }
-        const unsigned long long k = ((unsigned long long)(uint32_t)s.y << 32) | (uint32_t)s.x;
-        if (k == key) return int2{s.z, s.w};
-        if (k == kEmptyKey) return int2{-1, 0};
-    }
-    set_status(status, kDevTableFull);
-    return int2{-1, 0};
-}
-
 // TableLookup (src/algorithms/rewrite.cu:346-367) on a graph's region.
 CULS_HD int region_and_lookup(const TabRegion &t, int in0, int in1, int c0, int c1, int *status) {
     if (in0 > in1) {
@@ -531,115 +505,78 @@ struct EvalIn {
     const int *level;
     const RwLib *lib;
     TabRegion tab;       // the region of the evaluated node's graph
+    const unsigned long long *pairs;  // per node: the filter of its table keys (pair_bit)
     int *status;
 };
 
-// 8-entry reference table of CalcMFFC (src/algorithms/rewrite.cu:296-316).
-// Every access below names its entry by a literal index (CULS_EACH8), never
-// by a loop variable left to the unroller, so the table stays in registers
-// however large the calling kernel grows.
-struct MffcTab {
-    int size;
-    int id[8];
-    int num[8];
-};
+// A node's 64-bit filter says which ANDs it may be the higher fanin of: bit
+// pair_bit(lo) + 2 * c_lo + c_hi is set for every key (lo, this node, c_lo,
+// c_hi) in the table.  A clear bit proves the key absent.
+// Four such words a cut, read for all six input pairs, stand in for most of
+// the table probes that fail.
+CULS_HD int pair_bit(int lo) { return (int)(((uint32_t)lo * 0x9E3779B1u) >> 28) << 2; }
 
-#define CULS_EACH8(X) X(0) X(1) X(2) X(3) X(4) X(5) X(6) X(7)
-
-CULS_HD int pick8(const int (&v)[8], int i) {
-    int r = v[0];
-#define CULS_PICK8(k) \
-    if (k == i) r = v[k];
-    CULS_EACH8(CULS_PICK8)
-#undef CULS_PICK8
-    return r;
+CULS_HD int ctz64(uint64_t x) {
+#if defined(__CUDA_ARCH__)
+    return __ffsll((long long)x) - 1;
+#else
+    return __builtin_ctzll(x);
+#endif
 }
 
-// Decrease, src/algorithms/rewrite.cu:296-309.  *slot receives the table
-// entry whose count was returned (unchanged for leaves and a full table).
-CULS_HD int mffc_decrease(int v, MffcTab &t, const int (&leaves)[4], const int *ref, int *slot) {
-    if (v == leaves[0] || v == leaves[1] || v == leaves[2] || v == leaves[3]) return 1;
-    int found = -1;
-#define CULS_FIND8(k) \
-    if (found < 0 && k < t.size && t.id[k] == v) found = k;
-    CULS_EACH8(CULS_FIND8)
-#undef CULS_FIND8
-    if (found >= 0) {
-        int r = 0;
-#define CULS_DEC8(k) \
-    if (k == found) r = --t.num[k];
-        CULS_EACH8(CULS_DEC8)
-#undef CULS_DEC8
-        *slot = found;
-        return r;
-    }
-    if (t.size == 8) return 1;
-    const int r = ref[v] - 1;
-#define CULS_ADD8(k)    \
-    if (k == t.size) {  \
-        t.id[k] = v;    \
-        t.num[k] = r;   \
-    }
-    CULS_EACH8(CULS_ADD8)
-#undef CULS_ADD8
-    *slot = t.size;
-    t.size++;
-    return r;
-}
-
-// Bit i set when table entry i exists with a zero count: the entries
-// IsDeleted (src/algorithms/rewrite.cu:312-316) reports.  Table ids are
-// distinct, so the counts are no longer needed once this mask is taken.
-CULS_HD uint32_t mffc_zero_mask(const MffcTab &t) {
-    uint32_t z = 0;
-#define CULS_ZERO8(k) \
-    if (k < t.size && t.num[k] == 0) z |= 1u << k;
-    CULS_EACH8(CULS_ZERO8)
-#undef CULS_ZERO8
-    return z;
-}
-
-// IsDeleted, src/algorithms/rewrite.cu:312-316, on the ids and zero mask
-CULS_HD int mffc_deleted(int v, const int (&id)[8], uint32_t zero) {
-    if (!zero) return 0;  // the common case: the MFFC is the root alone
-    int del = 0;
-#define CULS_DEL8(k) del |= ((zero >> k) & 1u) && id[k] == v;
-    CULS_EACH8(CULS_DEL8)
-#undef CULS_DEL8
-    return del;
-}
-
-// CalcMFFC, src/algorithms/rewrite.cu:319-326, with the recursion replayed
-// on a register stack.  A frame above the root is entered only when a table
-// count reaches zero, so it is named by its table entry (3 bits); its state
-// (next fanin to visit) takes 2 bits.  At most nine frames exist (eight
-// table entries plus the root), and the result -- the root plus every node
-// entered -- is the number of frames pushed.
-CULS_HD int mffc_size(const EvalIn &E, int root, const int (&leaves)[4], MffcTab &t) {
-    uint32_t idxs = 0, states = 0;
-    int sp = 0, count = 1;
+// CalcMFFC (src/algorithms/rewrite.cu:296-326) of root: its count, and the
+// nDel table entries whose reference count reached zero, which are those that
+// IsDeleted reports, at del (room for 8).
+//
+// The reference's table of 8 entries is held as ids in registers, every access
+// by a literal index, and a byte per count.  A byte is enough: at most nine
+// nodes are entered, so at most 18 decrements happen, and a count that starts
+// at 255 or above never reaches zero.  The recursion visits a node's first
+// fanin and what is below it before the second, so the second fanins wait on a
+// stack, one per node entered.
+CULS_HD int mffc_size(const EvalIn &E, int root, const int (&leaves)[4], int *del, int *nDel) {
+    int id[8], wait[10];
+#pragma unroll
+    for (int k = 0; k < 8; k++) id[k] = -1;
+    uint64_t counts = 0;
+    int size = 0, sp = 1, count = 1;
+    wait[0] = E.L1[root] >> 1;
+    int v = E.L0[root] >> 1;
     while (true) {
-        const int cur = sp == 0 ? root : pick8(t.id, (int)((idxs >> (3 * sp)) & 7u));
-        const uint32_t st = (states >> (2 * sp)) & 3u;
-        if (st < 2) {
-            const int v = (st == 0 ? E.L0[cur] : E.L1[cur]) >> 1;
-            states += 1u << (2 * sp);
-            int slot = 0;
-            if (mffc_decrease(v, t, leaves, E.ref, &slot) == 0) {
-                if (sp + 1 >= 10) {
-                    set_status(E.status, kDevStackOverflow);
-                    return count;
-                }
-                sp++;
-                idxs = (idxs & ~(7u << (3 * sp))) | ((uint32_t)slot << (3 * sp));
-                states &= ~(3u << (2 * sp));
-                count++;
+        bool zero = false;  // Decrease(v) returned zero
+        if (v != leaves[0] && v != leaves[1] && v != leaves[2] && v != leaves[3]) {
+            uint32_t at = 0;
+#pragma unroll
+            for (int k = 0; k < 8; k++) at |= id[k] == v ? 1u << k : 0u;
+            if (at) {
+                const int sh = 8 * ctz64(at);
+                const uint64_t c = (counts >> sh) & 255u, c1 = (c - 1) & 255u;
+                counts ^= (c ^ c1) << sh;
+                zero = c1 == 0;
+            } else if (size < 8) {  // a full table returns 1
+                const uint32_t r = (uint32_t)E.ref[v] - 1u;
+#pragma unroll
+                for (int k = 0; k < 8; k++) id[k] = k == size ? v : id[k];
+                counts |= (uint64_t)(r < 255u ? r : 255u) << (8 * size);
+                size++;
+                zero = r == 0;
             }
-            continue;
         }
-        if (sp == 0) return count;
-        sp--;
+        if (zero) {
+            count++;
+            wait[sp++] = E.L1[v] >> 1;
+            v = E.L0[v] >> 1;
+        } else {
+            if (sp == 0) break;
+            v = wait[--sp];
+        }
     }
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++)
+        if (k < size && ((counts >> (8 * k)) & 255u) == 0) del[n++] = id[k];
+    *nDel = n;
+    return count;
 }
 
 // True when CalcMFFC of root w.r.t. these leaves is the root alone and no
@@ -654,71 +591,6 @@ CULS_HD bool mffc_trivial(const EvalIn &E, int root, const int (&leaves)[4]) {
     return (l0 || E.ref[f0] >= 2) && (l1 || E.ref[f1] >= 2);
 }
 
-CULS_HD int clz64(uint64_t x) {
-#if defined(__CUDA_ARCH__)
-    return __clzll((long long)x);
-#else
-    return __builtin_clzll(x);
-#endif
-}
-
-// Number of library nodes the subgraph rooted at rt adds: unmatched nodes
-// reachable from rt through unmatched nodes (Eval, rewrite.cu:369-374).
-// unmatched has bit j set for library node j without a match.  A node is
-// matched only when both its fanins are (inputs always are), so a matched
-// node's whole cone is matched and every unmatched node of rt's cone is
-// reached through unmatched nodes: the count is the unmatched part of the
-// cone.
-CULS_HD int lib_added(const RwLib *lib, int cls, int out, uint64_t unmatched) {
-    return popc64(lib->rootCone[cls][out] & unmatched);
-}
-
-// One library node of an evaluation batch (the body of EvaluateNode's node
-// loop, src/algorithms/rewrite.cu:400-428), split in two so that a batch's
-// table probes are in flight together: lib_probe_issue sets the node's level
-// from its fanins and, when both fanins are matched (and not to the root),
-// loads the home slot of its structural-hash key; lib_probe_finish resolves
-// the probe into a match or marks the node unmatched.
-struct LibProbe {
-    unsigned long long key;
-    int4 slot;  // the key's home slot
-    int num;    // library index, or -1 when no probe is pending
-};
-
-template <class LevT>
-CULS_HD void lib_probe_issue(const EvalIn &E, int q, uint32_t w, int isC, int *match, LevT *mlev, int stride,
-                             uint64_t &unmatched, LibProbe &p) {
-    p.num = -1;
-    if (w == kNoLibNode) return;
-    const int num = (int)((w >> 18) & 63u) + 4;
-    const int in0 = ln_f0(w), in1 = ln_f1(w);
-    const int m0 = match[in0 * stride], m1 = match[in1 * stride];
-    const int lv0 = mlev[in0 * stride], lv1 = mlev[in1 * stride];
-    mlev[num * stride] = (LevT)(1 + (lv0 > lv1 ? lv0 : lv1));
-    match[num * stride] = -1;
-    const bool uin0 = in0 >= 4 && ((unmatched >> in0) & 1ull);
-    const bool uin1 = in1 >= 4 && ((unmatched >> in1) & 1ull);
-    if (uin0 || uin1 || m0 == q || m1 == q) {
-        unmatched |= 1ull << num;
-        return;
-    }
-    // the reference's isC mask only has input bits (0..3)
-    int cc0 = (in0 < 4 ? ((isC >> in0) & 1) : 0) ^ ln_c0(w);
-    int cc1 = (in1 < 4 ? ((isC >> in1) & 1) : 0) ^ ln_c1(w);
-    int a = m0, b = m1;
-    if (a > b) {  // TableLookup orders the ids
-        const int x = a;
-        a = b;
-        b = x;
-        const int y = cc0;
-        cc0 = cc1;
-        cc1 = y;
-    }
-    p.key = and_key(a, b, cc0, cc1);
-    p.slot = region_load(E.tab, region_home(p.key, E.tab.size));
-    p.num = num;
-}
-
 // IsDeleted (src/algorithms/rewrite.cu:312-316) on the MFFC's nodes: the
 // table entries whose count reached zero, nDel of them at del.
 CULS_HD bool mffc_member(int v, int nDel, const int *del) {
@@ -727,85 +599,142 @@ CULS_HD bool mffc_member(int v, int nDel, const int *del) {
     return false;
 }
 
-template <class LevT>
-CULS_HD void lib_probe_finish(const EvalIn &E, const LibProbe &p, int nDel, const int *del, int *match, LevT *mlev,
-                              int stride, uint64_t &unmatched) {
-    if (p.num < 0) return;
-    // the slot carries the node's level, so a hit needs no second load
-    const int2 r = region_resolve(E.tab, p.key, p.slot, E.status);
-    if (r.x != -1 && !mffc_member(r.x, nDel, del)) {
-        match[p.num * stride] = r.x;
-        mlev[p.num * stride] = (LevT)r.y;
-    } else {
-        unmatched |= 1ull << p.num;
-    }
+// The four complement combinations of the AND of inputs lo < hi (nodes a and
+// b, input complements na and nb) that the filters leave possible, as bits
+// 2 * c_lo + c_hi in the library's terms.
+CULS_HD uint32_t pair_possible(int a, int b, unsigned long long fa, unsigned long long fb, int na, int nb) {
+    const bool sw = a > b;  // TableLookup orders the ids
+    uint32_t n = (uint32_t)((sw ? fa : fb) >> pair_bit(sw ? b : a)) & 15u;
+    if (!n) return 0;
+    const uint32_t t = (n & 9u) | ((n & 2u) << 1) | ((n & 4u) >> 1);
+    if (sw) n = t;
+    if (a == b) n |= t;
+    if (na) n = ((n << 2) | (n >> 2)) & 15u;
+    if (nb) n = ((n & 5u) << 1) | ((n >> 1) & 5u);
+    return n;
 }
 
-template <class T>
-CULS_HD T pick4v(const T (&v)[4], int i) {
-    return i == 0 ? v[0] : (i == 1 ? v[1] : (i == 2 ? v[2] : v[3]));
+// A cut as its class sees it: the four inputs' nodes, their complements (the
+// reference's isC mask only has input bits, 0..3), and the class's pair
+// entries that the filters leave possible.
+struct CutView {
+    int in[4];
+    int isC, cls;
+    uint32_t possible;
+};
+
+CULS_HD CutView cut_view(const EvalIn &E, int cpos, uint32_t pk, int4 l) {
+    CutView v;
+    const uint32_t npn = E.lib->npn[pk & 0xFFFFu];
+    v.isC = npn_phase(npn) & 15;
+    v.cls = npn_class(npn);
+    const uint32_t perm = *reinterpret_cast<const uint32_t *>(E.lib->perm4[npn_perm(npn)]);
+    const int leaves[4] = {l.x, l.y, l.z, packed_nleaves(pk) == 3 ? cpos : l.w};
+    unsigned long long f[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const int p = (int)((perm >> (8 * j)) & 255u);
+        v.in[j] = p == 0 ? leaves[0] : (p == 1 ? leaves[1] : (p == 2 ? leaves[2] : leaves[3]));
+        f[j] = E.pairs[v.in[j]];
+    }
+    v.possible = 0;
+#pragma unroll
+    for (int i = 0, k = 0; i < 3; i++)
+#pragma unroll
+        for (int j = i + 1; j < 4; j++, k += 4)
+            v.possible |= pair_possible(v.in[i], v.in[j], f[i], f[j], (v.isC >> i) & 1, (v.isC >> j) & 1) << k;
+    v.possible &= E.lib->pairMask[v.cls];
+    return v;
+}
+
+// The roots that may add no more than spare nodes, as a mask: a cone's pair
+// nodes that are not possible stay unmatched, and with them the root above
+// them.  Most cuts are left with one or two roots, one of them the node's own
+// structure.
+CULS_HD uint32_t open_roots(const EvalIn &E, const CutView &v, int spare) {
+    const int nr = E.lib->nRoots[v.cls];
+    uint32_t open = 0;
+    for (int out = 0; out < nr; out++) {
+        const uint32_t p = E.lib->rootPairs[v.cls][out];
+        const int missing = popc32(p & 0xFFFFFFu & ~v.possible);
+        if (missing + (missing ? (int)(p >> 31) : 0) <= spare) open |= 1u << out;
+    }
+    return open;
 }
 
 // Best replacement of one cut: the body of EvaluateNode's cut loop
-// (src/algorithms/rewrite.cu:386-445) for cut slot packed word pk with
-// leaves l.  match/mlev are 54-entry scratch arrays with element j at
-// index j * stride.  Returns the first root (in root order) with the highest
-// gain and, among equal gains, the lowest level: out < 0 when no root
-// qualifies.
+// (src/algorithms/rewrite.cu:386-445).  Returns the first root (in root
+// order) with the highest gain and, among equal gains, the lowest level:
+// out < 0 when no root qualifies.
 struct CutBest {
     int gain, level, out;
 };
 
-// LevT holds library-node levels: int, or uint16_t when every level of the
-// graph plus the forest depth stays below 65,535.
+// saved is CalcMFFC's count for this cut, del its nDel MFFC nodes (the table
+// entries whose count reached zero), least the smallest gain that counts and
+// roots the ones to consider (the others cannot qualify).
 //
-// saved is CalcMFFC's count for this cut, and del its nDel MFFC nodes (the
-// table entries whose count reached zero), computed beforehand.
-template <class LevT>
-CULS_HD CutBest eval_cut(const EvalIn &E, int q, int cpos, uint32_t pk, int4 l, bool useZeros, int *match, LevT *mlev,
-                         int stride, int saved, int nDel, const int *del) {
+// A library node can be matched only when both its fanins are, to nodes
+// other than q and its MFFC.  So the walk starts from the input pairs whose
+// AND the filters leave possible, and goes on through the readers of each
+// matched node, in index order (fanins precede their node): the nodes that it
+// does not reach are those that the reference's loop over the whole forest
+// (rewrite.cu:400-428) leaves unmatched.
+//
+// No level is kept: a matched node's fanins are the nodes its library fanins
+// are matched to, so every library node, matched or not, is one level above
+// the higher of its fanins, and a root's level follows from the inputs'
+// levels and its longest paths to them.
+CULS_HD CutBest eval_cut(const EvalIn &E, int q, const CutView &v, uint32_t roots, int least, int saved, int nDel,
+                         const int *del) {
     CutBest best{-1, 0, -1};
-    const uint32_t nLeaves = packed_nleaves(pk);
-    const int leaves[4] = {l.x, l.y, l.z, nLeaves == 3 ? cpos : l.w};
-    const uint32_t npn = E.lib->npn[pk & 0xFFFFu];
-    const int uPhase = npn_phase(npn), cls = npn_class(npn);
-    const uint32_t perm = *reinterpret_cast<const uint32_t *>(E.lib->perm4[npn_perm(npn)]);
-    int isC = 0;
+    const int cls = v.cls;
+    int match[kMaxLibNodes];
+    uint64_t cones = 0;
+    for (uint32_t m = roots; m; m &= m - 1) cones |= E.lib->rootCone[cls][ctz64(m)];
+    uint64_t todo = E.lib->pairRest[cls];
+    for (uint32_t p = v.possible; p; p &= p - 1) todo |= 1ull << E.lib->pairNode[cls][ctz64(p)];
+    todo &= cones;
+    uint64_t have = 15, self = 0;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-        const int m = pick4v(leaves, (int)((perm >> (8 * j)) & 255u));
-        match[j * stride] = m;
-        mlev[j * stride] = (LevT)E.level[m];
-        if (uPhase >> j & 1) isC |= 1 << j;
+    for (int j = 0; j < 4; j++) match[j] = v.in[j];
+    while (todo) {
+        const int n = ctz64(todo);
+        todo &= todo - 1;
+        const uint32_t w = E.lib->node[cls][n - 4];
+        const int in0 = ln_f0(w), in1 = ln_f1(w);
+        if (!((have >> in0) & (have >> in1) & 1ull)) continue;
+        const int cc0 = (in0 < 4 ? ((v.isC >> in0) & 1) : 0) ^ ln_c0(w);
+        const int cc1 = (in1 < 4 ? ((v.isC >> in1) & 1) : 0) ^ ln_c1(w);
+        const int r = region_and_lookup(E.tab, match[in0], match[in1], cc0, cc1, E.status);
+        if (r == -1 || mffc_member(r, nDel, del)) continue;
+        if (r == q) {
+            self |= 1ull << n;
+        } else {
+            match[n] = r;
+            have |= 1ull << n;
+            todo |= E.lib->uses[cls][n] & cones;
+        }
     }
-    // The library nodes in the reference's index order, regrouped into
-    // batches of equal depth: every node reads only its fanins' entries, so
-    // this order yields the same match, level and unmatched bits.
-    uint64_t unmatched = 0;
-    const int nb = E.lib->nBatches[cls];
-    const uint4 *lbatch = E.lib->batch[cls];
-    for (int bi = 0; bi < nb; bi++) {
-        const uint4 bw = lbatch[bi];
-        LibProbe p0, p1, p2, p3;  // the batch's probes in flight together
-        lib_probe_issue(E, q, bw.x, isC, match, mlev, stride, unmatched, p0);
-        lib_probe_issue(E, q, bw.y, isC, match, mlev, stride, unmatched, p1);
-        lib_probe_issue(E, q, bw.z, isC, match, mlev, stride, unmatched, p2);
-        lib_probe_issue(E, q, bw.w, isC, match, mlev, stride, unmatched, p3);
-        lib_probe_finish(E, p0, nDel, del, match, mlev, stride, unmatched);
-        lib_probe_finish(E, p1, nDel, del, match, mlev, stride, unmatched);
-        lib_probe_finish(E, p2, nDel, del, match, mlev, stride, unmatched);
-        lib_probe_finish(E, p3, nDel, del, match, mlev, stride, unmatched);
-    }
-    const int nr = E.lib->nRoots[cls];
-    for (int out = 0; out < nr; out++) {
-        const int rt = E.lib->roots[cls][out];
-        if (match[rt * stride] == q) continue;
-        const int added = lib_added(E.lib, cls, out, unmatched);
-        const int rtLevel = mlev[rt * stride];
-        const int gain = saved - added;
-        if (gain < 0 || (gain == 0 && !useZeros)) continue;
-        if (best.out >= 0 && (gain < best.gain || (gain == best.gain && rtLevel >= best.level))) continue;
-        best = CutBest{gain, rtLevel, out};
+    // Nodes a root adds (Eval, rewrite.cu:369-374): the unmatched ones of its
+    // cone.  A node is matched only when both its fanins are (inputs always
+    // are), so a matched node's whole cone is matched and every unmatched node
+    // of the cone is reached through unmatched nodes.
+    const uint64_t missing = ~(have | self);
+    for (uint32_t m = roots; m; m &= m - 1) {
+        const int out = ctz64(m);
+        const int gain = saved - popc64(E.lib->rootCone[cls][out] & missing);
+        if (gain < best.gain || gain < least) continue;
+        if ((self >> E.lib->roots[cls][out]) & 1ull) continue;
+        const uint32_t depth = E.lib->rootDepth[cls][out];
+        int level = 0;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const int d = (int)((depth >> (8 * j)) & 255u), x = E.level[v.in[j]] + d - 1;
+            level = d && x > level ? x : level;
+        }
+        if (best.out >= 0 && gain == best.gain && level >= best.level) continue;
+        best = CutBest{gain, level, out};
     }
     return best;
 }

@@ -6,10 +6,8 @@
 // so the region, cuts and fanin arrays a block touches belong to the few
 // graphs in flight.
 //
-// Evaluation works on (node, cut) items grouped by NPN class per warp (see
-// k_evaluate); the match/level scratch of a library walk lives in shared
-// memory laid out entry-major, so lanes reading the same library entry hit
-// distinct banks.
+// Evaluation works on (node, cut) items, and walks a class's library forest
+// only for those whose inputs' filters leave a root open (see k_evaluate).
 #include <algorithm>
 #include <vector>
 
@@ -20,14 +18,9 @@ namespace culs {
 namespace {
 
 constexpr int kEvalBlock = 64;
-constexpr int kLibSlots = 54;  // 4 inputs + at most 50 library nodes
-// Library scratch entries kept in shared memory per thread: forests of up to
-// kLibFast - 4 nodes (every frequent class) evaluate there; larger ones use
-// a per-thread column of a global scratch array.  The smaller shared
-// footprint keeps 22 warps resident per SM instead of 16.
-constexpr int kLibFast = 38;
-constexpr int kClassSlots = 224;  // >= the library's 222 classes, a multiple of 32
-static_assert(kClassSlots >= kNumClasses && kClassSlots % 32 == 0, "class slots");
+// Resident blocks an SM: at 56 registers a thread 16 fit.  256 graphs of up to
+// 200k ANDs: 8.8 ms with 12, 7.5 with 16, 7.7 with 20.
+constexpr int kEvalBlocksPerSm = 16;
 
 __global__ void k_table_clear(int64_t n, TabSlot *slots) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -37,7 +30,8 @@ __global__ void k_table_clear(int64_t n, TabSlot *slots) {
 
 // Inserts the AND nodes at graph-major indices [lo, hi) of byGraph.
 __global__ void k_table_build(int64_t nL0, int64_t lo, int64_t hi, const int *byGraph, const int *w0, const int *w1,
-                              const int *wg, const int *wlev, const DevGraph *dg, RegionTable tab, int *status) {
+                              const int *wg, const DevGraph *dg, RegionTable tab, unsigned long long *pairs,
+                              int *status) {
     int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i = lo + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += stride) {
         const int q = byGraph[i];
@@ -47,14 +41,15 @@ __global__ void k_table_build(int64_t nL0, int64_t lo, int64_t hi, const int *by
         int cp = dg[g].cpos;
         // rewrite.cu:454 skips nodes whose fanins are both the constant
         if ((f0 >> 1) == cp && (f1 >> 1) == cp) continue;
-        region_insert(table_region(tab, g), and_key(f0 >> 1, f1 >> 1, f0 & 1, f1 & 1), q, wlev[q], status);
+        region_insert(table_region(tab, g), and_key(f0 >> 1, f1 >> 1, f0 & 1, f1 & 1), q, status);
+        if ((f0 >> 1) <= (f1 >> 1))  // others no lookup finds
+            atomicOr(&pairs[f1 >> 1], 1ull << (pair_bit(f0 >> 1) + 2 * (f0 & 1) + (f1 & 1)));
     }
 }
 
 struct EvalArgs {
     int64_t nL0, lo, hi;  // evaluates the nodes at graph-major indices [lo, hi) of byGraph
     const int *byGraph;
-    int *scratch;  // 2 * kLibSlots ints per thread of the grid, thread-minor
     EvalIn E;
     RegionTable tab;
     const int4 *cutL;
@@ -68,188 +63,146 @@ struct EvalArgs {
     uint8_t *candFlag;
 };
 
-// Per-warp shared state of k_evaluate: the warp's nodes' evaluable cuts as
-// items grouped by class slot, and one result per (node, cut slot).
-// Nodes per lane in a warp's window: two (about 210 cut items to sort per
-// warp instead of 105) fill rounds better but measured slower on the
-// 4,096-graph batch.
-constexpr int kNodesPerLane = 1;
-constexpr int kWarpNodes = 32 * kNodesPerLane;
+// Per-warp shared state of k_evaluate: lists of the slots (local node * 8 +
+// cut slot) of the warp's nodes, and one result per slot.
+constexpr int kWarpNodes = 32;
 struct WarpItems {
-    int off[kClassSlots];          // class-slot counts, then exclusive offsets
-    uint16_t item[kWarpNodes * 8];  // local node * 8 + cut slot, in class-slot order
+    uint16_t item[kWarpNodes * 8];  // the evaluable cuts; then those that still need the walk
+    uint16_t full[kWarpNodes * 8];  // those whose MFFC needs the full traversal
     int2 res[kWarpNodes * 8];       // {gain * 16 + root index, level} or {-1, 0}
-    uint16_t full[kWarpNodes * 8];  // items whose MFFC needs the full traversal
-    uint8_t saved[kWarpNodes * 8];  // per item: CalcMFFC's count
-    uint8_t nDel[kWarpNodes * 8];   // per item: its MFFC nodes (in EvalArgs::mffcNodes)
+    uint16_t roots[kWarpNodes * 8];  // open_roots
+    uint8_t saved[kWarpNodes * 8];  // CalcMFFC's count
+    uint8_t nDel[kWarpNodes * 8];   // its MFFC nodes (in EvalArgs::mffcNodes)
 };
 
-// A warp takes 32 * kNodesPerLane consecutive nodes of the graph-major
-// order, sorts their evaluable cuts by NPN class -- classes ordered by their
-// forests' batch counts -- and evaluates them 32 at a time, so the lanes of
-// a round mostly walk the same library forest, or forests of as many
-// batches (the forests' sizes differ several-fold between classes).  Each
-// lane then folds its own nodes' results in slot order, the order of the
-// reference's loop.  Warps never wait for one another.  LevT is the type of
-// the library-node levels in the scratch (16-bit when the graph is shallow
-// enough, which halves that part of the shared memory).
-template <class LevT>
-__global__ void __launch_bounds__(kEvalBlock, 8) k_evaluate(EvalArgs A) {
-    __shared__ int s_match[kLibFast * kEvalBlock];
-    __shared__ LevT s_mlev[kLibFast * kEvalBlock];
+struct EvalItem {
+    int q, g, cpos;
+    uint32_t pk;
+    int4 l;
+};
+
+__device__ __forceinline__ EvalItem eval_item(const EvalArgs &A, int64_t base, int slot) {
+    EvalItem x;
+    x.q = A.byGraph[base + (slot >> 3)];
+    x.g = A.wg[x.q];
+    x.cpos = A.dg[x.g].cpos;
+    const int64_t idx = (int64_t)x.q * 8 + (slot & 7);
+    x.pk = (uint32_t)A.cutM[idx].y;
+    x.l = A.cutL[idx];
+    return x;
+}
+
+// Appends slot to list (n entries so far) for the lanes that keep theirs.
+__device__ __forceinline__ int append(uint16_t *list, int n, bool keep, int slot, int lane) {
+    const unsigned b = __ballot_sync(0xffffffffu, keep);
+    if (keep) list[n + __popc(b & ((1u << lane) - 1u))] = (uint16_t)slot;
+    return n + __popc(b);
+}
+
+// A warp takes 32 consecutive nodes of the graph-major order and sieves their
+// cuts, 32 items at a time and every list dense again after each step: the
+// evaluable cuts (about half of the slots), the MFFC traversal of those that
+// need one (a quarter), and the walk through the cones of the roots that
+// open_roots leaves.  Each lane then folds its own node's results in slot
+// order, the order of the reference's loop.  Warps never wait for one another.
+//
+// Bound by the walks' chains of dependent loads (three quarters of a warp's
+// time).  Walking the whole forest for every cut, cuts sorted by class so that
+// lanes walk forests of like depth, with the matches in shared memory (16
+// warps an SM): 13.3 ms for 256 graphs of up to 200k ANDs, 1.36 for a 1M-AND
+// layered graph; reached nodes only: 11.4 and 1.23; without the sort, 32 warps:
+// 7.6 and 0.81; open roots only: 7.4 and 0.81.  One probe a step for all lanes
+// of a warp: 7.7 and 0.84, as 2 of 6 roots are open on average and the lanes'
+// walks are short.
+__global__ void __launch_bounds__(kEvalBlock, kEvalBlocksPerSm) k_evaluate(EvalArgs A) {
     __shared__ WarpItems s_w[kEvalBlock / 32];
-    int *match = s_match + threadIdx.x;
-    LevT *mlev = s_mlev + threadIdx.x;
     const int lane = threadIdx.x & 31;
     WarpItems &W = s_w[threadIdx.x >> 5];
-    const int gtid = blockIdx.x * blockDim.x + threadIdx.x;
-    const int gstride = gridDim.x * blockDim.x;
-    int *gmatch = A.scratch + gtid;
-    LevT *gmlev = reinterpret_cast<LevT *>(A.scratch + (int64_t)kLibSlots * gstride) + gtid;
     const int64_t nWarpChunks = (A.hi - A.lo + kWarpNodes - 1) / kWarpNodes;
+    const int64_t warp = (int64_t)blockIdx.x * (kEvalBlock / 32) + (threadIdx.x >> 5);
     const int64_t warpStride = (int64_t)gridDim.x * (kEvalBlock / 32);
-    for (int64_t wc = (int64_t)blockIdx.x * (kEvalBlock / 32) + (threadIdx.x >> 5); wc < nWarpChunks;
-         wc += warpStride) {
+    int *const mffcNodes = A.mffcNodes + warp * (kWarpNodes * 8 * 8);
+    const int least = A.useZeros ? 0 : 1;
+    for (int64_t wc = warp; wc < nWarpChunks; wc += warpStride) {
         const int64_t base = A.lo + wc * kWarpNodes;
-        for (int c = lane; c < kClassSlots; c += 32) W.off[c] = 0;
-        __syncwarp();
-        // 1. this lane's nodes: their evaluable cuts and class slots
-        int64_t q[kNodesPerLane];
-        uint32_t clsRank[kNodesPerLane][8];
+        // 1. the evaluable cuts; a node's 8 slots lie side by side
+        const int q = base + lane < A.hi ? A.byGraph[base + lane] : -1;
+        int nItems = 0;
 #pragma unroll
-        for (int h = 0; h < kNodesPerLane; h++) {
-            const int local = h * 32 + lane;
-            q[h] = -1;
-            if (base + local < A.hi) {
-                q[h] = A.byGraph[base + local];
-                if (q[h] < A.nL0) q[h] = -1;  // constant or PI
+        for (int k = 0; k < 8; k++) {
+            const int slot = k * 32 + lane, nq = __shfl_sync(0xffffffffu, q, slot >> 3);
+            bool use = false;
+            if (nq >= A.nL0) {  // not the constant, a PI or past the end
+                const uint32_t pk = (uint32_t)A.cutM[(int64_t)nq * 8 + (slot & 7)].y;
+                use = packed_used(pk) && packed_nleaves(pk) >= 3;
             }
-#pragma unroll
-            for (int k = 0; k < 8; k++) {
-                clsRank[h][k] = 0xFFFFFFFFu;
-                W.res[local * 8 + k] = make_int2(-1, 0);
-                if (q[h] >= 0) {
-                    const uint32_t pk = (uint32_t)A.cutM[q[h] * 8 + k].y;
-                    if (packed_used(pk) && packed_nleaves(pk) >= 3) {
-                        const int cs = A.E.lib->classSlot[npn_class(A.E.lib->npn[pk & 0xFFFFu])];
-                        clsRank[h][k] = ((uint32_t)cs << 16) | (uint32_t)atomicAdd(&W.off[cs], 1);
-                    }
+            W.res[slot] = make_int2(-1, 0);
+            nItems = append(W.item, nItems, use, slot, lane);
+        }
+        __syncwarp();
+        // 2. the items whose MFFC is the root alone (nothing deleted): most
+        // end here.  Entries kept in item lie before those read.
+        int nFull = 0, nWalk = 0;
+        for (int it0 = 0; it0 < nItems; it0 += 32) {
+            const int slot = it0 + lane < nItems ? W.item[it0 + lane] : -1;
+            bool full = false, walk = false;
+            if (slot >= 0) {
+                const EvalItem x = eval_item(A, base, slot);
+                const int leaves[4] = {x.l.x, x.l.y, x.l.z, packed_nleaves(x.pk) == 3 ? x.cpos : x.l.w};
+                full = !mffc_trivial(A.E, x.q, leaves);
+                if (!full) {
+                    const uint32_t roots = open_roots(A.E, cut_view(A.E, x.cpos, x.pk, x.l), 1 - least);
+                    walk = roots != 0;
+                    W.roots[slot] = (uint16_t)roots;
+                    W.saved[slot] = 1;
+                    W.nDel[slot] = 0;
                 }
             }
+            __syncwarp();
+            nFull = append(W.full, nFull, full, slot, lane);
+            nWalk = append(W.item, nWalk, walk, slot, lane);
         }
         __syncwarp();
-        // 2. exclusive scan of the class-slot counts, kClassSlots / 32 per lane
-        int v[kClassSlots / 32], sum = 0;
-#pragma unroll
-        for (int t = 0; t < kClassSlots / 32; t++) {
-            v[t] = W.off[lane * (kClassSlots / 32) + t];
-            sum += v[t];
-        }
-        int inc = sum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, inc, d);
-            if (lane >= d) inc += y;
-        }
-        const int nItems = __shfl_sync(0xffffffffu, inc, 31);
-        int run = inc - sum;
-        __syncwarp();
-#pragma unroll
-        for (int t = 0; t < kClassSlots / 32; t++) {
-            W.off[lane * (kClassSlots / 32) + t] = run;
-            run += v[t];
-        }
-        __syncwarp();
-#pragma unroll
-        for (int h = 0; h < kNodesPerLane; h++)
-#pragma unroll
-            for (int k = 0; k < 8; k++)
-                if (clsRank[h][k] != 0xFFFFFFFFu)
-                    W.item[W.off[clsRank[h][k] >> 16] + (clsRank[h][k] & 0xFFFFu)] =
-                        (uint16_t)((h * 32 + lane) * 8 + k);
-        __syncwarp();
-        // 3. every item's MFFC: the trivial ones (the root alone, nothing
-        // deleted) at once, the others gathered and traversed 32 at a time,
-        // so the traversal runs in full rounds instead of in every round
-        int *const mffcNodes =
-            A.mffcNodes + ((int64_t)blockIdx.x * (kEvalBlock / 32) + (threadIdx.x >> 5)) * (kWarpNodes * 8 * 8);
-        int nFull = 0;
-        for (int it0 = 0; it0 < nItems; it0 += 32) {
-            const int it = it0 + lane;
-            bool full = false;
-            if (it < nItems) {
-                const int slot = W.item[it];
-                const int qq = A.byGraph[base + (slot >> 3)];
-                const int64_t idx = (int64_t)qq * 8 + (slot & 7);
-                const int4 l = A.cutL[idx];
-                const int leaves[4] = {l.x, l.y, l.z,
-                                       packed_nleaves((uint32_t)A.cutM[idx].y) == 3 ? A.dg[A.wg[qq]].cpos : l.w};
-                full = !mffc_trivial(A.E, qq, leaves);
-                W.saved[it] = 1;
-                W.nDel[it] = 0;
+        // 3. the others' MFFCs
+        for (int k0 = 0; k0 < nFull; k0 += 32) {
+            const int slot = k0 + lane < nFull ? W.full[k0 + lane] : -1;
+            bool walk = false;
+            if (slot >= 0) {
+                const EvalItem x = eval_item(A, base, slot);
+                const int leaves[4] = {x.l.x, x.l.y, x.l.z, packed_nleaves(x.pk) == 3 ? x.cpos : x.l.w};
+                int n;
+                const int saved = mffc_size(A.E, x.q, leaves, mffcNodes + slot * 8, &n);
+                const uint32_t roots = open_roots(A.E, cut_view(A.E, x.cpos, x.pk, x.l), saved - least);
+                walk = roots != 0;
+                W.roots[slot] = (uint16_t)roots;
+                W.saved[slot] = (uint8_t)saved;
+                W.nDel[slot] = (uint8_t)n;
             }
-            const unsigned b = __ballot_sync(0xffffffffu, full);
-            if (full) W.full[nFull + __popc(b & ((1u << lane) - 1u))] = (uint16_t)it;
-            nFull += __popc(b);
+            nWalk = append(W.item, nWalk, walk, slot, lane);
         }
         __syncwarp();
-        for (int k = lane; k < nFull; k += 32) {
-            const int it = W.full[k];
+        // 4. the walks
+        for (int it = lane; it < nWalk; it += 32) {
             const int slot = W.item[it];
-            const int qq = A.byGraph[base + (slot >> 3)];
-            const int64_t idx = (int64_t)qq * 8 + (slot & 7);
-            const int4 l = A.cutL[idx];
-            const int leaves[4] = {l.x, l.y, l.z,
-                                   packed_nleaves((uint32_t)A.cutM[idx].y) == 3 ? A.dg[A.wg[qq]].cpos : l.w};
-            MffcTab tab;
-            tab.size = 0;
-            const int saved = mffc_size(A.E, qq, leaves, tab);
-            const uint32_t zero = mffc_zero_mask(tab);
-            int *del = mffcNodes + it * 8;
-            int n = 0;
-#define CULS_KEEP(k)             \
-    if ((zero >> k) & 1u) del[n++] = tab.id[k];
-            CULS_EACH8(CULS_KEEP)
-#undef CULS_KEEP
-            W.saved[it] = (uint8_t)saved;
-            W.nDel[it] = (uint8_t)n;
-        }
-        __syncwarp();
-        // 4. evaluate the items, 32 per round, in class-slot order
-        for (int it = lane; it < nItems; it += 32) {
-            const int slot = W.item[it];
-            const int qq = A.byGraph[base + (slot >> 3)];
-            const int g = A.wg[qq];
+            const EvalItem x = eval_item(A, base, slot);
             EvalIn E = A.E;
-            E.tab = table_region(A.tab, g);
-            const int64_t idx = (int64_t)qq * 8 + (slot & 7);
-            const uint32_t pk = (uint32_t)A.cutM[idx].y;
-            const int4 l = A.cutL[idx];
-            const int cpos = A.dg[g].cpos;
-            CutBest b;
-            const int saved = W.saved[it], nDel = W.nDel[it];
-            const int *del = mffcNodes + it * 8;
-            if (4 + A.E.lib->nNodes[npn_class(A.E.lib->npn[pk & 0xFFFFu])] <= kLibFast)
-                b = eval_cut(E, qq, cpos, pk, l, A.useZeros != 0, match, mlev, kEvalBlock, saved, nDel, del);
-            else  // a large forest: scratch in global memory
-                b = eval_cut(E, qq, cpos, pk, l, A.useZeros != 0, gmatch, gmlev, gstride, saved, nDel, del);
+            E.tab = table_region(A.tab, x.g);
+            const CutBest b = eval_cut(E, x.q, cut_view(E, x.cpos, x.pk, x.l), W.roots[slot], least, W.saved[slot],
+                                       W.nDel[slot], mffcNodes + slot * 8);
             if (b.out >= 0) W.res[slot] = make_int2(b.gain * 16 + b.out, b.level);
         }
         __syncwarp();
-        // 5. fold each of this lane's nodes' cuts in slot order
-#pragma unroll
-        for (int h = 0; h < kNodesPerLane; h++) {
-            if (q[h] < 0) continue;
-            const int local = h * 32 + lane;
+        // 5. fold this lane's node's cuts in slot order
+        if (q >= A.nL0) {
             int bc = -1, bo = -1, gain = 0, level = 0;
 #pragma unroll
             for (int k = 0; k < 8; k++) {
-                const int2 r = W.res[local * 8 + k];
+                const int2 r = W.res[lane * 8 + k];
                 if (r.x >= 0) fold_cut_best(CutBest{r.x >> 4, r.y, r.x & 15}, k, bc, bo, gain, level);
             }
-            A.bestCut[q[h]] = (int8_t)bc;
-            A.bestOut[q[h]] = (uint8_t)(bo < 0 ? 0 : bo);
-            A.candFlag[q[h]] = bc >= 0;
+            A.bestCut[q] = (int8_t)bc;
+            A.bestOut[q] = (uint8_t)(bo < 0 ? 0 : bo);
+            A.candFlag[q] = bc >= 0;
         }
         __syncwarp();
     }
@@ -275,12 +228,12 @@ int rw_evaluate(ExecCtx &X, RwWork &w, const Batch &b) {
     w.bestOut = X.ar->get<uint8_t>(N);
     uint8_t *candFlag = X.ar->get<uint8_t>(N);
     w.cand = X.ar->get<int>(N);
-    // one resident wave: 8 blocks an SM (registers and shared memory); a
-    // second wave of a grid-stride kernel would only start as the first ends
-    const unsigned evalGrid = grid_1d(N, kEvalBlock, X.sms * 8);
-    int *scratch = X.ar->get<int>((size_t)2 * kLibSlots * evalGrid * kEvalBlock);
+    // one resident wave; a second wave of a grid-stride kernel would only start as the first ends
+    const unsigned evalGrid = grid_1d(N, kEvalBlock, X.sms * kEvalBlocksPerSm);
     int *mffcNodes = X.ar->get<int>((size_t)evalGrid * (kEvalBlock / 32) * kWarpNodes * 8 * 8);
-    if (!slots || !dOff || !w.bestCut || !w.bestOut || !candFlag || !w.cand || !scratch || !mffcNodes)
+    const size_t kept = X.ar->used();
+    unsigned long long *pairs = X.ar->get<unsigned long long>(N);
+    if (!slots || !dOff || !w.bestCut || !w.bestOut || !candFlag || !w.cand || !mffcNodes || !pairs)
         return X.fail(CULS_E_OOM, "rw: scratch arena exhausted (table)");
     w.tab = RegionTable{slots, dOff};
     int rc;
@@ -289,6 +242,7 @@ int rw_evaluate(ExecCtx &X, RwWork &w, const Batch &b) {
         return rc;
     if ((rc = X.check(cudaMemsetAsync(w.bestCut, 0xFF, N, s), "memset"))) return rc;
     if ((rc = X.check(cudaMemsetAsync(candFlag, 0, N, s), "memset"))) return rc;
+    if ((rc = X.check(cudaMemsetAsync(pairs, 0, sizeof *pairs * N, s), "memset"))) return rc;
     if (nAnd > 0) {
         k_table_clear<<<X.grid(nSlots), kBlock, 0, s>>>(nSlots, slots);
         X.mark(kMkEvalK0);
@@ -298,31 +252,26 @@ int rw_evaluate(ExecCtx &X, RwWork &w, const Batch &b) {
         // find them in L2 instead of DRAM (a single larger graph is a group
         // of its own).
         const int64_t kGroupSlots = (int64_t)X.tune->evalGroupMSlots << 20;
-        const bool lev16 = w.maxLevel + 64 < 0xFFFF;  // see the launch below
         int g0 = 0;
         while (g0 < w.G) {
             int g1 = g0 + 1;
             while (g1 < w.G && off[g1 + 1] - off[g0] <= kGroupSlots) g1++;
             const int64_t lo = b.hg[g0].base, hi = g1 < w.G ? (int64_t)b.hg[g1].base : N;
-            k_table_build<<<X.grid(hi - lo), kBlock, 0, s>>>(w.nL0, lo, hi, w.byGraph, w.w0, w.w1, w.wg, w.wlev,
-                                                             w.dg, w.tab, X.status);
-            EvalArgs A{w.nL0,  lo,     hi,     w.byGraph, scratch,
-                       EvalIn{w.w0, w.w1, w.ref, w.wlev, X.lib, TabRegion{}, X.status},
+            k_table_build<<<X.grid(hi - lo), kBlock, 0, s>>>(w.nL0, lo, hi, w.byGraph, w.w0, w.w1, w.wg,
+                                                             w.dg, w.tab, pairs, X.status);
+            EvalArgs A{w.nL0,  lo,     hi,     w.byGraph,
+                       EvalIn{w.w0, w.w1, w.ref, w.wlev, X.lib, TabRegion{}, pairs, X.status},
                        w.tab,  w.cutL, w.cutM, w.wg,      w.dg,
                        w.useZeros ? 1 : 0, mffcNodes, w.bestCut, w.bestOut, candFlag};
             const unsigned grid = std::min(evalGrid, X.grid(hi - lo, kEvalBlock));
-            // 16-bit library levels when no level of the batch, plus a
-            // forest's depth (at most 50 nodes), can reach 65,535
-            if (lev16)
-                k_evaluate<uint16_t><<<grid, kEvalBlock, 0, s>>>(A);
-            else
-                k_evaluate<int><<<grid, kEvalBlock, 0, s>>>(A);
+            k_evaluate<<<grid, kEvalBlock, 0, s>>>(A);
             X.launched(2);
             g0 = g1;
         }
         X.mark(kMkEvalK1);
         X.launched(1);
     }
+    X.ar->release(kept);  // the filters end here; what reuses their room comes later on this stream
     if ((rc = X.check(compact_flags(candFlag, N, w.cand, X.counters + 8, *X.ar, s), "compact"))) return rc;
     if ((rc = X.fetch("rw evaluate"))) return rc;
     w.nCand = X.hostSmall[8];
