@@ -247,6 +247,7 @@ __device__ __forceinline__ void enum_node_warp(const EnumArgs &A, int64_t q, int
     int ok = 1;
     if (lane < 2) ok = wait_ge(&A.done[lane ? u1 : u0], 1, A.status);
     ok = __all_sync(F, ok);
+    __syncwarp();  // orders the other lanes' reads below behind lanes 0 and 1's waits, which a vote does not
     int held = lane == 0 ? kTrivial : -1;  // candidate in this lane's slot
     uint32_t used = 1;
     if (ok) {

@@ -58,3 +58,24 @@ def test_every_cut_slot_matches_oracle(n_pis, n_ands, reach, wide_min):
             np.testing.assert_array_equal(D["selected"].reshape(-1, 10), o.dump_selected())
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("name", ["mult48", "deep"])
+def test_records_are_read_after_their_node_is_ready(name):
+    """Deep graphs, where a node's fanins become ready on another SM while its
+    warp waits for them: two lanes wait, the others read the fanins' records.
+    Repeated, as a read that came too early would not come so every time."""
+    g = C.gen_multiplier(48) if name == "mult48" else C.gen_layered(3, 40, 20, 20000, 400, 2, 0.0, True)
+    o = Oracle()
+    o.set_graph(to_oracle(g))
+    o.rw()
+    cuts, selected = o.dump_cuts(), o.dump_selected()
+    ctx = C.Context()
+    try:
+        for _ in range(6):
+            ctx.rw(ctx.upload(g), dump=True)
+            D = ctx.dump()
+            np.testing.assert_array_equal(D["cuts"].reshape(-1, 8, 9), cuts)
+            np.testing.assert_array_equal(D["selected"].reshape(-1, 10), selected)
+    finally:
+        ctx.close()
