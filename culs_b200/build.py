@@ -58,7 +58,7 @@ def _run(cmd):
 
 def build(force=False, jobs=None, verbose=False):
     BUILD.mkdir(exist_ok=True)
-    headers = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h")) + list(INC.glob("*.h"))
+    headers = list(CSRC.glob("*.cuh")) + list(CSRC.glob("*.h*")) + list(INC.glob("*.h"))
     blob = _embed_library()
     tasks = []
     objs = []

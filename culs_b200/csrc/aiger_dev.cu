@@ -24,12 +24,10 @@
 #include <atomic>
 #include <cstdio>
 #include <cstring>
-#include <exception>
-#include <mutex>
 #include <string>
-#include <thread>
 #include <vector>
 
+#include "host_runs.hpp"
 #include "kernels.cuh"
 #include "rw_work.cuh"
 
@@ -235,44 +233,16 @@ __global__ void k_gather_i64(int n, const int64_t *idx, const long long *src, lo
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) dst[k] = src[idx[k]];
 }
 
-// Graphs [0, G) in contiguous runs of about equal weight, each run on its own
-// host thread (the first on the caller's); `grain`: the weight that is worth a
-// thread (starting one costs about 15 us).
+// Runs fn(g0, g1) over graphs [0, G) in runs of about equal weight, each on a
+// host thread with `device` current; `grain`: the weight that is worth a
+// thread.  Returns the first error code.
 template <class W, class F>
-void for_runs(int G, int64_t grain, W weight, F fn) {
+int for_runs(int G, int device, int64_t grain, W weight, F fn) {
     int64_t total = 0;
     for (int g = 0; g < G; g++) total += weight(g);
-    const unsigned hw = std::thread::hardware_concurrency();
-    const int parts = (int)std::max<int64_t>(1, std::min({(int64_t)(hw ? hw : 1u), (int64_t)32, (int64_t)G, total / grain}));
-    std::vector<int> cut{0};
-    int64_t acc = 0;
-    for (int g = 0; g < G; g++) {
-        acc += weight(g);
-        if ((int)cut.size() < parts && acc * parts >= total * (int64_t)cut.size() && g + 1 < G) cut.push_back(g + 1);
-    }
-    cut.push_back(G);
-    // an exception of any run is rethrown here once every started thread has
-    // been joined
-    std::exception_ptr err;
-    std::mutex mu;
-    auto call = [&](size_t r) {
-        try {
-            fn(cut[r], cut[r + 1]);
-        } catch (...) {
-            std::lock_guard<std::mutex> lk(mu);
-            if (!err) err = std::current_exception();
-        }
-    };
-    std::vector<std::thread> th;
-    try {
-        for (size_t r = 1; r + 1 < cut.size(); r++) th.emplace_back(call, r);
-    } catch (...) {
-        for (auto &t : th) t.join();
-        throw;
-    }
-    call(0);
-    for (auto &t : th) t.join();
-    if (err) std::rethrow_exception(err);
+    const std::vector<int> cut = split_runs(G, host_threads(total, grain, G), weight);
+    return run_parallel((int)cut.size() - 1, [&] { return (int)cudaSetDevice(device); },
+                        [&](int r) { return fn(cut[r], cut[r + 1]); });
 }
 
 // Decimal digits of v >= 0 followed by '\n' at p; returns the end.
@@ -357,18 +327,22 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
     std::vector<size_t> text(count), body(count);
     std::vector<int> head(3 * (size_t)count);
     std::atomic<int> bad{-1};
+    int rc = 0;
     for (int g = 0; g < count && bad.load() < 0; g++)
         if (!data[g] || !parse_head(data[g], len[g], head[3 * g], head[3 * g + 1], head[3 * g + 2], text[g])) bad = g;
     if (bad.load() < 0)
-        for_runs(count, kLinesPerThread, [&](int g) { return (int64_t)head[3 * g + 1] + 1; }, [&](int g0, int g1) {
-            for (int g = g0; g < g1; g++)
-                if (!parse_outs(data[g], len[g], 1 + head[3 * g] + head[3 * g + 2], head[3 * g + 1], text[g], outs[g],
-                                body[g])) {
-                    int none = -1;
-                    bad.compare_exchange_strong(none, g);
-                    return;
-                }
-        });
+        rc = for_runs(count, device_, kLinesPerThread, [&](int g) { return (int64_t)head[3 * g + 1] + 1; },
+                      [&](int g0, int g1) {
+                          for (int g = g0; g < g1; g++)
+                              if (!parse_outs(data[g], len[g], 1 + head[3 * g] + head[3 * g + 2], head[3 * g + 1],
+                                              text[g], outs[g], body[g])) {
+                                  int none = -1;
+                                  bad.compare_exchange_strong(none, g);
+                                  return 0;
+                              }
+                          return 0;
+                      });
+    if ((rc = check((cudaError_t)rc, "upload"))) return rc;
     if (bad.load() >= 0) return fail(CULS_E_IO, "upload: not binary AIGER (graph " + std::to_string(bad.load()) + ")");
     for (int g = 0; g < count; g++) {
         const int nPIs = head[3 * g], nPOs = head[3 * g + 1], nAnds = head[3 * g + 2];
@@ -383,7 +357,6 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
     }
     regOff[count] = bytes;
     andBase[count] = nAnd;
-    int rc;
     // staging: the number sections, then the output literals
     if ((rc = ensure_stage((size_t)(bytes + 3) / 4 + (size_t)nPO + 1))) return rc;
     uint8_t *sB = reinterpret_cast<uint8_t *>(stage_);
@@ -405,17 +378,21 @@ int Engine::upload_aiger(Batch &b, int count, const uint8_t *const *data, const 
     cudaStream_t s = s_;
     ExecCtx X = ctx();
     // a run's copies follow its staging and overlap the other runs'
-    for_runs(count, kBytesPerThread, [&](int g) { return regOff[g + 1] - regOff[g] + 1; }, [&](int g0, int g1) {
+    StreamDrain drain{s};
+    rc = for_runs(count, device_, kBytesPerThread, [&](int g) { return regOff[g + 1] - regOff[g] + 1; }, [&](int g0, int g1) {
         for (int g = g0; g < g1; g++) {
             memcpy(sB + regOff[g], data[g] + body[g], len[g] - body[g]);
             if (!outs[g].empty()) memcpy(sPO + hg[g].poOff, outs[g].data(), sizeof(int32_t) * outs[g].size());
         }
         const int64_t p0 = hg[g0].poOff, p1 = g1 < count ? (int64_t)hg[g1].poOff : nPO;
+        cudaError_t e = cudaSuccess;
         if (regOff[g1] > regOff[g0])
-            cudaMemcpyAsync(dB + regOff[g0], sB + regOff[g0], (size_t)(regOff[g1] - regOff[g0]), cudaMemcpyHostToDevice, s);
-        if (p1 > p0) cudaMemcpyAsync(b.PO + p0, sPO + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyHostToDevice, s);
+            e = cudaMemcpyAsync(dB + regOff[g0], sB + regOff[g0], (size_t)(regOff[g1] - regOff[g0]), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess && p1 > p0)
+            e = cudaMemcpyAsync(b.PO + p0, sPO + p0, sizeof(int32_t) * (p1 - p0), cudaMemcpyHostToDevice, s);
+        return (int)e;
     });
-    if ((rc = check(cudaGetLastError(), "h2d"))) return rc;
+    if ((rc = check((cudaError_t)rc, "h2d"))) return rc;
     if ((rc = check(cudaMemcpyAsync(dReg, regOff.data(), sizeof(int64_t) * (count + 1), cudaMemcpyHostToDevice, s),
                     "h2d")))
         return rc;
@@ -526,6 +503,7 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
     if ((rc = sync())) return rc;
     // the numbers land while the output lines are measured (the sizes need
     // their lengths only)
+    StreamDrain drain{s};
     if (buf && total && (rc = check(cudaMemcpyAsync(sB, dB, (size_t)total, cudaMemcpyDeviceToHost, s), "d2h")))
         return rc;
     // file g = header, output lines, numbers, "c\n"; files back to back
@@ -536,20 +514,22 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
         const DevGraph &d = b.hg[g];
         headLen[g] = snprintf(hline, sizeof hline, "aig %d %d 0 %d %d\n", d.nPIs + d.nAnds, d.nPIs, d.nPOs, d.nAnds);
     }
-    for_runs(G, 4 * kLinesPerThread, [&](int g) { return (int64_t)b.hg[g].nPOs + 1; }, [&](int g0, int g1) {
+    rc = for_runs(G, device_, 4 * kLinesPerThread, [&](int g) { return (int64_t)b.hg[g].nPOs + 1; }, [&](int g0, int g1) {
         for (int g = g0; g < g1; g++) {
             int64_t t = 0;
             for (int o = 0; o < b.hg[g].nPOs; o++) t += line_len(aig_inv_const(sPO[b.hg[g].poOff + o]));
             textLen[g] = t;
         }
+        return 0;
     });
+    if ((rc = check((cudaError_t)rc, "download"))) return rc;
     offsets[0] = 0;
     for (int g = 0; g < G; g++)
         offsets[g + 1] = offsets[g] + (size_t)headLen[g] + (size_t)textLen[g] + (size_t)(hOff[g + 1] - hOff[g]) + 2;
     if (!buf) return 0;  // sizes only
     if ((rc = sync())) return rc;
     if (cap < offsets[G]) return fail(CULS_E_INVALID, "download: AIGER buffer too small");
-    for_runs(G, kBytesPerThread, [&](int g) { return (int64_t)(offsets[g + 1] - offsets[g]); }, [&](int g0, int g1) {
+    rc = for_runs(G, device_, kBytesPerThread, [&](int g) { return (int64_t)(offsets[g + 1] - offsets[g]); }, [&](int g0, int g1) {
         char line[96];
         for (int g = g0; g < g1; g++) {
             const DevGraph &d = b.hg[g];
@@ -563,8 +543,9 @@ int Engine::download_aiger(const Batch &b, uint8_t *buf, size_t cap, size_t *off
             *p++ = 'c';
             *p++ = '\n';
         }
+        return 0;
     });
-    return 0;
+    return check((cudaError_t)rc, "download");
 }
 
 }  // namespace culs

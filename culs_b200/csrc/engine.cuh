@@ -152,6 +152,13 @@ enum Mark : int {
     kNumMarks
 };
 
+// Waits for a stream where its scope ends, also by an error or an exception:
+// copies in flight use host memory that is reused or freed afterwards.
+struct StreamDrain {
+    cudaStream_t s;
+    ~StreamDrain() { cudaStreamSynchronize(s); }
+};
+
 class Engine {
   public:
     Engine();

@@ -6,65 +6,16 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
-#include <exception>
 #include <mutex>
-#include <thread>
 #include <vector>
 
 #include "engine.cuh"
+#include "host_runs.hpp"
 
 namespace culs {
 
-namespace {
-
-// Splits graphs [0, G) into at most `parts` contiguous runs of about equal
-// weight; returns the run starts (size runs + 1).
-std::vector<int> split_runs(const std::vector<DevGraph> &hg, int64_t total, int parts) {
-    std::vector<int> cut{0};
-    int64_t acc = 0;
-    const int G = (int)hg.size();
-    for (int g = 0; g < G; g++) {
-        acc += 1 + (int64_t)hg[g].nPIs + hg[g].nAnds;
-        if ((int)cut.size() < parts && acc * parts >= total * (int64_t)cut.size() && g + 1 < G) cut.push_back(g + 1);
-    }
-    cut.push_back(G);
-    return cut;
-}
-
-int host_threads(int64_t work, int G) {
-    if (work < (1 << 20) || G < 2) return 1;
-    const unsigned hw = std::thread::hardware_concurrency();
-    return (int)std::max(1u, std::min({hw ? hw : 1u, 32u, (unsigned)G}));
-}
-
-// Runs fn(run) for every run on its own thread (the first on the caller's).
-// An exception of any run is rethrown on the caller's thread once every
-// started thread has been joined.
-template <class F>
-void run_parallel(int runs, F fn) {
-    std::exception_ptr err;
-    std::mutex mu;
-    auto call = [&](int r) {
-        try {
-            fn(r);
-        } catch (...) {
-            std::lock_guard<std::mutex> lk(mu);
-            if (!err) err = std::current_exception();
-        }
-    };
-    std::vector<std::thread> th;
-    try {
-        for (int r = 1; r < runs; r++) th.emplace_back(call, r);
-    } catch (...) {
-        for (auto &t : th) t.join();
-        throw;
-    }
-    call(0);
-    for (auto &t : th) t.join();
-    if (err) std::rethrow_exception(err);
-}
-
-}  // namespace
+// A transfer of fewer than a million objects stays on the caller's thread.
+static int transfer_threads(int64_t nObj, int G) { return nObj < (1 << 20) ? 1 : host_threads(nObj, 1, G); }
 
 int Engine::prepare(int64_t nObj) {
     int rc = ensure_arena((size_t)nObj * 640 + ((size_t)256 << 20));
@@ -107,11 +58,13 @@ int Engine::upload(Batch &b, int count, const int32_t *const *f0, const int32_t 
     if (!b.pool) b.pool = pool_;
     if ((rc = check(b.reserve(nObj, nPO, count), "cudaMalloc"))) return rc;
     int32_t *sF0 = stage_, *sF1 = stage_ + nObj, *sPO = stage_ + 2 * nObj;
-    const std::vector<int> runs = split_runs(hg, nObj, host_threads(nObj, count));
+    auto size = [&](int g) { return 1 + (int64_t)nPIs[g] + nAnds[g]; };
+    const std::vector<int> runs = split_runs(count, transfer_threads(nObj, count), size);
     std::atomic<int> bad{0};
     std::mutex mu;
     std::string why;
-    auto work = [&](int r) {
+    StreamDrain drain{s_};  // copies in flight read the staging buffer
+    auto work = [&](int r) -> int {
         std::vector<int> d;
         for (int g = runs[r]; g < runs[r + 1] && !bad.load(std::memory_order_relaxed); g++) {
             const int n = 1 + nPIs[g] + nAnds[g];
@@ -124,7 +77,7 @@ int Engine::upload(Batch &b, int count, const int32_t *const *f0, const int32_t 
                 if (a < 0 || c < 0 || (a >> 1) >= i || (c >> 1) >= i) {
                     std::lock_guard<std::mutex> lk(mu);
                     if (!bad.exchange(1)) why = "upload: fanin literal out of range or not topological";
-                    return;
+                    return 0;
                 }
                 sF0[base + i] = a;
                 sF1[base + i] = c;
@@ -137,7 +90,7 @@ int Engine::upload(Batch &b, int count, const int32_t *const *f0, const int32_t 
                 if (o < 0 || (o >> 1) >= n) {
                     std::lock_guard<std::mutex> lk(mu);
                     if (!bad.exchange(1)) why = "upload: PO literal out of range";
-                    return;
+                    return 0;
                 }
                 sPO[hg[g].poOff + k] = o;
             }
@@ -147,16 +100,18 @@ int Engine::upload(Batch &b, int count, const int32_t *const *f0, const int32_t 
         const DevGraph &a = hg[runs[r]], &z = hg[runs[r + 1] - 1];
         const int64_t o0 = a.base, o1 = (int64_t)z.base + 1 + z.nPIs + z.nAnds;
         const int64_t p0 = a.poOff, p1 = (int64_t)z.poOff + z.nPOs;
-        cudaMemcpyAsync(b.F0 + o0, sF0 + o0, sizeof(int) * (o1 - o0), cudaMemcpyHostToDevice, s_);
-        cudaMemcpyAsync(b.F1 + o0, sF1 + o0, sizeof(int) * (o1 - o0), cudaMemcpyHostToDevice, s_);
-        if (p1 > p0) cudaMemcpyAsync(b.PO + p0, sPO + p0, sizeof(int) * (p1 - p0), cudaMemcpyHostToDevice, s_);
+        cudaError_t e = cudaMemcpyAsync(b.F0 + o0, sF0 + o0, sizeof(int) * (o1 - o0), cudaMemcpyHostToDevice, s_);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(b.F1 + o0, sF1 + o0, sizeof(int) * (o1 - o0), cudaMemcpyHostToDevice, s_);
+        if (e == cudaSuccess && p1 > p0)
+            e = cudaMemcpyAsync(b.PO + p0, sPO + p0, sizeof(int) * (p1 - p0), cudaMemcpyHostToDevice, s_);
+        return (int)e;
     };
-    run_parallel((int)runs.size() - 1, work);
-    if (bad.load()) {
-        sync();  // copies already issued read the staging buffer
-        return fail(CULS_E_INVALID, why);
-    }
-    cudaMemcpyAsync(b.dg, hg.data(), sizeof(DevGraph) * count, cudaMemcpyHostToDevice, s_);
+    const int copied = run_parallel((int)runs.size() - 1, [&] { return (int)cudaSetDevice(device_); }, work);
+    if (bad.load()) return fail(CULS_E_INVALID, why);
+    if ((rc = check((cudaError_t)copied, "h2d"))) return rc;
+    if ((rc = check(cudaMemcpyAsync(b.dg, hg.data(), sizeof(DevGraph) * count, cudaMemcpyHostToDevice, s_), "h2d")))
+        return rc;
     b.G = count;
     b.nObj = nObj;
     b.nPO = nPO;
@@ -170,7 +125,8 @@ int Engine::download_all(const Batch &b, int32_t *const *f0, int32_t *const *f1,
     int rc;
     if ((rc = ensure_stage((size_t)2 * b.nObj + b.nPO))) return rc;
     int32_t *sF0 = stage_, *sF1 = stage_ + b.nObj, *sPO = stage_ + 2 * b.nObj;
-    const std::vector<int> runs = split_runs(b.hg, b.nObj, host_threads(b.nObj, b.G));
+    auto size = [&](int g) { return 1 + (int64_t)b.hg[g].nPIs + b.hg[g].nAnds; };
+    const std::vector<int> runs = split_runs(b.G, transfer_threads(b.nObj, b.G), size);
     const int nr = (int)runs.size() - 1;
     // one event per run: a thread scatters its run as soon as it has landed
     std::vector<cudaEvent_t> ev(nr, nullptr);
@@ -193,12 +149,8 @@ int Engine::download_all(const Batch &b, int32_t *const *f0, int32_t *const *f1,
             if (e) cudaEventDestroy(e);
         return rc;
     }
-    std::atomic<int> bad{0};
-    run_parallel(nr, [&](int r) {
-        if (cudaEventSynchronize(ev[r]) != cudaSuccess) {
-            bad.store(1);
-            return;
-        }
+    const int landed = run_parallel(nr, [&] { return (int)cudaSetDevice(device_); }, [&](int r) -> int {
+        if (const cudaError_t e = cudaEventSynchronize(ev[r])) return (int)e;
         for (int g = runs[r]; g < runs[r + 1]; g++) {
             const DevGraph &d = b.hg[g];
             const size_t n = 1 + (size_t)d.nPIs + d.nAnds;
@@ -206,10 +158,10 @@ int Engine::download_all(const Batch &b, int32_t *const *f0, int32_t *const *f1,
             if (f1 && f1[g]) memcpy(f1[g], sF1 + d.base, sizeof(int32_t) * n);
             if (outs && outs[g] && d.nPOs) memcpy(outs[g], sPO + d.poOff, sizeof(int32_t) * d.nPOs);
         }
+        return 0;
     });
     for (cudaEvent_t e : ev) cudaEventDestroy(e);
-    if (bad.load()) return check(cudaErrorUnknown, "d2h");
-    return 0;
+    return check((cudaError_t)landed, "d2h");
 }
 
 }  // namespace culs
