@@ -803,7 +803,7 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
     uint32_t *keys = reinterpret_cast<uint32_t *>(A.lists[0]), *keys2 = reinterpret_cast<uint32_t *>(A.lists[1]);
     if (!flags || !ids || !sorted) return fail(CULS_E_OOM, "balance: arena exhausted");
     k_bal_cover_flags<<<grid_1d(nObj, kBlock, sms_ * 8), kBlock, 0, s>>>(nObj, A.covLen, flags);
-    check(compact_flags(flags, nObj, ids, counters_, ar_, s), "compact");
+    if (int e = check(compact_flags(flags, nObj, ids, counters_, ar_, s), "compact")) return e;
     std::vector<int> hc((size_t)G * kBcSize);
     check(cudaMemcpyAsync(hc.data(), A.cnt, sizeof(int) * (size_t)G * kBcSize, cudaMemcpyDeviceToHost, s), "d2h");
     if ((rc = fetch("balance covers"))) return rc;
@@ -831,7 +831,7 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
                                                                             lvCnt, lvMax);
         if ((rc = check(radix_sort_pairs(keys, ids, keys2, sorted, nCov, bits_for(nLv), ar_, s), "sort"))) return rc;
     }
-    check(scan_exclusive(lvCnt, lvStart, nLv, nullptr, ar_, s), "scan");
+    if (int e = check(scan_exclusive(lvCnt, lvStart, nLv, nullptr, ar_, s), "scan")) return e;
     A.sorted = sorted, A.lvCnt = lvCnt, A.lvMax = lvMax, A.lvStart = lvStart;
     k_bal_init_tables<<<grid_1d(nTab, kBlock, sms_ * 16), kBlock, 0, s>>>(nTab, A);
     if ((rc = check(launch_team(k_bal_rebuild<BlockTeam>, k_bal_rebuild<ClusterTeam>, k_bal_rebuild<GridTeam>, A, W, s),
@@ -862,7 +862,7 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
     if (nB > 0) {
         const unsigned gs = grid_1d(nB, kBlock, sms_ * 8);
         k_bal_used<<<grid_1d(nTab, kBlock, sms_ * 16), kBlock, 0, s>>>(nTab, A.tab, used);
-        check(compact_flags(used, nTab, slots, counters_, ar_, s), "compact");
+        if (int e = check(compact_flags(used, nTab, slots, counters_, ar_, s), "compact")) return e;
         k_bal_ids<<<gs, kBlock, 0, s>>>(nB, slots, A.tab, bk);
         if ((rc = check(radix_sort_pairs(bk, slots, bk2, slots2, nB, bits_for((int64_t)maxId + 1), ar_, s), "sort")))
             return rc;

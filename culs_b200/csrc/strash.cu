@@ -776,7 +776,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         k_dead_seed_flags<<<gridM, kBlock, 0, s>>>(M, L0, cnt, flags);
         check(fill_i32(items, -1, M + 1, s), "fill");
         check(cudaMemsetAsync(qc, 0, sizeof(int) * 8, s), "memset");
-        check(compact_flags(flags, M, items, qc + 1, ar_, s), "compact");
+        if (int e = check(compact_flags(flags, M, items, qc + 1, ar_, s), "compact")) return e;
         k_dead_queue<<<gridQ, kBlock, 0, s>>>(WorkQueue{items, qc + 0, qc + 1, qc + 2, (int)(M + 1)}, L0, L1, cnt,
                                               dead, status_);
         launches_ += 4;
@@ -796,7 +796,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         check(cudaMemsetAsync(graphLevels, 0, sizeof(int) * (G + 1), s), "memset");
         check(cudaMemsetAsync(level, 0, sizeof(int) * (M + 1), s), "memset");
         k_live_flags<<<gridM, kBlock, 0, s>>>(M, L0, dead, liveFlag, done);
-        check(compact_flags(liveFlag, M, liveIdx, qc + 3, ar_, s), "compact");  // live list and count
+        if (int e = check(compact_flags(liveFlag, M, liveIdx, qc + 3, ar_, s), "compact")) return e;  // live list and count
         if (prof_) this->mark(kMkLevelK0);
         if (inBlock) {
             LevelsArgs A;
@@ -826,7 +826,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         check(cudaMemsetAsync(graphLevels, 0, sizeof(int) * (G + 1), s), "memset");
         check(cudaMemsetAsync(level, 0, sizeof(int) * (M + 1), s), "memset");
         k_live_flags<<<gridM, kBlock, 0, s>>>(M, L0, dead, liveFlag, done);
-        check(compact_flags(liveFlag, M, liveIdx, qc + 3, ar_, s), "compact");  // live list and count
+        if (int e = check(compact_flags(liveFlag, M, liveIdx, qc + 3, ar_, s), "compact")) return e;  // live list and count
         launches_ += 1;
         if (prof_) this->mark(kMkLevelK0);
         const int *list = procInv;
@@ -837,7 +837,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
             LevelsArgs A;
             A.n = M, A.a0 = a0, A.a1 = a1, A.posOf = procInv, A.level = level;
             A.depth0 = qc + 4, A.depth1 = graphLevels, A.unsettled = qc + 6, A.status = qc + 7;
-            check(levels_block(A, s), "levels");
+            if (int e = check(levels_block(A, s), "levels")) return e;
             launches_ += 2;
             if (int e = fetch("strash levels")) return e;
             leveled = hostSmall_[6] == 0 && hostSmall_[7] == 0;
@@ -848,7 +848,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
                                                       graphLevels, qc + 5, qc + 4, qc + 7);
             k_unresolved_flags<<<grid_1d(n, kBlock, sms_ * 16), kBlock, 0, s>>>(n, list, done, flags);
             launches_ += 2;
-            check(compact_flags(flags, n, idx, qc + 6, ar_, s), "compact");
+            if (int e = check(compact_flags(flags, n, idx, qc + 6, ar_, s), "compact")) return e;
             if (int e = fetch("strash levels")) return e;
             const int64_t nu = hostSmall_[6];
             if (hostSmall_[7] != 0) break;  // a wait timed out
@@ -868,7 +868,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     if (!leveled) {
     check(cudaMemsetAsync(off, 0, sizeof(int) * (M + 2), s), "memset");
     k_live_degrees<<<gridM, kBlock, 0, s>>>(M, L0, L1, dead, level, off, liveFlag, flags);
-    check(scan_exclusive(off, off, M + 1, nullptr, ar_, s), "scan");
+    if (int e = check(scan_exclusive(off, off, M + 1, nullptr, ar_, s), "scan")) return e;
     int *cursor = cnt;  // reuse
     check(cudaMemcpyAsync(cursor, off, sizeof(int) * (M + 1), cudaMemcpyDeviceToDevice, s), "copy");
     // number of live edges = off[M]
@@ -884,8 +884,8 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     check(cudaMemsetAsync(qc, 0, sizeof(int) * 8, s), "memset");
     check(cudaMemsetAsync(ring, 0, sizeof(int) * 8, s), "memset");
     check(cudaMemsetAsync(graphLevels, 0, sizeof(int) * (G + 1), s), "memset");
-    check(compact_flags(flags, M, items, ring + 1, ar_, s), "compact");     // level 1: the seeds
-    check(compact_flags(liveFlag, M, liveIdx, qc + 3, ar_, s), "compact");  // live list and count
+    if (int e = check(compact_flags(flags, M, items, ring + 1, ar_, s), "compact")) return e;     // level 1: the seeds
+    if (int e = check(compact_flags(liveFlag, M, liveIdx, qc + 3, ar_, s), "compact")) return e;  // live list and count
     launches_ += 2;
     if (prof_) this->mark(kMkLevelK0);
     // levels in launches of 64, until a level comes out empty; the ring
@@ -933,7 +933,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         int bits = 1;
         while ((1ll << bits) <= maxLevel) bits++;
         check(cudaMemcpyAsync(vals2, liveIdx, sizeof(int) * nLive, cudaMemcpyDeviceToDevice, s), "copy");
-        check(radix_sort_pairs(keys, vals2, keys2, srt, nLive, bits, ar_, s), "sort");
+        if (int e = check(radix_sort_pairs(keys, vals2, keys2, srt, nLive, bits, ar_, s), "sort")) return e;
         k_inverse<<<gl, kBlock, 0, s>>>(nLive, srt, tOf);
         // tentative rank: processing order, or id order for the CPU variants
         k_inverse<<<gl, kBlock, 0, s>>>(nLive, idOrder ? liveIdx : srt, rankOf);
@@ -1029,8 +1029,8 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         check(cudaMemsetAsync(lvlDone, 0, sizeof(int) * (maxLevel + 2), s), "memset");
         check(cudaMemsetAsync(qc + 5, 0, sizeof(int), s), "memset");
         k_level_chunks<<<grid_1d(maxLevel + 1, kBlock, sms_ * 16), kBlock, 0, s>>>(maxLevel + 1, lvlCnt, chunkCnt);
-        check(scan_exclusive(lvlCnt, lvlStart, maxLevel + 1, nullptr, ar_, s), "scan");
-        check(scan_exclusive(chunkCnt, chunkStart, maxLevel + 1, chunkStart + maxLevel + 1, ar_, s), "scan");
+        if (int e = check(scan_exclusive(lvlCnt, lvlStart, maxLevel + 1, nullptr, ar_, s), "scan")) return e;
+        if (int e = check(scan_exclusive(chunkCnt, chunkStart, maxLevel + 1, chunkStart + maxLevel + 1, ar_, s), "scan")) return e;
         launches_ += 1;
         check(and_table_clear(ts, cap, s), "fill");
         DedupArgs A{nLive,      srt,      rankOf,
@@ -1048,7 +1048,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         k_winner_flags<<<grid_1d(nLive, kBlock, sms_ * 16), kBlock, 0, s>>>(nLive, srt, rankOf, idOrder, slotT, ts, wflags);
         launches_ += 1;
     }
-    check(compact_flags(wflags, nLive, wl, qc + 6, ar_, s), "compact");
+    if (int e = check(compact_flags(wflags, nLive, wl, qc + 6, ar_, s), "compact")) return e;
     // In id order (CPU variants) the winners are ranked by position, not by
     // processing order: sort the winner list by rank.
     if (int e = fetch("strash hashing")) return e;
@@ -1067,7 +1067,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         while ((1ll << bits) <= nLive) bits++;
         k_gather_rank<<<grid_1d(nW, kBlock, sms_ * 16), kBlock, 0, s>>>(nW, wl, srt, rankOf, wk);
         check(cudaMemcpyAsync(wv, wl, sizeof(int) * nW, cudaMemcpyDeviceToDevice, s), "copy");
-        check(radix_sort_pairs(wk, wv, wk2, wl, nW, bits, ar_, s), "sort");
+        if (int e = check(radix_sort_pairs(wk, wv, wk2, wl, nW, bits, ar_, s), "sort")) return e;
         launches_ += 1;
     }
     std::vector<int> hCnt(G), hLev(G);
@@ -1085,9 +1085,9 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
             int bits = 1;
             while ((1ll << bits) < G) bits++;
             check(cudaMemcpyAsync(wv, wl, sizeof(int) * nW, cudaMemcpyDeviceToDevice, s), "copy");
-            check(radix_sort_pairs(wk, wv, wk2, wlByG, nW, bits, ar_, s), "sort");
+            if (int e = check(radix_sort_pairs(wk, wv, wk2, wlByG, nW, bits, ar_, s), "sort")) return e;
         }
-        check(scan_exclusive(cntG, gStart, G, nullptr, ar_, s), "scan");
+        if (int e = check(scan_exclusive(cntG, gStart, G, nullptr, ar_, s), "scan")) return e;
         check(cudaMemcpyAsync(hCnt.data(), cntG, sizeof(int) * G, cudaMemcpyDeviceToHost, s), "d2h");
         check(cudaMemcpyAsync(hLev.data(), graphLevels, sizeof(int) * G, cudaMemcpyDeviceToHost, s), "d2h");
         if (int e = sync()) return e;
