@@ -640,11 +640,12 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w) {
     int64_t stackCap = (int64_t)w.maxLevel + 64;
     stackCap = std::min<int64_t>(2 * stackCap + w.nNew / std::max(G, 1) + 64, 1 << 20);
     int4 *stack = ar.get<int4>((size_t)stackCap * G);
-    // the records and marks take the place of the enumeration's cut
-    // attributes (64 bytes per original node), which nothing reads any more
+    // the records and marks take the place of the enumeration's cuts, 256
+    // bytes per original node, which are not read any more once the
+    // candidates' records are made
     int4 *rec, *mark;
-    if (32 * M <= 64 * w.N) {
-        rec = reinterpret_cast<int4 *>(w.cutA);
+    if (32 * M <= 256 * w.N) {
+        rec = w.cutL;
         mark = rec + M;
     } else {
         rec = ar.get<int4>(M);

@@ -365,9 +365,7 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
     Arena &ar = *X.ar;
     int rc;
     w.repW = ar.get<int>(nCand + 1);
-    w.withRep = ar.get<int>(nCand + 1);
-    uint8_t *hasRep = ar.get<uint8_t>(nCand + 1);
-    if (!w.repW || !w.withRep || !hasRep) return X.fail(CULS_E_OOM, "rw: arena exhausted (replace)");
+    if (!w.repW) return X.fail(CULS_E_OOM, "rw: arena exhausted (replace)");
     if (nCand == 0) return rep_extend_only(X, w, 0);
     int *kcnt = ar.get<int>(nCand + 1), *koff = ar.get<int>(nCand + 1), *rootRef = ar.get<int>(nCand + 1);
     int *repT = ar.get<int>(nCand + 1);
@@ -422,14 +420,26 @@ int rw_replace(ExecCtx &X, Batch &b, RwWork &w) {
     k_rep_rebuild<<<X.grid(nCand, 64), 64, 0, s>>>(nCand, N, rootRef, canon, f0, f1, owner, nullptr, kpo, newPos,
                                                      X.status);
     X.launched(1);
-    // the new nodes' number is read with the last fetch: their arrays get
-    // room for all K, of which they are the first nNew
-    if ((rc = rep_extend_only(X, w, K))) return rc;
-    w.newOwnLev = ar.get<int>(K + 1);
+    // Where the records are few, the new nodes' arrays get room for all K of
+    // them, and the new nodes' number (they are the first nNew) is read with
+    // the last fetch: a host wait less.  That room is 21 bytes a record, which
+    // is 2.6 of the arena's 640 bytes a node at K = N / 8, or 22 of its spare
+    // 256 MB at a million.  A graph with many duplicates has most of its
+    // records merged, and needs its scratch for the deduplication to come:
+    // there the number is read first.
+    int64_t room = K;
+    if (K > std::max<int64_t>(1 << 20, N / 8)) {
+        if ((rc = X.fetch("rw replace"))) return rc;
+        room = X.hostSmall[18];
+    }
+    if ((rc = rep_extend_only(X, w, room))) return rc;
+    w.newOwnLev = ar.get<int>(room + 1);
     if (!w.newOwnLev) return X.fail(CULS_E_OOM, "rw: arena exhausted (replace)");
     if (K > 0)
         k_rep_newnodes<<<X.grid(K), kBlock, 0, s>>>(K, N, canon, f0, f1, c0, c1, newPos, owner, w.cand, w.wg, w.wlev,
                                                     w.L0, w.L1, w.gidAll, w.newOwnLev);
+    w.withRep = kp;  // kp and koff are not read any more
+    uint8_t *hasRep = reinterpret_cast<uint8_t *>(koff);
     k_rep_final<<<X.grid(nCand), kBlock, 0, s>>>(nCand, N, repT, newPos, w.repW, hasRep);
     X.launched(2);
     if ((rc = X.check(compact_flags(hasRep, nCand, w.withRep, cnt + 3, ar, s), "compact"))) return rc;
