@@ -15,9 +15,9 @@
 // covers from a PO, is the round in which the last cover above it was taken,
 // counting down those counts.  (The reference rebuilds a frontier of all
 // covers at each distance by a copy_if over all nodes, so a cover is visited
-// at every level it appears on.)  A DFS keeps up to 32 leaves in local
-// memory; a larger cover (up to 1,024 leaves) is redone by the team's first
-// threads, each with a leaf buffer in global memory.
+// at every level it appears on.)  A thread's DFS keeps up to 32 leaves in
+// local memory; a larger cover (up to 1,024 leaves) is redone by a warp, which
+// looks a literal up among the leaves 32 at a time.
 //
 // Phase 2, reconstruction (k_bal_rebuild).  Covers are taken deepest level
 // first, in increasing node id, in chunks of 32,768 (the reference's
@@ -63,7 +63,7 @@ constexpr int kBalStack = 128;      // DFS_COVER_STACK_SIZE, balance.cu:18
 constexpr int kBalChunk = 32768;    // iterLen, balance.cu:1125
 constexpr int kBalLocal = 32;       // leaves a DFS keeps in local memory
 constexpr int kBalThreads = 512;    // threads of a team's block
-constexpr int kBalBig = 128;        // threads of a team with a 1,024-leaf buffer for the large covers
+constexpr int kBalWarps = kBalThreads / 32;  // of a block, each with a 1,024-leaf buffer for large covers
 constexpr int kBalMaxCluster = 8;   // the portable cluster size
 constexpr unsigned kNoId = 0xFFFFFFFFu;
 constexpr int kNoEpoch = INT_MAX;
@@ -115,13 +115,14 @@ struct BalArgs {
     int *found, *lists[2], *big;
     int2 *newLit;  // a cover's new {literal, level}
     int *flat;     // every collected cover's leaves
-    int *scratch;  // per team: kBalBig leaf buffers
+    int *scratch;  // per warp of the grid: a leaf buffer
     // per cover in processing order: (graph, last level, node id)
     const int *sorted;
     const int *lvCnt, *lvMax, *lvStart;
     int *len, *mask, *val;
     int2 *work;  // {literal, level} arrays, longest level first, at the cover's leaves' offset
     BalSlot *tab;
+    int spread;  // the reconstruction deals covers by Team::spread
     int *status;
 };
 
@@ -132,11 +133,15 @@ __device__ __forceinline__ BalView bal_view(const BalArgs &A, const BalGraph &g)
 // ------------------------------------------------------------------ teams
 // The threads that work on one graph together.  ld reads a word that another
 // thread of the team may have written: through L1 inside a block, past it
-// where the team spans several SMs.  counters: where the graph's counters
-// are kept while the team works on it.
+// where the team spans several SMs.  spread: a rank that deals consecutive
+// covers to different SMs of a cluster, so that the arrays of long covers share
+// an L1 with as few others as possible (short ones are read together, and
+// dealt by rank: 60,000 ANDs in 60 layers 4.16 ms, 4.44 by spread).  counters:
+// where the graph's counters are kept while the team works on it.
 struct BlockTeam {
     __device__ static int threads() { return blockDim.x; }
     __device__ static int rank() { return threadIdx.x; }
+    __device__ static int spread() { return rank(); }
     __device__ static int index() { return blockIdx.x; }
     __device__ static int count() { return gridDim.x; }
     __device__ static void sync() { __syncthreads(); }
@@ -151,6 +156,9 @@ struct BlockTeam {
 struct ClusterTeam {
     __device__ static int threads() { return (int)cg::this_cluster().num_threads(); }
     __device__ static int rank() { return (int)cg::this_cluster().thread_rank(); }
+    __device__ static int spread() {
+        return (int)(threadIdx.x * cg::this_cluster().num_blocks() + cg::this_cluster().block_rank());
+    }
     __device__ static int index() { return blockIdx.x / (int)cg::this_cluster().num_blocks(); }
     __device__ static int count() { return gridDim.x / (int)cg::this_cluster().num_blocks(); }
     __device__ static void sync() { cg::this_cluster().sync(); }
@@ -162,6 +170,7 @@ struct ClusterTeam {
 struct GridTeam {
     __device__ static int threads() { return gridDim.x * blockDim.x; }
     __device__ static int rank() { return blockIdx.x * blockDim.x + threadIdx.x; }
+    __device__ static int spread() { return rank(); }
     __device__ static int index() { return 0; }
     __device__ static int count() { return 1; }
     __device__ static void sync() { cg::this_grid().sync(); }
@@ -221,6 +230,47 @@ __device__ int bal_cover_dfs(const BalView &V, const int *nfo, int v, int *leave
     return n;
 }
 
+// The same DFS by a whole warp, with room for every leaf (the DFS stops at
+// 1,024): all lanes hold the walk's state, the stack lies in shared memory and
+// the leaves, in global memory, are compared 32 at a time.  A thread a large
+// cover, as in bal_cover_dfs, takes 4 ms for 190 leaves, a warp 0.1.
+template <class Team>
+__device__ int bal_cover_dfs_warp(const BalView &V, const int *nfo, int v, int *stk, int *leaves) {
+    const unsigned F = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    int top = 0, n = 0, cur = 2 * v;  // cur: the literal popped, with `top` left on the stack
+    while (true) {
+        // read at once what the literal's node may need
+        const int id = lit_id_(cur), f0 = V.F0[id], f1 = V.F1[id], fanouts = Team::ld(&nfo[id]);
+        bool same = false, other = false;
+        for (int j = lane; j < n; j += 32) {
+            const int x = leaves[j];
+            same |= x == cur;
+            other |= x == (cur ^ 1);
+        }
+        if (__any_sync(F, other)) return -1;
+        if (!__any_sync(F, same)) {
+            if (cur != 2 * v && ((cur & 1) || id <= V.nPIs || fanouts > 1 || top + 1 >= kBalStack ||
+                                 n + 2 * top + 1 >= kBalMaxCover)) {
+                if (n == kBalMaxCover) return -2;
+                if (lane == 0) leaves[n] = cur;
+                n++;
+                __syncwarp();
+            } else {
+                // fanin 1 waits on the stack, fanin 0 is next
+                cur = f0;
+                if (lane == 0) stk[top] = f1;
+                top++;
+                __syncwarp();
+                continue;
+            }
+        }
+        if (top == 0) return n;
+        cur = stk[--top];
+        __syncwarp();  // read before the place is written again
+    }
+}
+
 // Appends v to a list, one atomic per converged group of lanes.
 __device__ __forceinline__ void bal_append(int *list, int *cnt, int v) {
     const unsigned m = __activemask();
@@ -231,30 +281,37 @@ __device__ __forceinline__ void bal_append(int *list, int *cnt, int v) {
     list[at + __popc(m & ((1u << lane) - 1u))] = v;
 }
 
-// Stores v's cover of n leaves (0: constant false), counts it at its AND
-// leaves and lists the leaves found for the first time.
-__device__ __forceinline__ void bal_store_cover(const BalArgs &A, const BalGraph &g, int *c, int v, const int *leaves,
-                                                int n) {
-    int off = 0;
-    if (n > 0) {
-        off = atomicAdd(&c[kBcCursor], n);
-        if (n > g.flatCap - off) {
-            set_status(A.status, kDevCapacity);
-            n = 0;
-        }
+// Room for a cover's n leaves: its place among the graph's, n = 0 when there
+// is none.
+__device__ __forceinline__ int bal_take_leaves(const BalArgs &A, const BalGraph &g, int *c, int &n) {
+    const int off = n > 0 ? atomicAdd(&c[kBcCursor], n) : 0;
+    if (n > g.flatCap - off) {
+        set_status(A.status, kDevCapacity);
+        n = 0;
     }
-    for (int j = 0; j < n; j++) {
+    return off;
+}
+
+// Stores leaves first, first + step, ... of v's cover of n leaves (0: constant
+// false) at place off, counts the cover at its AND leaves and lists the leaves
+// found for the first time.
+__device__ __forceinline__ void bal_store_cover(const BalArgs &A, const BalGraph &g, int *c, int v, const int *leaves,
+                                                int n, int off, int first, int step) {
+    for (int j = first; j < n; j += step) {
         A.flat[(int64_t)g.flatOff + off + j] = leaves[j];
         const int x = lit_id_(leaves[j]);
         if (x > g.nPIs && atomicAdd(&A.pend[g.obj + x], 1) == 0 && !__ldcg(&A.drives[g.obj + x]))
             bal_append(A.found + g.obj, &c[kBcFound], x);
     }
-    A.covOff[g.obj + v] = g.flatOff + off;
-    A.covLen[g.obj + v] = n;
+    if (first == 0) {
+        A.covOff[g.obj + v] = g.flatOff + off;
+        A.covLen[g.obj + v] = n;
+    }
 }
 
 template <class Team>
 __global__ void __launch_bounds__(kBalThreads) k_bal_covers(BalArgs A) {
+    __shared__ int s_stk[kBalWarps][kBalStack];
     const int T = Team::threads(), r = Team::rank();
     for (int gi = Team::index(); gi < A.G; gi += Team::count()) {
         const BalGraph g = A.g[A.order[gi]];
@@ -281,22 +338,30 @@ __global__ void __launch_bounds__(kBalThreads) k_bal_covers(BalArgs A) {
                 const int v = Team::ld(&found[i]);
                 int leaves[kBalLocal];
                 const int len = bal_cover_dfs<Team>(V, nfo, v, leaves, kBalLocal);
-                if (len == -2)
+                if (len == -2) {
                     bal_append(big, &c[kBcBig], v);
-                else
-                    bal_store_cover(A, g, c, v, leaves, len < 0 ? 0 : len);
+                } else {
+                    int n = max(len, 0);
+                    const int off = bal_take_leaves(A, g, c, n);
+                    bal_store_cover(A, g, c, v, leaves, n, off, 0, 1);
+                }
             }
             Team::sync();
             const int nBig = Team::ld(&c[kBcBig]);
             if (nBig > 0) {
-                if (r < kBalBig) {
-                    int *leaves = A.scratch + ((int64_t)Team::index() * kBalBig + r) * kBalMaxCover;
-                    for (int i = r; i < nBig; i += kBalBig) {
-                        const int v = Team::ld(&big[i]);
-                        const int len = bal_cover_dfs<Team>(V, nfo, v, leaves, kBalMaxCover);
-                        if (len == -2) set_status(A.status, kDevCapacity);  // cannot happen: the DFS stops at 1,024 leaves
-                        bal_store_cover(A, g, c, v, leaves, len < 0 ? 0 : len);
-                    }
+                const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+                int *leaves = A.scratch + ((int64_t)blockIdx.x * kBalWarps + warp) * kBalMaxCover;
+                for (int i = r >> 5; i < nBig; i += T >> 5) {
+                    const int v = Team::ld(&big[i]);
+                    int n = bal_cover_dfs_warp<Team>(V, nfo, v, s_stk[warp], leaves);
+                    if (n == -2) set_status(A.status, kDevCapacity);  // cannot happen: the DFS stops at 1,024 leaves
+                    n = max(n, 0);
+                    int off = 0;
+                    if (lane == 0) off = bal_take_leaves(A, g, c, n);
+                    n = __shfl_sync(0xffffffffu, n, 0);
+                    off = __shfl_sync(0xffffffffu, off, 0);
+                    bal_store_cover(A, g, c, v, leaves, n, off, lane, 32);
+                    __syncwarp();  // the leaves are read before the next cover's
                 }
                 Team::sync();
                 if (r == 0) c[kBcBig] = 0;
@@ -561,7 +626,7 @@ __device__ __forceinline__ void bal_step2(const BalChunk &C, const BalTable &T, 
 
 template <class Team>
 __global__ void __launch_bounds__(kBalThreads) k_bal_rebuild(BalArgs A) {
-    const int T = Team::threads(), r = Team::rank();
+    const int T = Team::threads(), r = A.spread ? Team::spread() : Team::rank();
     for (int gi = Team::index(); gi < A.G; gi += Team::count()) {
         const BalGraph g = A.g[A.order[gi]];
         int *const c = bal_open<Team>(A.cnt + (int64_t)A.order[gi] * kBcSize);
@@ -701,6 +766,15 @@ struct BalTeams {
     bool grid;
     int sms;
 };
+// As many blocks a graph as its widest level wants threads, while every graph
+// can have its team at once; a single graph wider than the largest cluster
+// gets the whole grid, whose barrier costs several times a cluster's.
+BalTeams bal_teams(int G, int64_t width, int sms) {
+    int cluster = 1;
+    while (cluster < kBalMaxCluster && cluster * kBalThreads < width && 2 * cluster * G <= sms) cluster *= 2;
+    const bool grid = G == 1 && width > kBalMaxCluster * kBalThreads;
+    return BalTeams{cluster, grid ? 1 : std::min(G, std::max(1, 2 * sms / cluster)), grid, sms};
+}
 // Runs one phase, given as its three forms.
 template <class K>
 cudaError_t launch_team(K block, K cluster, K all, const BalArgs &A, const BalTeams &W, cudaStream_t s) {
@@ -752,16 +826,9 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
         bytes += bal_bytes(d);
         width = std::max(width, d.nAnds / std::max(d.nLevels, 1));
     }
-    // Teams: as many blocks a graph as its levels are wide (one thread per
-    // frontier node or cover), while every graph can have its team at once;
-    // a single graph wider than the largest cluster gets the whole grid,
-    // whose barrier costs several times a cluster's.
-    int cluster = 1;
-    while (cluster < kBalMaxCluster && cluster * kBalThreads < width && 2 * cluster * G <= sms_) cluster *= 2;
-    const bool grid = G == 1 && width > kBalMaxCluster * kBalThreads;
-    const int teams = grid ? 1 : std::min(G, std::max(1, 2 * sms_ / cluster));
-    const BalTeams W{cluster, teams, grid, sms_};
-    bytes += (size_t)teams * kBalBig * kBalMaxCover * 4 + (size_t)G * 256 + ((size_t)16 << 20);
+    const BalTeams W = bal_teams(G, width, sms_);
+    const size_t warps = (size_t)(W.grid ? W.sms : W.teams * W.clusterSize) * kBalWarps;
+    bytes += warps * kBalMaxCover * 4 + (size_t)G * 256 + ((size_t)16 << 20);
     if ((rc = ensure_arena(bytes))) return rc;
     ar_.reset();
     std::vector<int> order(G);
@@ -778,7 +845,7 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
     A.newLit = ar_.get<int2>(nObj);
     A.found = reinterpret_cast<int *>(A.newLit);  // discovery ends before the first new literal
     A.flat = ar_.get<int>(nFlat);
-    A.scratch = ar_.get<int>((size_t)teams * kBalBig * kBalMaxCover);
+    A.scratch = ar_.get<int>(warps * kBalMaxCover);
     if (!dg || !dOrder || !A.cnt || !per[8] || !A.newLit || !A.flat || !A.scratch)
         return fail(CULS_E_OOM, "balance: arena exhausted");
     A.g = dg, A.order = dOrder, A.G = G;
@@ -808,11 +875,19 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
     check(cudaMemcpyAsync(hc.data(), A.cnt, sizeof(int) * (size_t)G * kBcSize, cudaMemcpyDeviceToHost, s), "d2h");
     if ((rc = fetch("balance covers"))) return rc;
     const int nCov = hostSmall_[0];
-    int64_t nLv = 0, nTab = 0;
+    // The reconstruction's teams: where covers are long on average, up to the
+    // largest cluster, as their arrays and lookups outgrow the L1 of few SMs
+    // (1,000 covers of 190 leaves: the call takes 35 ms with the two blocks
+    // that 1,000 threads fill, 27 with eight).
+    int64_t nLv = 0, nTab = 0, width2 = width;
     for (int i = 0; i < G; i++) {
         BalGraph &g = bg[i];
-        g.lvOff = (int)nLv, g.nLv = hc[(size_t)i * kBcSize + kBcLevels];
-        const uint32_t cap = pow2_at_least(2 * (int64_t)hc[(size_t)i * kBcSize + kBcCursor] + 64);
+        const int *c = &hc[(size_t)i * kBcSize];
+        const DevGraph &d = b.hg[ga + i];
+        const int64_t wide = d.nAnds / std::max(d.nLevels, 1), mean = c[kBcCursor] / std::max(c[kBcFound], 1);
+        width2 = std::max(width2, std::min<int64_t>(wide * (mean / kBalLocal), kBalMaxCluster * kBalThreads));
+        g.lvOff = (int)nLv, g.nLv = c[kBcLevels];
+        const uint32_t cap = pow2_at_least(2 * (int64_t)c[kBcCursor] + 64);
         g.tabOff = (int)nTab, g.mask = cap - 1;
         nLv += g.nLv, nTab += cap;
     }
@@ -834,7 +909,9 @@ int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> 
     if (int e = check(scan_exclusive(lvCnt, lvStart, nLv, nullptr, ar_, s), "scan")) return e;
     A.sorted = sorted, A.lvCnt = lvCnt, A.lvMax = lvMax, A.lvStart = lvStart;
     k_bal_init_tables<<<grid_1d(nTab, kBlock, sms_ * 16), kBlock, 0, s>>>(nTab, A);
-    if ((rc = check(launch_team(k_bal_rebuild<BlockTeam>, k_bal_rebuild<ClusterTeam>, k_bal_rebuild<GridTeam>, A, W, s),
+    A.spread = width2 > width;
+    if ((rc = check(launch_team(k_bal_rebuild<BlockTeam>, k_bal_rebuild<ClusterTeam>, k_bal_rebuild<GridTeam>, A,
+                                bal_teams(G, width2, sms_), s),
                     "balance launch")))
         return rc;
     launches_ += 4;

@@ -89,3 +89,40 @@ def test_batch_and_tight_budget_match_oracle(ctx):
                 assert same_graph(got, ref) and got.nLevels == ref.nLevels, i
     finally:
         tight.close()
+
+
+def caterpillar(n_pis, length, seed, repeat):
+    """Chains x = x & (p & q) whose pair nodes come after the chain's node, so
+    that a cover's DFS has every pair waiting on its stack; with `repeat`, the
+    pairs' literals recur (a leaf met again, or its complement)."""
+    rng = np.random.default_rng(seed)
+    f0, f1, outs = [-1] * (1 + n_pis), [-1] * (1 + n_pis), []
+
+    def new(a, b):
+        f0.append(min(a, b))
+        f1.append(max(a, b))
+        return 2 * (len(f0) - 1)
+
+    for k in range(60):
+        pool = iter(rng.permutation(np.arange(1, 1 + n_pis)))
+        x = 2 * int(next(pool))
+        for i in range(length if k % 4 else 40):
+            if repeat and i % 7 == 3:
+                p = int(rng.integers(1, 1 + n_pis))
+                q = 1 + (p + int(rng.integers(0, n_pis - 1))) % n_pis
+                x = new(x, new(2 * p, 2 * q))
+            else:
+                x = new(x, new(*[int(2 * next(pool) + (0 if repeat else rng.integers(0, 2))) for _ in range(2)]))
+        outs.append(x)
+    return C.Aig(n_pis, np.array(f0, np.int32), np.array(f1, np.int32), np.array(outs, np.int32))
+
+
+@pytest.mark.parametrize("length", [17, 60, 125, 127, 128, 200, 510])
+def test_deep_stacks_and_repeated_leaves_match_oracle(ctx, length):
+    check(ctx, caterpillar(1100, length, length, False))
+    check(ctx, caterpillar(1100, length, length, True))
+
+
+@pytest.mark.parametrize("count,size", [(700, 34), (3000, 100), (300, 400)])
+def test_many_long_covers_at_once_match_oracle(ctx, count, size):
+    check(ctx, products(7, 600, [size] * count))
