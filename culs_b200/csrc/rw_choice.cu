@@ -43,6 +43,9 @@ namespace {
 constexpr int kOverlay = 32;  // a multiple of 8
 constexpr int kSpecFrames = 16;
 
+// Candidates replayed one after another at a stretch, at most (see k_choice).
+constexpr int kMaxAlone = 64;
+
 struct ChoiceArgs {
     int64_t nL0;  // W positions [0, nL0) are constants and PIs
     const DevGraph *dg;
@@ -67,20 +70,22 @@ struct ChoiceArgs {
 // deleted, and the choice's caller does not read them, so nothing is kept
 // for them.
 
-// The committed graph, changed in place; a node's handle is its position.
+// The committed graph, changed in place by one thread between two barriers of
+// its block or cluster (so its loads may come from L1); a node's handle is its
+// position.
 struct GraphMem {
     int4 *rec;
     int64_t nL0;
-    __device__ __forceinline__ int4 ld(int x) const { return __ldcg(rec + x); }
+    __device__ __forceinline__ int4 ld(int x) const { return rec[x]; }
     __device__ __forceinline__ int append(int x, const int4 &) const { return x >= nL0 ? x : -1; }
     __device__ __forceinline__ void slots(int x0, const int4 &, int x1, const int4 &, int &k0, int &k1) const {
         k0 = x0 >= nL0 ? x0 : -1;
         k1 = x1 >= nL0 ? x1 : -1;
     }
-    __device__ __forceinline__ int del(int k) const { return k >= 0 ? __ldcg(&rec[k].w) : 0; }
-    __device__ __forceinline__ int ref(int k, int base) const { return k >= 0 ? __ldcg(&rec[k].z) : base; }
+    __device__ __forceinline__ int del(int k) const { return k >= 0 ? rec[k].w : 0; }
+    __device__ __forceinline__ int ref(int k, int base) const { return k >= 0 ? rec[k].z : base; }
     __device__ __forceinline__ void add(int k, int d) {
-        if (k >= 0) rec[k].z = __ldcg(&rec[k].z) + d;
+        if (k >= 0) rec[k].z += d;
     }
     __device__ __forceinline__ void set_del(int k, int v) { rec[k].w = v; }
     __device__ __forceinline__ void use_del(int) {}
@@ -395,28 +400,37 @@ struct Replay {
 
 // Rounds of a window of candidates, one per thread (see the top of the
 // file); T threads on each of B blocks (a cluster when B > 1), the window's
-// places dealt to the warps in turn.  A round
-// is three barriers: every thread replays its candidate and marks each
-// node it changes with its place in the window; a thread that saw one of its
-// nodes stale must wait, and the lowest such place ends the part that is
-// committed; committing adds the overlay's changes to the records.  Flags and
-// fanins that a committed candidate changes, no later committed one has used;
-// counts change by sums.  A candidate that outgrows its overlay ends the window and, at its
-// start, is replayed by thread 0 on the committed graph.  The next window is
-// up to four times the part committed, at least two places a warp.
+// places dealt to the warps in turn.  A round is three barriers: every thread
+// replays its candidate and marks each node it changes with its place in the
+// window; a thread that saw one of its nodes stale must wait, and the lowest
+// such place ends the part that is committed; committing adds the overlay's
+// changes to the records.  Flags and fanins that a committed candidate changes,
+// no later committed one has used; counts change by sums.  A candidate that
+// outgrows its overlay ends the window and, at its start, is replayed by thread
+// 0 on the committed graph.  The next window is up to four times the part
+// committed, at least two places a warp.
+//
+// Where candidates depend on one another in a row -- the stages of a ripple
+// carry chain, whose every replacement changes what the next one reads -- a
+// window commits hardly more than one of them.  After a window that committed
+// fewer than kFew, thread 0 replays the next ones on the committed graph: two
+// of them, and twice as many after each further such window.
 //
 // Bound: the latency of a replay's dependent record loads (about ten), 10-16
-// us a round.  One thread walking the candidates took 2.3-2.5 us for each.
-// 64x64 multiplier (4,157 candidates, 61 committed at a time; 25 when every
-// change of a node made it stale): 9.6 -> 0.76 ms; 1M-AND layered graph with
-// rw -z (80,251 tried, 345 at a time): 202 -> 3.7 ms; 256 graphs of up to 200k
-// ANDs: 15.1 -> 2.5 ms.
+// us a round, 2 us for a candidate replayed alone, whose records are in L1.
+// One thread walking the candidates took 2.3-2.5 us for each. 64x64 multiplier
+// (4,157 candidates, 61 committed at a time; 25 when every change of a node
+// made it stale): 9.6 -> 0.76 ms; 1M-AND layered graph with rw -z (80,251
+// tried, 345 at a time): 202 -> 3.7 ms; 256 graphs of up to 200k ANDs: 15.1 ->
+// 2.5 ms.  A ripple carry adder of 4,000 bits, rw -z: 29 ms by one thread, 135
+// in windows alone, 24 now; 300 of 64 bits: 0.79, 4.03, 0.92.
 template <int T, int B>
 __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
     using Overlay = OverlayMem<B == 1>;
     extern __shared__ int4 s_overlay[];
     __shared__ int s_stop[2];
     constexpr int kWarps = T / 32 * B;
+    constexpr int kFew = B == 1 ? 4 : 8;  // a round's time over a replay's
     const int tid = threadIdx.x, g = blockIdx.x / B, rank = blockIdx.x % B;
     const int t = (tid & 31) * kWarps + rank * (T / 32) + (tid >> 5);  // place in the window
     auto barrier = [] {
@@ -433,7 +447,7 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
     if (tid < 2) s_stop[tid] = INT_MAX;
     barrier();
     int nDone[kChReverted + 1] = {}, nPos = 0, expected = 0;
-    int window = A.serial ? 1 : T * B;
+    int window = A.serial ? 1 : T * B, alone = 0;
     for (int round = 0; base < end; round++) {
         const int nAct = min(window, end - base);
         const bool act = t < nAct;
@@ -455,9 +469,9 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
             if (R.busy) R.step();
             __syncwarp();
         }
-        const bool alone = R.m.full || R.st.full || A.serial;
+        const bool outgrown = R.m.full || R.st.full || A.serial;
         // the overlay's entries four at a time, so that their accesses overlap
-        const int n = act && !alone ? R.m.n : 0;
+        const int n = act && !outgrown ? R.m.n : 0;
         for (int k = 0; k < n; k += 4) {
             const int4 x = R.m.ids[(k >> 2) * T];
             const int node[4] = {x.x, x.y, x.z, x.w};
@@ -475,7 +489,7 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
         if (rank == 0 && tid == 0) s_stop[(round + 1) & 1] = INT_MAX;
         barrier();
         if (act) {
-            bool wait = alone;
+            bool wait = outgrown;
             for (int k = 0; k < n; k += 8) {
                 int4 m[8];
                 const int4 x = R.m.ids[(k >> 2) * T], y = R.m.ids[((k >> 2) + 1) * T];
@@ -489,7 +503,7 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
             if (wait) atomicMin(stop, t);
         }
         barrier();
-        int done = min(*stop, nAct);
+        const int done = min(*stop, nAct);
         for (int k = 0; k < n; k += 4) {
             const int4 x = R.m.ids[(k >> 2) * T];
             const int node[4] = {x.x, x.y, x.z, x.w};
@@ -509,8 +523,22 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
                 }
             }
         }
-        int code = R.code, gain = R.gain;
-        if (done == 0) {  // the first candidate alone
+        auto count = [&](int c, int code, int gain) {
+            A.choice[c] = code;
+#pragma unroll
+            for (int k = 0; k <= kChReverted; k++) nDone[k] += code == k;
+            if (code == kChCommitted) {
+                nPos += gain > 0;
+                expected += gain;
+            }
+        };
+        if (t < done) count(a.x, R.code, R.gain);
+        base += done;
+        // the next candidates alone: more and more while windows commit few
+        alone = done >= nAct || done >= kFew ? 0 : min(max(2, 2 * alone), kMaxAlone);
+        const int single = min(A.serial ? 1 : alone, end - base);
+        window = A.serial ? 1 : min(T * B, max(2 * kWarps, 4 * done));
+        if (single > 0) {
             barrier();
             if (t == 0) {
                 Replay<GraphMem, GraphStack> S;
@@ -519,24 +547,20 @@ __global__ void __launch_bounds__(T, 1) k_choice(ChoiceArgs A) {
                 S.trueLit = trueLit;
                 S.nL0 = nL0;
                 S.useZeros = A.useZeros;
-                S.code = kChNotVisited;
-                S.start(a, A.recB[base]);
-                while (S.busy) S.step();
-                code = S.code, gain = S.gain;
+                int4 na = A.recA[base], nb = A.recB[base];
+                for (int k = base; k < base + single; k++) {
+                    const int4 x = na, lv = nb;
+                    if (k + 1 < base + single) {  // the next one's, while this one is replayed
+                        na = A.recA[k + 1], nb = A.recB[k + 1];
+                    }
+                    S.code = kChNotVisited;
+                    S.start(x, lv);
+                    while (S.busy) S.step();
+                    count(x.x, S.code, S.gain);
+                }
             }
-            done = 1;
+            base += single;
         }
-        if (t < done) {
-            A.choice[a.x] = code;
-#pragma unroll
-            for (int k = 0; k <= kChReverted; k++) nDone[k] += code == k;
-            if (code == kChCommitted) {
-                nPos += gain > 0;
-                expected += gain;
-            }
-        }
-        base += done;
-        window = A.serial ? 1 : min(T * B, max(2 * kWarps, 4 * done));
         barrier();
     }
     const int tot[7] = {nDone[kChCommitted],   nPos,     nDone[kChCommitted] - nPos, nDone[kChReverted],

@@ -91,3 +91,51 @@ def test_every_block_width_matches_oracle(ctx, count):
         for k in STATS:
             want[k] += rs[k]
     assert {k: total[k] for k in STATS} == want
+
+
+def carry_chains(chains, bits, xors):
+    """Ripple carry adders of majority gates, or (xors) chains of two-input
+    exclusive ors in two forms: every stage's replacement changes what the next
+    stage's reads, so that windows commit hardly more than one candidate."""
+    n_pis = 2 * bits * chains
+    f0, f1, outs = [-1] * (1 + n_pis), [-1] * (1 + n_pis), []
+
+    def land(a, b):
+        f0.append(min(a, b))
+        f1.append(max(a, b))
+        return 2 * (len(f0) - 1)
+
+    def lor(a, b):
+        return land(a ^ 1, b ^ 1) ^ 1
+
+    def xor(a, b, form=0):
+        return land(lor(a, b), land(a, b) ^ 1) if form else lor(land(a, b ^ 1), land(a ^ 1, b))
+
+    for k in range(chains):
+        first = 1 + 2 * bits * k
+        c = land(2 * first, 2 * first + 2)
+        for i in range(1, bits):
+            x, y = 2 * (first + 2 * i), 2 * (first + 2 * i + 1)
+            if xors:
+                c = xor(xor(c, x, i & 1), y, ~i & 1)
+                continue
+            outs.append(xor(xor(x, y), c))
+            c = lor(lor(land(x, y), land(x, c)), land(y, c))
+        outs.append(c)
+    return C.Aig(n_pis, np.array(f0, np.int32), np.array(f1, np.int32), np.array(outs, np.int32))
+
+
+@pytest.mark.parametrize("xors", [False, True])
+@pytest.mark.parametrize("graphs,chains,bits", [(1, 1, 5), (1, 1, 60), (1, 1, 700), (1, 3, 300), (3, 1, 600), (40, 1, 33),
+                                                (160, 2, 12), (460, 1, 20)])
+def test_dependent_candidates_match_oracle(ctx, graphs, chains, bits, xors):
+    g = carry_chains(chains, bits, xors)
+    for zeros in [False, True]:
+        ref, rs = oracle(g, zeros)
+        assert not zeros or rs["replaced"] >= 1
+        d = ctx.upload_batch([g] * graphs) if graphs > 1 else ctx.upload(g)
+        ctx.rw(d, zeros=zeros)
+        st = ctx.rw_stats()
+        ctx.st(d)
+        assert all(same_graph(r, ref) for r in (d.download_all() if graphs > 1 else [d.download()])), zeros
+        assert {k: st[k] for k in STATS} == {k: graphs * rs[k] for k in STATS}, zeros
