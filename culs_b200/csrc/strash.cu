@@ -964,7 +964,7 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
     // (the 10M-AND single graph: each strash 22 -> 6 ms); the level dataflow
     // (k_dedup) for larger ones, whose rounds each move gigabytes and whose
     // merges can cascade for many rounds, and whenever the rounds do not
-    // settle within kMaxRounds.  CULS_DEDUP_MODE=levels|rounds forces either
+    // settle within kMaxHashRounds.  CULS_DEDUP_MODE=levels|rounds forces either
     // (the tests run both on the same graphs).
     constexpr int64_t kRoundsMaxLive = 16ll << 20;
     bool useRounds = nLive > 0 && nLive <= kRoundsMaxLive;
@@ -986,9 +986,12 @@ int Engine::strash_core(Batch &b, int64_t M, const int *L0, const int *L1, const
         if (prof_) this->mark(kMkDedupK0);
         k_round_init<<<gl, kBlock, 0, s>>>(nLive, srt, cur);
         launches_ += 1;
+        // later rounds' keys come on top of every node's first: a quarter of
+        // the table, or what a lowered capacity leaves
+        const int room = (int)std::min<int64_t>(cap / 4, std::max<int64_t>((int64_t)cap - nLive, 0));
         RoundArgs R{nLive, M,   srt,    tOf, rankOf, liveFlag, L0, L1, gidA, b.dg, AndTable{ts, cap - 1}, cur, slotT,
                     mapEnc, kl0, kl1,   foldTrivial ? 1 : 0, unique ? 1 : 0, nullptr, nullptr, slotBits, nullptr, nullptr,
-                    counters_ + kCtInserted, (int)(cap / 4), counters_ + kCtFull, status_};
+                    counters_ + kCtInserted, room, counters_ + kCtFull, status_};
         check(cudaMemsetAsync(flag, 0, sizeof(int) * kMaxHashRounds, s), "memset");
         bool all = true;  // the next round takes all nodes
         for (int r = 0; r < kMaxHashRounds && !settled;) {

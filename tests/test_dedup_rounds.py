@@ -80,3 +80,41 @@ def test_batch_of_copies_matches_oracle(monkeypatch):
             assert same_graph(got, o.graph())
     finally:
         ctx.close()
+
+
+def readers_of_a_duplicate(n):
+    """At most n ANDs: a node and its duplicate, a ladder of nodes none alike,
+    and one reader of the duplicate over each of those, which all get another
+    key when the duplicate has merged."""
+    n_pis, m = 40, (n - 2) // 2
+    first = 1 + n_pis  # the node, its duplicate, the ladder, the readers
+    v = np.arange(m)
+    f0 = 2 * (1 + v % n_pis) + (v // n_pis & 1)
+    f1 = np.where(v < 3, 2 * (1 + (v + 1) % n_pis), 2 * (first + 2 + v - 3) + 1)
+    r0, r1 = np.full(m, 2 * (first + 1)), 2 * (first + 2 + v)
+    pad, pair = np.full(first, -1), np.array([2, 2])
+    f0, f1 = np.concatenate([pad, pair, f0, r0]), np.concatenate([pad, pair + 2 * 7, f1, r1])
+    return C.Aig(n_pis, np.minimum(f0, f1).astype(np.int32), np.maximum(f0, f1).astype(np.int32),
+                 np.append(2 * (first + 2 + m + v), 2 * first).astype(np.int32))
+
+
+@pytest.mark.parametrize("cap,n", [(4096, 4096), (4096, 4094), (4096, 3900), (64, 64), (64, 50), (4096, 2048)])
+def test_a_table_with_room_for_every_node_is_enough(cap, n, monkeypatch):
+    """A table that the level dataflow gets along with does for the rounds
+    too, although their later rounds make further keys."""
+    g = readers_of_a_duplicate(n)
+    assert n - 1 <= g.nAnds <= n
+    o = Oracle()
+    o.set_graph(to_oracle(g))
+    o.st()
+    assert o.graph().nAnds == g.nAnds - 1
+    monkeypatch.setenv("CULS_STRASH_TABLE_CAP", str(cap))
+    ctx = C.Context()
+    try:
+        for mode in ["levels", "rounds"]:
+            monkeypatch.setenv("CULS_DEDUP_MODE", mode)
+            d = ctx.upload(g)
+            ctx.st(d)
+            assert same_graph(d.download(), o.graph()), mode
+    finally:
+        ctx.close()
