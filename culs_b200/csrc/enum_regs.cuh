@@ -50,11 +50,6 @@ __device__ __forceinline__ uint32_t rc_value(const RCut &c) {
     return (uint32_t)value & 0x7FFu;
 }
 
-template <class T>
-__device__ __forceinline__ T pick4(const T (&v)[4], int i) {
-    return i == 0 ? v[0] : (i == 1 ? v[1] : (i == 2 ? v[2] : v[3]));
-}
-
 // MergeCutOrdered / MergeCut with the leaf attributes carried along: four
 // merge steps, each taking the smaller head leaf (both when equal) and moving
 // the lists up, without branches -- the lanes of the warp-wide enumeration
@@ -101,10 +96,6 @@ __device__ __forceinline__ bool rc_merge(const RCut &a, const RCut &b, RCut &o, 
     o.sign = a.sign | b.sign;
     o.used = 1;
     return x[0] == kEnd && y[0] == kEnd;
-}
-__device__ __forceinline__ bool rc_merge(const RCut &a, const RCut &b, RCut &o) {
-    int pa, pb;
-    return rc_merge(a, b, o, pa, pb);
 }
 
 // CutTruthtable (rewrite.cu:223-229); pa, pb as rc_merge gives them.

@@ -3,7 +3,8 @@
 // tt_stretch / tt_shrink (CutTruthStretch / CutTruthShrink, CULS
 // src/algorithms/rewrite.cu:213-241) for every 16-bit table and phase, and
 // rc_merge against the step-by-step merge with early exits (MergeCutOrdered,
-// rewrite.cu:111-176) on two million random cut pairs.  Built and run by
+// rewrite.cu:111-176), with the phases that CutTruthPhase (rewrite.cu:195-201)
+// finds in the merged cut, on two million random cut pairs.  Built and run by
 // tests/test_flat_helpers.py.
 #include <cstdio>
 #include <random>
@@ -13,6 +14,18 @@
 #define __forceinline__ inline
 #include "enum_regs.cuh"
 using namespace culs;
+template <class T>
+static T pick4(const T (&v)[4], int i) {
+    return v[i < 3 ? i : 3];
+}
+// bit s: the merged cut's leaf s is one of x's
+static int phase_of(const RCut &m, const RCut &x) {
+    int p = 0;
+    for (int s = 0; s < (int)m.n; s++)
+        for (int j = 0; j < (int)x.n; j++)
+            if (x.l[j] == m.l[s]) p |= 1 << s;
+    return p;
+}
 // the merge with early exits: stop when both inputs are used up, fail when
 // leaves remain after four steps
 static bool seq_merge(const RCut &a0, const RCut &b0, RCut &o) {
@@ -62,11 +75,12 @@ int main() {
             x->sign = rng();
         }
         RCut o1{}, o2{};
-        bool r1 = seq_merge(a, b, o1), r2 = rc_merge(a, b, o2);
+        int pa, pb;
+        bool r1 = seq_merge(a, b, o1), r2 = rc_merge(a, b, o2, pa, pb);
         n++;
         if (r1 != r2) { bad++; continue; }
         if (!r1) continue;
-        bool same = o1.n == o2.n && o1.sign == o2.sign;
+        bool same = o1.n == o2.n && o1.sign == o2.sign && pa == phase_of(o1, a) && pb == phase_of(o1, b);
         for (int j = 0; j < 4; j++) same &= o1.l[j] == o2.l[j] && o1.ref[j] == o2.ref[j] && o1.lid[j] == o2.lid[j];
         if (!same) bad++;
     }

@@ -126,3 +126,27 @@ def test_deep_stacks_and_repeated_leaves_match_oracle(ctx, length):
 @pytest.mark.parametrize("count,size", [(700, 34), (3000, 100), (300, 400)])
 def test_many_long_covers_at_once_match_oracle(ctx, count, size):
     check(ctx, products(7, 600, [size] * count))
+
+
+def no_ands(n_pis, n_pos):
+    pad = np.full(1 + n_pis, -1, np.int32)
+    return C.Aig(n_pis, pad, pad.copy(), (np.arange(n_pos) % (2 + 2 * n_pis)).astype(np.int32))
+
+
+def test_graphs_without_and_nodes_match_oracle(ctx):
+    """Alone, a batch of them, and among others, together and one at a time."""
+    check(ctx, no_ands(3, 8))
+    check(ctx, no_ands(1, 0))
+    gs = [no_ands(5, 4), C.gen_multiplier(6), no_ands(2, 1), C.gen_layered(3, 600, 400, 22000, 10, 3, 0.1, True),
+          no_ands(300, 700)]
+    tight = C.Context(hbm_budget=max(g.nObjs for g in gs) * 900 + (200 << 20))
+    try:
+        for c in [ctx, tight]:
+            for batch in [gs, gs[:1] + gs[2:3] + gs[4:], gs[::-1]]:
+                d = c.upload_batch(batch)
+                c.b(d)
+                for g, got in zip(batch, d.download_all()):
+                    ref = oracle_b(g)
+                    assert same_graph(got, ref) and got.nLevels == ref.nLevels
+    finally:
+        tight.close()

@@ -1,13 +1,13 @@
-"""The choice loop of a single graph (CULS src/algorithms/rewrite.cu:830-921)
-runs on a thread-block cluster with the graph's fanins, deletion flags and
-reference counts in distributed shared memory when the graph has at most
-65,536 objects (rewritten nodes included), and one thread per graph over
-HBM otherwise (CULS_CHOICE_GLOBAL forces the latter).  Both must give the
-oracle's graph, with the same choice statistics."""
+"""The choice loop (CULS src/algorithms/rewrite.cu:830-921) gives each graph
+a block, or, where at most 18 graphs have 1,024 candidates each on average, a
+cluster of eight blocks, and replays their candidates in windows;
+CULS_CHOICE_GLOBAL replays every candidate alone on the graph instead.  Each
+way must give the oracle's graph, with the same choice statistics."""
 import pytest
 
 import culs_b200 as C
 from oracle.oracle import Oracle
+from test_choice_windows import STATS, carry_chains
 from util import same_graph, to_oracle
 
 pytestmark = pytest.mark.gpu
@@ -15,11 +15,11 @@ pytestmark = pytest.mark.gpu
 
 def graphs():
     return [
-        C.gen_multiplier(4),                                  # one block of 256 objects
+        C.gen_multiplier(4),  # a block
         C.gen_multiplier(16),
-        C.gen_multiplier(64),                                 # config 2: six blocks
-        C.gen_layered(11, 64, 32, 60000, 120, 4, 0.0, True),  # near the bound
-        C.gen_layered(13, 128, 64, 130000, 160, 4, 0.0, True),  # above it: one thread over HBM
+        C.gen_multiplier(64),  # a cluster
+        C.gen_layered(11, 64, 32, 60000, 120, 4, 0.0, True),
+        C.gen_layered(13, 128, 64, 130000, 160, 4, 0.0, True),
     ]
 
 
@@ -53,5 +53,49 @@ def test_cluster_choice_matches_oracle_and_global_walk(zeros, monkeypatch):
             assert same_graph(got["global"][0], ref), i
             for k in ["replaced", "replaced_pos", "replaced_zero", "reverted", "compromised"]:
                 assert got["cluster"][1][k] == got["global"][1][k] == rs[k], (i, k)
+    finally:
+        ctx.close()
+
+
+def replacements(st):
+    return st["candidates"] - st["new_idx"]
+
+
+@pytest.mark.parametrize("bits,cluster", [(342, False), (343, True)])
+def test_both_sides_of_the_line_match_oracle(bits, cluster):
+    g = carry_chains(1, bits, False)
+    ref, rs = oracle(g, True)
+    ctx = C.Context()
+    try:
+        d = ctx.upload(g)
+        ctx.rw(d, zeros=True)
+        st = ctx.rw_stats()
+        assert abs(replacements(st) - 1024) <= 3 and (replacements(st) >= 1024) == cluster
+        ctx.st(d)
+        assert same_graph(d.download(), ref) and {k: st[k] for k in STATS} == {k: rs[k] for k in STATS}
+    finally:
+        ctx.close()
+
+
+@pytest.mark.parametrize("first", [0, 2, 3])
+def test_several_graphs_on_clusters_match_oracle(first):
+    """Graphs of very different numbers of candidates, each on its cluster."""
+    gs = [C.gen_multiplier(8), C.gen_multiplier(48), C.gen_layered(11, 64, 32, 60000, 120, 4, 0.0, True),
+          carry_chains(2, 400, False), carry_chains(30, 40, True), C.gen_multiplier(2)][first:]
+    ctx = C.Context()
+    try:
+        for zeros in [False, True]:
+            d = ctx.upload_batch(gs)
+            ctx.rw(d, zeros=zeros)
+            st = ctx.rw_stats()
+            assert not zeros or replacements(st) >= 1024 * len(gs)
+            ctx.st(d)
+            want = dict.fromkeys(STATS, 0)
+            for g, got in zip(gs, d.download_all()):
+                ref, rs = oracle(g, zeros)
+                assert same_graph(got, ref)
+                for k in STATS:
+                    want[k] += rs[k]
+            assert {k: st[k] for k in STATS} == want
     finally:
         ctx.close()

@@ -139,3 +139,44 @@ def test_dependent_candidates_match_oracle(ctx, graphs, chains, bits, xors):
         ctx.st(d)
         assert all(same_graph(r, ref) for r in (d.download_all() if graphs > 1 else [d.download()])), zeros
         assert {k: st[k] for k in STATS} == {k: graphs * rs[k] for k in STATS}, zeros
+
+
+def hub_cones(n, drop, extra):
+    """n cones over one AND node h and inputs of their own, ((h & b) | (h & !b))
+    & (c | d) = h & (c | d), each replacement taking one of h's two references
+    away, or with `drop` ((h & b) | (!h & b)) & (c | d) = b & (c | d), both of
+    them, so that the last replacement deletes h; `extra` more references from
+    outputs."""
+    n_pis = 2 + 3 * n
+    f0, f1, outs = [-1] * (1 + n_pis), [-1] * (1 + n_pis), []
+
+    def new(a, b):
+        f0.append(min(a, b))
+        f1.append(max(a, b))
+        return 2 * (len(f0) - 1)
+
+    h = new(2, 4)
+    for i in range(n):
+        b, c, d = [2 * (3 + 3 * i + k) for k in range(3)]
+        x = new(new(h, b) ^ 1, new(h ^ drop, b ^ 1 ^ drop) ^ 1) ^ 1
+        outs.append(new(x, new(c ^ 1, d ^ 1) ^ 1))
+    return C.Aig(n_pis, np.array(f0, np.int32), np.array(f1, np.int32), np.array(outs + [h] * extra, np.int32))
+
+
+@pytest.mark.parametrize("drop", [0, 1])
+@pytest.mark.parametrize("n,extra", [(1, 0), (126, 2), (127, 0), (127, 1), (127, 2), (127, 3), (128, 2), (200, 1), (510, 1),
+                                     (511, 0), (511, 1), (512, 0), (600, 0), (1100, 0), (1100, 3000), (3000, 0), (3000, 1)])
+def test_a_node_with_many_references_matches_oracle(ctx, n, extra, drop):
+    """Reference counts around 255, where the MFFC count of a node saturates,
+    and around 1,022, where the lowest count that mattered to a candidate does;
+    windows that take more references away than that."""
+    g = hub_cones(n, drop, extra)
+    for zeros in [False, True]:
+        ref, rs = oracle(g, zeros)
+        assert rs["replaced"] >= n
+        d = ctx.upload(g)
+        ctx.rw(d, zeros=zeros)
+        st = ctx.rw_stats()
+        ctx.st(d)
+        assert same_graph(d.download(), ref), zeros
+        assert {k: st[k] for k in STATS} == {k: rs[k] for k in STATS}, zeros
