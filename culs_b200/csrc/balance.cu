@@ -804,9 +804,9 @@ cudaError_t launch_team(K block, K cluster, K all, const BalArgs &A, const BalTe
 
 }  // namespace
 
-// Graphs [ga, gb) of b, at least one of them with an AND node; their results
-// go to b's spare buffers from object ng[ga].base on, and ng's sizes and
-// following bases are set.
+// Graphs [ga, gb) of b (any of them may have no AND node); their results go to
+// b's spare buffers from object ng[ga].base on, and ng's sizes and following
+// bases are set.
 int Engine::balance_group(const Batch &b, int ga, int gb, std::vector<DevGraph> &ng) {
     cudaStream_t s = s_;
     const int G = gb - ga;

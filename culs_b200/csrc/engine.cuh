@@ -235,7 +235,6 @@ class Engine {
   private:
     int fail(int code, const std::string &msg);
     int check(cudaError_t e, const char *what);
-    int check_status(const char *what);
     int fetch(const char *what);  // ExecCtx::fetch
     int ensure_arena(size_t bytes);
     int ensure_stage(size_t ints);  // pinned host staging of at least `ints` int32

@@ -303,8 +303,6 @@ int Engine::fetch(const char *what) {
     return X.fetch(what);
 }
 
-int Engine::check_status(const char *what) { return fetch(what); }
-
 // CULS_SPIN_LIMIT (spin iterations, 0 or unset = the built-in bound of about
 // one second) bounds every dependency wait of the next calls; the tests lower
 // it to make waits run out on purpose.  Read at each call, like

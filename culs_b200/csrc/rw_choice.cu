@@ -704,11 +704,11 @@ int rw_choice(ExecCtx &X, Batch &b, RwWork &w) {
         // cluster), so that the replays of a window share no SM's load path
         // (1M-AND rw -z 4.6 -> 3.7 ms, 64x64 multiplier 0.87 -> 0.76; its
         // barriers cost more where 95 candidates are all there are: 0.28 ->
-        // 0.31); else a window as wide
-        // as an SM's shared memory allows while there is an SM for every graph, narrower ones so that more
-        // graphs are resident when there are more (a batch's graphs have
-        // short windows: 7 candidates are committed at a time on the c4
-        // family's, 340 on the 1M-AND graph).
+        // 0.31); else a window as wide as an SM's shared memory allows while
+        // there is an SM for every graph, narrower ones so that more graphs
+        // are resident when there are more (a batch's graphs have short
+        // windows: 7 candidates are committed at a time in 256 graphs of up to
+        // 200k ANDs, 345 in the 1M-AND graph).
         if (X.clusters && 8 * G <= X.sms && nRep >= 1024 * (int64_t)G)
             rc = X.check(launch_choice<128, 8>(A, G, s), "choice launch");
         else if (G <= X.sms)

@@ -2,14 +2,17 @@
 // Inputs + CutEnumerate (CULS src/algorithms/rewrite.cu:63-74,268-294).
 //
 // The reference launches one kernel per level (rewrite.cu:703-704).  Here a
-// single persistent dataflow kernel walks the level-major layout in order:
-// each thread owns one node, waits (bounded) until both fanins have published
-// their cut sets, and replays the reference's per-pair slot policy exactly.
-// The 8 slots live in registers (fully unrolled slot loops), and every cut
-// record carries its leaves' reference counts and local-id bits (cutA), so a
-// node reads nothing but its two fanins' 16 cut records.  Pairs whose 32-bit
-// signatures already exceed 4 leaves are rejected from the fanins' {sign,
-// packed} words before any leaf data is fetched.
+// run of levels of like width is one launch of a persistent dataflow kernel,
+// which walks the level-major layout in order: a node waits (bounded) until
+// both fanins have published their cut sets, and the reference's per-pair slot
+// policy is replayed exactly.  Wide levels take a node per thread
+// (k_enumerate), with the 8 slots in registers (fully unrolled slot loops);
+// narrower ones a node per warp (k_enumerate_warp), which builds the candidate
+// cuts of all pairs side by side.  Every cut record carries its leaves'
+// reference counts and local-id bits (cutA), so a node reads nothing but its
+// two fanins' 16 cut records.  Pairs whose 32-bit signatures already exceed 4
+// leaves are rejected from the fanins' {sign, packed} words before any leaf
+// data is used.
 #include <algorithm>
 #include <vector>
 

@@ -19,10 +19,12 @@
 //
 // B200 design: no per-frontier host loop.  Liveness is a reverse Kahn
 // worklist, levels an in-order dataflow (a forward Kahn worklist over a
-// fanout CSR as the fallback), and hashing either a few full-width rounds
-// that iterate the mapping to its fixed point (batches of up to 16M live
-// nodes) or a single in-order dataflow pass whose dependency waits are
-// per-level completion counters (bounded spins).
+// fanout CSR as the fallback; a single graph of up to 57,000 nodes in one
+// block's shared memory), and hashing either rounds that iterate the mapping
+// to its fixed point, the first over all nodes and the later ones over those
+// whose fanins' mapping changed (batches of up to 16M live nodes), or a single
+// in-order dataflow pass whose dependency waits are per-level completion
+// counters (bounded spins).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -504,13 +506,17 @@ __global__ void __launch_bounds__(kDedupChunk) k_dedup(DedupArgs A) {
 // of slots that received a key.  No thread waits on another, so a deep,
 // narrow graph costs a few launches instead of one wait latency per level.
 //
-// Keys a node had earlier stay in the table.  They do no harm: mappings are
-// equivalences that only grow (two nodes with equal keys under a part of the
-// final equivalence are equal under all of it), so every node ever inserted
-// with what is a final key has that key in the end, and a slot's lowest rank
-// is its lowest final member's.  For the same reason the mappings may be
-// read and written in place: a reader of an older one is visited again in
-// the round after.
+// The mappings are read and written in place, so that of two nodes that map
+// alike one may move a round before the other, and keys that a node had
+// earlier stay in the table.  Neither does harm.  Every mapping on the way is
+// sound: what it makes equal is equal in the fixed point (nodes with equal
+// keys under a sound mapping are).  So a node that was ever inserted with a
+// key of the fixed point, whose literals are final ones, has that key in the
+// end.  Every change is seen by the node's readers a round later, so in a round
+// without any, all nodes are keyed by the mapping as it stands; by induction
+// over the levels it is the fixed point: a node's fanins map right, so its key
+// is final, its slot holds just the nodes of that key, and it maps to the
+// lowest.
 //
 // A round over all nodes moves their keys and table sectors (9.5M nodes: 1.1
 // ms, and merges cascade for 15 rounds on a 256-graph batch); a later round
