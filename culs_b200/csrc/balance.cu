@@ -233,9 +233,12 @@ __device__ int bal_cover_dfs(const BalView &V, const int *nfo, int v, int *leave
 // The same DFS by a whole warp, with room for every leaf (the DFS stops at
 // 1,024): all lanes hold the walk's state, the stack lies in shared memory and
 // the leaves, in global memory, are compared 32 at a time.  A thread a large
-// cover, as in bal_cover_dfs, takes 4 ms for 190 leaves, a warp 0.1.
+// cover, as in bal_cover_dfs, takes 4 ms for 190 leaves, a warp 0.1.  (A
+// function of its own, so that the kernel's registers need not be spilled for
+// it: 48x48 multiplier, which has no such cover, 1.217 ms in the kernel before
+// there was this function, 1.234 with it inlined, 1.222.)
 template <class Team>
-__device__ int bal_cover_dfs_warp(const BalView &V, const int *nfo, int v, int *stk, int *leaves) {
+__device__ __noinline__ int bal_cover_dfs_warp(BalView V, const int *nfo, int v, int *stk, int *leaves) {
     const unsigned F = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     int top = 0, n = 0, cur = 2 * v;  // cur: the literal popped, with `top` left on the stack
